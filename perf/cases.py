@@ -153,7 +153,7 @@ def _sched(case):
 def prepare(case, seed):
     st = {"case": case}
     if case["kind"] == "ensemble":
-        st["sizes"] = fqbatch.log_uniform_sizes(case["count"], case["lo"], case["hi"], seed=seed)
+        st["sizes"] = fqbatch.log_uniform_sizes(case["count"], case["lo"], case["hi"], seed=3)
         st["seeds"] = 1000 * (seed % 1_000_003) + np.arange(case["count"])
         return st
     u0 = _initial(case, seed)
