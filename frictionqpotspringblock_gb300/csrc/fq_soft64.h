@@ -2,20 +2,21 @@
  * IEEE-754 binary64 addition, subtraction and multiplication, rounded to nearest with ties to even,
  * computed with 32-bit integer instructions.
  *
- * Why: the step kernels are bound by the fp64 pipe, which on this GPU retires under two fp64
- * operations per clock per SM, while the 32-bit integer pipes (ALU and IMAD) sit mostly idle.
- * Issuing a share of a kernel's fp64 operations through these functions runs the pipes side by side.
- * The results are bit-identical to the hardware instruction for every input, so the arithmetic of the
- * step (and its parity with the reference) does not change.  Everything is written on 32-bit words:
- * 64-bit integer instructions would go back to the fp64 pipe on this GPU.
+ * Why: the step kernels are bound by the fp64 pipe, which takes an addition or multiplication of a warp
+ * every 19 cycles per SM, while the 32-bit pipes mostly idle.  Issuing a share of a kernel's fp64
+ * operations through these functions runs the pipes side by side.  The results are bit-identical to the
+ * hardware instruction for every input, so the arithmetic of the step (and its parity with the
+ * reference) does not change.  Cost per warp and SM, measured in streams of independent operations: an
+ * addition 25 cycles (57 instructions, 45 of them on the ALU pipe, which takes one every half cycle), a
+ * multiplication by a prepared factor 12 cycles (31 instructions, 14 ALU and 14 multiply-add).
  *
  * Method (the definition of the format, nothing more): unpack sign, exponent and significand; for a
- * sum, align the smaller significand with a sticky bit, add or subtract, normalise; for a product,
- * form the 106-bit product of the significands from 32 x 32-bit partial products; round to nearest
- * even on the guard bits.  The fast path covers normal operands with a normal result; everything else
- * (zero, subnormal, infinite or NaN operands, a subnormal or overflowing result) is handed to the
- * hardware instruction in a branch that is not taken in practice.  The host build of the same source
- * (tests) checks the fast path against the host's IEEE arithmetic.
+ * sum, align the smaller significand, add or subtract, normalise; for a product, form the product of
+ * the significands from 32 x 32-bit partial products; round to nearest even.  The fast path covers
+ * normal operands with a normal result; everything else is handed to the hardware instruction in a
+ * branch that is not taken in practice.  Bits that only decide rare ties are not formed at all: where
+ * they could matter, the hardware decides too.  The host build of the same source (tests) checks the
+ * fast path against the host's IEEE arithmetic.
  */
 #ifndef FQSB_FQ_SOFT64_H
 #define FQSB_FQ_SOFT64_H
@@ -24,7 +25,8 @@
 
 #if defined(__CUDA_ARCH__)
 /* Slow paths: not inlined, so the compiler branches around them instead of predicating an fp64
- * instruction into every call site. */
+ * instruction into every call site (a predicated one takes its pipe cycles even when no lane needs it:
+ * the step at N = 2^22 takes 225 us with inlined ones, 159 us with calls). */
 static __device__ __noinline__ double fq_s_hw_add(double a, double b)
 {
     return __dadd_rn(a, b);
@@ -55,36 +57,67 @@ FQ_HD uint32_t fq_s_shl64hi(uint32_t lo, uint32_t hi, uint32_t n)
 {
     return __funnelshift_lc(lo, hi, n);
 }
+FQ_HD uint32_t fq_s_max(uint32_t a, uint32_t b)
+{
+    return umax(a, b);
+}
+FQ_HD uint32_t fq_s_min(uint32_t a, uint32_t b)
+{
+    return umin(a, b);
+}
 FQ_HD uint32_t fq_s_clz(uint32_t x)
 {
     return (uint32_t)__clz((int)x);
 }
-/* (rh:rl) = (ah:al) + (bh:bl) mod 2^64, on 32-bit adds with carry */
-FQ_HD void fq_s_add64(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& rh, uint32_t& rl)
-{
-    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, %5;" : "=r"(rl), "=r"(rh) : "r"(al), "r"(bl), "r"(ah), "r"(bh));
-}
-FQ_HD void fq_s_sub64(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& rh, uint32_t& rl)
-{
-    asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, %4, %5;" : "=r"(rl), "=r"(rh) : "r"(al), "r"(bl), "r"(ah), "r"(bh));
-}
-/* 64 x 64 -> 128-bit product of (ah:al) and (bh:bl) in 32-bit multiply-adds: p3:p2:p1:p0 */
-FQ_HD void fq_s_mul128(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& p3, uint32_t& p2, uint32_t& p1,
-                       uint32_t& p0)
+/* subtract: (mh:ml:g) = (xh:xl:0) - (h:l:g), else (xh:xl:0) + (h:l:g); one predicated chain each */
+FQ_HD void fq_s_addsub96(uint32_t diff, uint32_t xh, uint32_t xl, uint32_t h, uint32_t l, uint32_t& g, uint32_t& mh,
+                         uint32_t& ml)
 {
     asm("{\n\t"
-        "mul.lo.u32     %0, %4, %6;\n\t"
-        "mul.hi.u32     %1, %4, %6;\n\t"
-        "mad.lo.cc.u32  %1, %5, %6, %1;\n\t"
-        "madc.hi.u32    %2, %5, %6, 0;\n\t"
-        "mad.lo.cc.u32  %1, %4, %7, %1;\n\t"
-        "madc.hi.cc.u32 %2, %4, %7, %2;\n\t"
-        "addc.u32       %3, 0, 0;\n\t"
-        "mad.lo.cc.u32  %2, %5, %7, %2;\n\t"
-        "madc.hi.u32    %3, %5, %7, %3;\n\t"
+        ".reg .pred p;\n\t"
+        "setp.lt.s32 p, %7, 0;\n\t"
+        "@p sub.cc.u32  %0, 0, %0;\n\t"
+        "@p subc.cc.u32 %1, %4, %6;\n\t"
+        "@p subc.u32    %2, %3, %5;\n\t"
+        "@!p add.cc.u32 %1, %4, %6;\n\t"
+        "@!p addc.u32   %2, %3, %5;\n\t"
         "}"
-        : "=&r"(p0), "=&r"(p1), "=&r"(p2), "=&r"(p3)
-        : "r"(al), "r"(ah), "r"(bl), "r"(bh));
+        : "+r"(g), "=&r"(ml), "=&r"(mh)
+        : "r"(xh), "r"(xl), "r"(h), "r"(l), "r"(diff));
+}
+/* (rh:rl) = (ah:al) + (c != 0) */
+FQ_HD void fq_s_add64c(uint32_t ah, uint32_t al, uint32_t c, uint32_t& rh, uint32_t& rl)
+{
+    asm("{\n\t"
+        ".reg .u32 t;\n\t"
+        "add.cc.u32  t, %4, 0xffffffff;\n\t"
+        "addc.cc.u32 %0, %2, 0;\n\t"
+        "addc.u32    %1, %3, 0;\n\t"
+        "}"
+        : "=&r"(rl), "=r"(rh)
+        : "r"(al), "r"(ah), "r"(c));
+}
+/* (rh:rl) = (ah:al) + (t:0) + (g >= 2^31) */
+FQ_HD void fq_s_round64(uint32_t ah, uint32_t al, uint32_t g, uint32_t t, uint32_t& rh, uint32_t& rl)
+{
+    asm("{\n\t"
+        ".reg .u32 z;\n\t"
+        "add.cc.u32  z, %4, 0x80000000;\n\t"
+        "addc.cc.u32 %0, %2, 0;\n\t"
+        "addc.u32    %1, %3, %5;\n\t"
+        "}"
+        : "=&r"(rl), "=r"(rh)
+        : "r"(al), "r"(ah), "r"(g), "r"(t));
+}
+/* words 3, 2, 1 of the product of (ah:al) < 2^53 and (bh:bl) */
+FQ_HD void fq_s_mul53(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& p3, uint32_t& p2, uint32_t& p1)
+{
+    const uint64_t t1 = (uint64_t)ah * bl + __umulhi(al, bl); /* < 2^54 */
+    const uint64_t t2 = (uint64_t)al * bh + (uint32_t)t1;
+    const uint64_t t3 = (uint64_t)ah * bh + (t1 >> 32) + (t2 >> 32);
+    p1 = (uint32_t)t2;
+    p2 = (uint32_t)t3;
+    p3 = (uint32_t)(t3 >> 32);
 }
 #define FQ_S_UNLIKELY(x) __builtin_expect(!!(x), 0)
 #else
@@ -127,105 +160,122 @@ static inline uint32_t fq_s_shl64hi(uint32_t lo, uint32_t hi, uint32_t n)
     n = n > 32 ? 32 : n;
     return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32);
 }
+static inline uint32_t fq_s_max(uint32_t a, uint32_t b)
+{
+    return a > b ? a : b;
+}
+static inline uint32_t fq_s_min(uint32_t a, uint32_t b)
+{
+    return a < b ? a : b;
+}
 static inline uint32_t fq_s_clz(uint32_t x)
 {
     return x ? (uint32_t)__builtin_clz(x) : 32u;
 }
-static inline void fq_s_add64(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& rh, uint32_t& rl)
+static inline void fq_s_addsub96(uint32_t diff, uint32_t xh, uint32_t xl, uint32_t h, uint32_t l, uint32_t& g,
+                                 uint32_t& mh, uint32_t& ml)
 {
-    uint64_t r = (((uint64_t)ah << 32) | al) + (((uint64_t)bh << 32) | bl);
+    const unsigned __int128 x = (unsigned __int128)(((uint64_t)xh << 32) | xl) << 32;
+    const unsigned __int128 y = ((unsigned __int128)(((uint64_t)h << 32) | l) << 32) | g;
+    const unsigned __int128 r = (int32_t)diff < 0 ? x - y : x + y;
+    g = (uint32_t)r;
+    ml = (uint32_t)(r >> 32);
+    mh = (uint32_t)(r >> 64);
+}
+static inline void fq_s_add64c(uint32_t ah, uint32_t al, uint32_t c, uint32_t& rh, uint32_t& rl)
+{
+    const uint64_t r = (((uint64_t)ah << 32) | al) + (c != 0u ? 1u : 0u);
     rh = (uint32_t)(r >> 32);
     rl = (uint32_t)r;
 }
-static inline void fq_s_sub64(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& rh, uint32_t& rl)
+static inline void fq_s_round64(uint32_t ah, uint32_t al, uint32_t g, uint32_t t, uint32_t& rh, uint32_t& rl)
 {
-    uint64_t r = (((uint64_t)ah << 32) | al) - (((uint64_t)bh << 32) | bl);
+    const uint64_t r = (((uint64_t)ah << 32) | al) + ((uint64_t)t << 32) + (g >> 31);
     rh = (uint32_t)(r >> 32);
     rl = (uint32_t)r;
 }
-static inline void fq_s_mul128(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& p3, uint32_t& p2,
-                               uint32_t& p1, uint32_t& p0)
+static inline void fq_s_mul53(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, uint32_t& p3, uint32_t& p2,
+                              uint32_t& p1)
 {
-    unsigned __int128 p = (unsigned __int128)((((uint64_t)ah << 32) | al)) * (((uint64_t)bh << 32) | bl);
-    p0 = (uint32_t)p;
-    p1 = (uint32_t)(p >> 32);
-    p2 = (uint32_t)(p >> 64);
-    p3 = (uint32_t)(p >> 96);
+    const uint64_t t1 = (uint64_t)ah * bl + (((uint64_t)al * bl) >> 32);
+    const uint64_t t2 = (uint64_t)al * bh + (uint32_t)t1;
+    const uint64_t t3 = (uint64_t)ah * bh + (t1 >> 32) + (t2 >> 32);
+    p1 = (uint32_t)t2;
+    p2 = (uint32_t)t3;
+    p3 = (uint32_t)(t3 >> 32);
 }
 #define FQ_S_UNLIKELY(x) __builtin_expect(!!(x), 0)
 #endif
 
-/* Sum of (ah:al) and (bh:bl), the bit patterns of two doubles (b's sign already flipped for a
- * subtraction); a and b are the same values as doubles, for the hardware path. */
+/* What fq_s_add_words leaves over.  Sums that cancel (opposite signs, exponents at most one apart, both well
+ * above the subnormals) are exact and formed here as well; the rest is the hardware's. */
+#if defined(__CUDA_ARCH__)
+static __device__ __noinline__ double fq_s_add_rest(double a, double b)
+#else
+static inline double fq_s_add_rest(double a, double b)
+#endif
+{
+    const uint64_t x = fq_bits(a), y = fq_bits(b);
+    const int ex = (int)((x >> 52) & 0x7ff), ey = (int)((y >> 52) & 0x7ff);
+    const int e = ex < ey ? ex : ey;
+    if (e < 56 || ex > 0x7fe || ey > 0x7fe || ex - e > 1 || ey - e > 1 || (int64_t)(x ^ y) >= 0) {
+        return fq_s_hw_add(a, b);
+    }
+    const uint64_t one = 1ULL << 52;
+    const uint64_t mx = ((x & (one - 1)) | one) << (ex - e), my = ((y & (one - 1)) | one) << (ey - e);
+    const bool less = mx < my;
+    uint64_t m = less ? my - mx : mx - my;
+    const uint32_t hi = (uint32_t)(m >> 32);
+    const int z = (int)(hi != 0u ? fq_s_clz(hi) : 32u + fq_s_clz((uint32_t)m)) - 11;
+    if (m == 0 || z < 0) {
+        return fq_s_hw_add(a, b);
+    }
+    m <<= z;
+    return fq_from_bits(((less ? y : x) & (1ULL << 63)) | ((uint64_t)(e - z - 1) << 52) + m);
+}
+
+/*
+ * x + y of two doubles given as words (b's sign already flipped for a subtraction); a and b are the
+ * same values, for the hardware path.  Bound by the ALU pipe.
+ *
+ * The operands are ordered by their high words alone; y's significand is aligned into 96 bits
+ * (h:l:g, g below the last place of x), added to or subtracted from x's, and normalised so that the
+ * leading bit sits at bit 53 of (mh:ml) and the bit below the last place at bit 0.  No sticky bit is
+ * kept: bits of y below g can change the rounding only where the bits kept below the rounding bit are
+ * all zero, and that case is left to fq_s_add_rest, as are a result below 2^-20 of x (or negative, when
+ * the high words were equal) and operands or results near the ends of the exponent range.  A y that is
+ * zero or subnormal needs no test: whatever its significand, it is far below half a place of x.
+ */
 FQ_HD double fq_s_add_words(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl, double a, double b)
 {
-    const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-    if (FQ_S_UNLIKELY(ea - 1u >= 0x7feu || eb - 1u >= 0x7feu)) {
-        return fq_s_hw_add(a, b);
-    }
-    /* X: the operand of larger magnitude (sign of |A| - |B| from a 64-bit subtraction) */
-    uint32_t dh, dl;
-    fq_s_sub64(ah & 0x7fffffffu, al, bh & 0x7fffffffu, bl, dh, dl);
-    (void)dl;
-    const bool swap = (int32_t)dh < 0;
-    const uint32_t xh = swap ? bh : ah, xl = swap ? bl : al;
-    const uint32_t yh = swap ? ah : bh, yl = swap ? al : bl;
-    const uint32_t ex = swap ? eb : ea, ey = swap ? ea : eb;
-    /* significands with the implicit bit, moved up by 10 guard bits: leading bit at 62 */
-    const uint32_t mxh = fq_s_shl64hi(xl, (xh & 0xfffffu) | 0x100000u, 10), mxl = xl << 10;
-    uint32_t myh = fq_s_shl64hi(yl, (yh & 0xfffffu) | 0x100000u, 10), myl = yl << 10;
-    /* align y by d = ex - ey (clamped to 63; y then only feeds the sticky bit) with a sticky bit */
-    uint32_t d = ex - ey;
-    d = d > 63u ? 63u : d;
-    uint32_t sticky = 0;
-    if (d >= 32u) {
-        sticky = myl;
-        myl = myh;
-        myh = 0;
-        d -= 32u;
-    }
-    sticky |= myl & ((1u << d) - 1u);
-    myl = fq_s_shr64lo(myl, myh, d) | (sticky != 0u ? 1u : 0u);
-    myh = myh >> d;
-    /* add or subtract */
+    const uint32_t A = ah & 0x7fffffffu, B = bh & 0x7fffffffu;
+    const bool swap = A < B;
+    const uint32_t X = fq_s_max(A, B), Y = fq_s_min(A, B);
+    const uint32_t xl = swap ? bl : al, yl = swap ? al : bl;
+    const uint32_t sx = swap ? bh : ah; /* sign and exponent of the result before normalisation */
+    const uint32_t mxh = (X & 0xfffffu) | 0x100000u, myh = (Y & 0xfffffu) | 0x100000u;
+    uint32_t d = (X >> 20) - (Y >> 20);
+    d = fq_s_min(d, 63u);
+    const bool far = d > 31u;
+    const uint32_t w2 = far ? 0u : myh, w1 = far ? myh : yl, w0 = far ? yl : 0u;
+    const uint32_t n = d & 31u;
+    uint32_t g = fq_s_shr64lo(w0, w1, n);
+    const uint32_t l = fq_s_shr64lo(w1, w2, n), h = w2 >> n;
     uint32_t mh, ml;
-    const bool sub = (int32_t)(xh ^ yh) < 0;
-    if (sub) {
-        fq_s_sub64(mxh, mxl, myh, myl, mh, ml);
+    fq_s_addsub96(ah ^ bh, mxh, xl, h, l, g, mh, ml);
+    /* leading bit to 53: by 0 after a carry, 1 normally, more after a cancellation */
+    const uint32_t z = fq_s_clz(mh) - 10u;
+    mh = fq_s_shl64hi(ml, mh, z);
+    ml = fq_s_shl64hi(g, ml, z);
+    g <<= (z & 31u);
+    if (FQ_S_UNLIKELY(X - 0x03800000u >= 0x7fe00000u - 0x03800000u || z > 21u || (g == 0u && w0 != 0u))) {
+        return fq_s_add_rest(a, b);
     }
-    else {
-        fq_s_add64(mxh, mxl, myh, myl, mh, ml);
-    }
-    if ((mh | ml) == 0u) {
-        return 0.0; /* exact cancellation: +0 when rounding to nearest */
-    }
-    /* normalise the leading bit to position 62: right by one on a carry, left after a cancellation */
-    int32_t e = (int32_t)ex;
-    if ((int32_t)mh < 0) {
-        ml = fq_s_shr64lo(ml, mh, 1) | (ml & 1u);
-        mh >>= 1;
-        e += 1;
-    }
-    else {
-        uint32_t lz = (mh != 0u ? fq_s_clz(mh) : 32u + fq_s_clz(ml)) - 1u;
-        e -= (int32_t)lz;
-        if (lz >= 32u) {
-            mh = ml;
-            ml = 0;
-            lz -= 32u;
-        }
-        mh = fq_s_shl64hi(ml, mh, lz);
-        ml = ml << lz;
-    }
-    if (FQ_S_UNLIKELY(e <= 0 || e >= 0x7ff)) {
-        return fq_s_hw_add(a, b);
-    }
-    /* round to nearest even on the 10 guard bits: up when guard > half, or == half and lsb odd */
-    uint32_t ql = fq_s_shr64lo(ml, mh, 10), qh = mh >> 10;
-    const uint32_t up = ((ml & 0x3ffu) + 0x1ffu + (ql & 1u)) >> 10;
-    fq_s_add64(qh, ql, 0u, up, qh, ql);
+    /* nearest even: bit 0 of ml is the rounding bit, bit 1 the last place, g what is left below */
+    uint32_t qh, ql;
+    fq_s_add64c(mh, ml, g | (ml & 2u), qh, ql);
     /* the implicit bit (and a carry out of the significand) adds into the exponent field */
-    return fq_s_make((xh & 0x80000000u) | (((uint32_t)(e - 1) << 20) + qh), ql);
+    return fq_s_make((qh >> 1) + ((sx & 0xfff00000u) - (z << 20)), fq_s_shr64lo(ql, qh, 1));
 }
 
 FQ_HD double fq_sadd(double a, double b)
@@ -239,35 +289,84 @@ FQ_HD double fq_ssub(double a, double b)
     return fq_s_add_words(fq_s_hi(a), fq_s_lo(a), bh, fq_s_lo(b), a, fq_s_make(bh, fq_s_lo(b)));
 }
 
+/*
+ * A factor prepared for fq_smulc: its significand with the leading bit at 63 (ch:cl), the range of
+ * exponent fields of the other operand for which operand and product are normal (first one, and how
+ * many, both << 21), and what is added to the other operand's sign and exponent (e).  A factor that
+ * is not normal has an empty range: the hardware multiplies.
+ */
+typedef struct {
+    uint32_t ch, cl, lo, span, e;
+    double c;
+} fq_sfactor;
+
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+static inline fq_sfactor fq_s_factor(double c)
+{
+    fq_sfactor f;
+    const uint64_t b = fq_bits(c);
+    const int ec = (int)((b >> 52) & 0x7ff);
+    const uint64_t m = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;
+    /* product's exponent field ex + ec - 1023, one more when the significands' product reaches 2 and
+     * one more when it rounds up to the next power of two */
+    const int lo = 1024 - ec < 1 ? 1 : 1024 - ec, hi = 0x7fd + 1022 - ec > 0x7fe ? 0x7fe : 0x7fd + 1022 - ec;
+    f.c = c;
+    f.ch = (uint32_t)(m >> 32);
+    f.cl = (uint32_t)m;
+    f.lo = (uint32_t)lo << 21;
+    f.span = ec == 0 || ec == 0x7ff || hi < lo ? 0u : (uint32_t)(hi - lo + 1) << 21;
+    f.e = ((uint32_t)(ec - 1023) << 20) + (uint32_t)((b >> 63) << 31);
+    return f;
+}
+
+/*
+ * x * f: the 53 x 64-bit product of the significands as 32-bit multiply-adds (without the low word of
+ * its lowest partial product), its top 53 bits in (p3:p2) and the bits below in p1.  A p1 of exactly
+ * half a place goes to the hardware (a tie, or bits below that were not formed).
+ */
+FQ_HD double fq_smulc(double x, const fq_sfactor f)
+{
+    const uint32_t xh = fq_s_hi(x), xl = fq_s_lo(x);
+    uint32_t p3, p2, p1;
+    fq_s_mul53((xh & 0xfffffu) | 0x100000u, xl, f.ch, f.cl, p3, p2, p1);
+    uint32_t t = (xh & 0xfff00000u) + f.e;
+    if (!(p3 & 0x100000u)) {
+        p3 = fq_s_shl64hi(p2, p3, 1);
+        p2 = fq_s_shl64hi(p1, p2, 1);
+        p1 <<= 1;
+        t -= 0x100000u;
+    }
+    if (FQ_S_UNLIKELY((xh << 1) - f.lo >= f.span || p1 == 0x80000000u)) {
+        return fq_s_hw_mul(x, f.c);
+    }
+    uint32_t rh, rl;
+    fq_s_round64(p3, p2, p1, t, rh, rl);
+    return fq_s_make(rh, rl);
+}
+
 FQ_HD double fq_smul(double a, double b)
 {
     const uint32_t ah = fq_s_hi(a), al = fq_s_lo(a), bh = fq_s_hi(b), bl = fq_s_lo(b);
     const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-    if (FQ_S_UNLIKELY(ea - 1u >= 0x7feu || eb - 1u >= 0x7feu)) {
-        return fq_s_hw_mul(a, b);
-    }
-    /* significands moved up by 11: leading bit at 63, product in [2^126, 2^128) */
-    const uint32_t mah = fq_s_shl64hi(al, (ah & 0xfffffu) | 0x100000u, 11), mal = al << 11;
-    const uint32_t mbh = fq_s_shl64hi(bl, (bh & 0xfffffu) | 0x100000u, 11), mbl = bl << 11;
-    uint32_t p3, p2, p1, p0;
-    fq_s_mul128(mah, mal, mbh, mbl, p3, p2, p1, p0);
-    int32_t e = (int32_t)(ea + eb) - 1022;
-    uint32_t lostw = p0 | p1;
-    if ((int32_t)p3 >= 0) {
+    uint32_t p3, p2, p1;
+    /* b's significand with its leading bit at 63 */
+    fq_s_mul53((ah & 0xfffffu) | 0x100000u, al, fq_s_shl64hi(bl, bh & 0xfffffu, 11) | 0x80000000u, bl << 11, p3, p2,
+               p1);
+    uint32_t e = ea + eb - 1023u;
+    if (!(p3 & 0x100000u)) {
         p3 = fq_s_shl64hi(p2, p3, 1);
         p2 = fq_s_shl64hi(p1, p2, 1);
-        lostw = p0 | (p1 << 1);
-        e -= 1;
+        p1 <<= 1;
+        e -= 1u;
     }
-    if (FQ_S_UNLIKELY(e <= 0 || e >= 0x7ff)) {
+    if (FQ_S_UNLIKELY(ea - 1u >= 0x7feu || eb - 1u >= 0x7feu || e >= 0x7fdu || p1 == 0x80000000u)) {
         return fq_s_hw_mul(a, b);
     }
-    /* q = (p3:p2) >> 11; guard bits p2[10:0]; sticky: the words below */
-    uint32_t ql = fq_s_shr64lo(p2, p3, 11), qh = p3 >> 11;
-    const uint32_t g = p2 & 0x7ffu;
-    const uint32_t up = (g + 0x3ffu + ((ql & 1u) | (lostw != 0u ? 1u : 0u))) >> 11;
-    fq_s_add64(qh, ql, 0u, up, qh, ql);
-    return fq_s_make(((ah ^ bh) & 0x80000000u) | (((uint32_t)(e - 1) << 20) + qh), ql);
+    uint32_t rh, rl;
+    fq_s_round64(p3, p2, p1, ((ah ^ bh) & 0x80000000u) + (e << 20), rh, rl);
+    return fq_s_make(rh, rl);
 }
 
 #endif

@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
             int64_t g = off + l0 + q;
             vr[q] = v0[g];
             ar[q] = a0[g];
-            un[q] = S_ADD(3, S_ADD(2, u0[g], S_MUL(0, s.dt, vr[q])), S_MUL(1, s.hdt2, ar[q]));
+            un[q] = S_ADD(3, S_ADD(2, u0[g], S_MULC(0, s.f_dt, s.dt, vr[q])), S_MULC(1, s.f_hdt2, s.hdt2, ar[q]));
             sh_un[threadIdx.x * PPT + q] = un[q];
         }
         __syncthreads();
@@ -405,8 +405,16 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
             }
             int64_t g = off + l;
             double up = un[q];
-            double4_32a w = s.wc[g];
-            if (!in_well(w.x, w.y, up) && is_nan_bits(up) == false &&
+            double2 wk = s.wk[g];
+            double d = S_SUB(5, wk.x, up);
+            double2 wy = make_double2(0.0, 0.0);
+            if (!surely_in_well(wk, d)) {
+                wy = s.wy[g];
+                if (is_nan_bits(up)) {
+                    sh.nan = 1;
+                }
+            }
+            if (!surely_in_well(wk, d) && !in_well(wy.x, wy.y, up) && is_nan_bits(up) == false &&
                 (__double_as_longlong(up) & 0x7fffffffffffffffLL) < 0x7ff0000000000000LL) {
                 const double* y = s.data + g * s.W;
                 bool ok = false;
@@ -426,8 +434,9 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                         int64_t gold = s.gidx[g];
                         s.cidx[g] = (int32_t)li;
                         s.gidx[g] = s.start[g] + li;
-                        w = make_wc(s, y[li], y[li + 1]);
-                        s.wc[g] = w;
+                        const double4_32a w = make_wc(s, y[li], y[li + 1]);
+                        store_well(s, g, w);
+                        d = FQ_SUB(w.z, up);
                         atomicAdd(&sh.ds, (unsigned long long)(s.gidx[g] - gold));
                         ok = true;
                     }
@@ -436,8 +445,9 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                     pending = true;
                 }
             }
-            double fp = pot_force<POT_CUSPY, SOFT>(s, w, up);
-            double ff = scale(S_SUB(4, uf, up), skf);
+            const double fp = scale(d, s.s_mu);
+            const double uff = S_SUB(4, uf, up);
+            const double ff = scale<true>(uff, skf);
             int li2 = threadIdx.x * PPT + q;
             double uL = li2 > 0 ? sh_un[li2 - 1]
                                 : (l == 0 ? FQ_ADD(FQ_ADD(u0[off + n - 1], FQ_MUL(s.dt, v0[off + n - 1])),
@@ -451,23 +461,12 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                 int64_t gr = l + 1 == n ? off : g + 1;
                 uR = FQ_ADD(FQ_ADD(u0[gr], FQ_MUL(s.dt, v0[gr])), FQ_MUL(s.hdt2, a0[gr]));
             }
-            double fi = scale(S_ADD(8, S_SUB(7, uL, scale_pow2(up, 1, 2.0)), uR), s.s_k);
-            double sfi = S_ADD(9, S_ADD(6, ff, fp), fi);
-            double v = S_ADD(11, vr[q], S_MUL(10, s.dt, ar[q]));
-            double f = S_ADD(13, sfi, S_MUL(12, s.me, v));
-            double a = scale(f, s.s_im);
-            v = S_ADD(16, vr[q], S_MUL(15, s.hdt, S_ADD(14, ar[q], a)));
-            f = S_ADD(18, sfi, S_MUL(17, s.me, v));
-            a = scale(f, s.s_im);
-            v = S_ADD(21, vr[q], S_MUL(20, s.hdt, S_ADD(19, ar[q], a)));
-            f = S_ADD(23, sfi, S_MUL(22, s.me, v));
-            a = scale(f, s.s_im);
+            const double sfi = add_ring_force<INTER_LAPLACE1D, SOFT>(s, S_ADD(6, ff, fp), uL, up, uR);
+            double v, a, f;
+            verlet_velocity<SOFT>(s, sfi, vr[q], ar[q], v, a, f);
             u1[g] = up;
             v1[g] = v;
             a1[g] = a;
-            if (is_nan_bits(up)) {
-                sh.nan = 1;
-            }
             double f2 = FQ_MUL(f, f), ff2 = FQ_MUL(ff, ff);
             if (q == 0) {
                 rf = f2;
@@ -483,7 +482,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                 int64_t l = l0 + q;
                 if (l < n) {
                     int64_t g = off + l;
-                    double4_32a w = s.wc[g];
+                    double2 w = s.wy[g];
                     if (!in_well(w.x, w.y, un[q]) &&
                         (__double_as_longlong(un[q]) & 0x7fffffffffffffffLL) < 0x7ff0000000000000LL) {
                         int k = atomicAdd(&b.run->n_regen, 1);
@@ -506,7 +505,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
             u1[g] = x;
             v1[g] = v0[g];
             a1[g] = a0[g];
-            double4_32a w = s.wc[g];
+            double2 w = s.wy[g];
             if (!in_well(w.x, w.y, x) && (__double_as_longlong(x) & 0x7fffffffffffffffLL) < 0x7ff0000000000000LL) {
                 const double* y = s.data + g * s.W;
                 bool ok = false;
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                         int64_t gold = s.gidx[g];
                         s.cidx[g] = (int32_t)li;
                         s.gidx[g] = s.start[g] + li;
-                        s.wc[g] = make_wc(s, y[li], y[li + 1]);
+                        store_well(s, g, make_wc(s, y[li], y[li + 1]));
                         atomicAdd(&sh.ds, (unsigned long long)(s.gidx[g] - gold));
                         ok = true;
                     }
@@ -548,7 +547,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
             int64_t l = l0 + q;
             if (l < n) {
                 int64_t g = off + l;
-                double du = FQ_SUB(s.wc[g].y, u0[g]);
+                double du = FQ_SUB(s.wy[g].y, u0[g]);
                 unsigned long long k = (unsigned long long)__double_as_longlong(du);
                 best = k < best ? k : best;
             }
@@ -734,7 +733,7 @@ __global__ void k_batch_init(DevSys d, const int64_t* owner_valid)
     d.cidx[g] = 0;
     d.gidx[g] = 0;
     d.acc_end[g] = acc;
-    d.wc[g] = make_wc(d, y[0], y[1]);
+    store_well(d, g, make_wc(d, y[0], y[1]));
     dev_align(d, g, 0.0);
 }
 
@@ -844,25 +843,6 @@ static int berr(fqsb_batch* h, int code, const std::string& m)
         }                                                                                                \
     } while (0)
 
-static Scale classify(double c)
-{
-    Scale sc;
-    sc.c = c;
-    sc.e = 0;
-    sc.mode = SCALE_GENERAL;
-    if (c == 1.0) {
-        sc.mode = SCALE_ONE;
-        return sc;
-    }
-    int e = 0;
-    double m = std::frexp(c, &e);
-    if (c > 0.0 && m == 0.5 && std::isnormal(c)) {
-        sc.mode = SCALE_POW2;
-        sc.e = e - 1;
-    }
-    return sc;
-}
-
 extern "C" const char* fqsb_batch_last_error(const fqsb_batch* h)
 {
     return h ? h->err.c_str() : g_batch_error.c_str();
@@ -961,7 +941,7 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
         I.tile0 = (int64_t)tile_inst.size();
         I.ntiles = nt;
         I.k_frame = c->k_frame[j];
-        I.s_kf = classify(c->k_frame[j]);
+        I.s_kf = classify_scale(c->k_frame[j]);
         I.u_frame = 0.0;
         I.phase = PH_EVT_MIN;
         I.min_key = 0x7ff0000000000000ULL;
@@ -993,10 +973,14 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     d.me = -c->eta;
     d.m = c->m;
     d.inv_m = 1.0 / c->m;
-    d.s_mu = classify(d.mu);
-    d.s_k = classify(d.k);
-    d.s_kf = classify(1.0);
-    d.s_im = classify(d.inv_m);
+    d.s_mu = classify_scale(d.mu);
+    d.s_k = classify_scale(d.k);
+    d.s_kf = classify_scale(1.0);
+    d.s_im = classify_scale(d.inv_m);
+    d.f_dt = fq_s_factor(d.dt);
+    d.f_hdt = fq_s_factor(d.hdt);
+    d.f_hdt2 = fq_s_factor(d.hdt2);
+    d.f_me = fq_s_factor(d.me);
     d.W = c->window;
     d.n0 = c->nchunk;
     d.dist = dist;
@@ -1035,7 +1019,8 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     BA(d.start, N);
     BA(d.cidx, N);
     BA(d.gidx, N);
-    BA(d.wc, N);
+    BA(d.wy, N);
+    BA(d.wk, N);
     BA(d.acc_end, N);
     BA(d.anc_kind, N);
     BA(d.anc_k, N);

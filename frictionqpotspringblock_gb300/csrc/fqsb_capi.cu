@@ -126,7 +126,7 @@ __global__ void k_init_chunk(DevSys d)
     d.cidx[p] = 0;
     d.gidx[p] = 0;
     d.acc_end[p] = acc;
-    d.wc[p] = make_wc(d, y[0], y[1]);
+    store_well(d, p, make_wc(d, y[0], y[1]));
 }
 
 __global__ void k_align(DevSys d, const double* u)
@@ -152,7 +152,7 @@ __global__ void k_advance(DevSys d, double* u, double du)
 __device__ __forceinline__ void pi_force(const DevSys& d, const double* u, int64_t p, double& fp, double& fi)
 {
     double up = u[p];
-    double4_32a w = d.wc[p];
+    double4_32a w = load_well(d, p);
     switch (d.pot) {
         case POT_CUSPY: fp = pot_force<POT_CUSPY>(d, w, up); break;
         case POT_SEMISMOOTH: fp = pot_force<POT_SEMISMOOTH>(d, w, up); break;
@@ -308,7 +308,7 @@ __global__ void k_min_du(DevSys d, const double* u, int direction, unsigned long
         return;
     }
     double up = u[p];
-    double4_32a w = d.wc[p];
+    double4_32a w = load_well(d, p);
     double du;
     if (d.pot == POT_CUSPY) {
         du = direction > 0 ? FQ_SUB(w.y, up) : FQ_SUB(up, w.x);
@@ -327,7 +327,7 @@ __global__ void k_min_du(DevSys d, const double* u, int direction, unsigned long
 /* Cuspy::trigger :193-205 / SemiSmooth :339-350 / Smooth :427-438 (after the align, if any) */
 __global__ void k_trigger(DevSys d, double* u, int64_t p, double eps, int direction)
 {
-    double4_32a w = d.wc[p];
+    double4_32a w = load_well(d, p);
     if (direction > 0) {
         u[p] = FQ_ADD(w.y, FQ_MUL(0.5, eps));
     }
@@ -387,7 +387,7 @@ __global__ void k_restore(DevSys d, const uint64_t* state, const double* value, 
     d.cidx[p] = 0;
     d.gidx[p] = index[p];
     d.acc_end[p] = acc;
-    d.wc[p] = make_wc(d, y[0], y[1]);
+    store_well(d, p, make_wc(d, y[0], y[1]));
 }
 
 __global__ void k_cidx64(const int32_t* c, int64_t* out, int64_t n)
@@ -398,11 +398,11 @@ __global__ void k_cidx64(const int32_t* c, int64_t* out, int64_t n)
     }
 }
 
-__global__ void k_wc_lr(const double4_32a* wc, double* left, double* right, int64_t n)
+__global__ void k_well_lr(const double2* wy, double* left, double* right, int64_t n)
 {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p < n) {
-        double4_32a w = wc[p];
+        double2 w = wy[p];
         left[p] = w.x;
         right[p] = w.y;
     }
@@ -433,27 +433,6 @@ static uint64_t host_pcg_advance(uint64_t state, uint64_t delta)
 }
 
 /* ------------------------------------------------------------ helpers */
-
-/* How the kernels multiply by a parameter c: skip for 1, exponent add for a positive normal power of
- * two, fp64 multiply otherwise (all three give x * c exactly as IEEE multiplication does). */
-static Scale classify_scale(double c)
-{
-    Scale sc;
-    sc.c = c;
-    sc.e = 0;
-    sc.mode = SCALE_GENERAL;
-    if (c == 1.0) {
-        sc.mode = SCALE_ONE;
-        return sc;
-    }
-    int e = 0;
-    double m = std::frexp(c, &e);
-    if (c > 0.0 && m == 0.5 && std::isnormal(c)) {
-        sc.mode = SCALE_POW2;
-        sc.e = e - 1;
-    }
-    return sc;
-}
 
 /* state arrays are padded so that a CTA's vector loads of a partial last tile stay in bounds */
 static int64_t padded(int64_t n)
@@ -805,7 +784,7 @@ static void free_all(fqsb_system* h)
         return;
     }
     DevSys& d = h->d;
-    void* ptrs[] = {d.data, d.nx, d.nx_end, d.start, d.cidx, d.gidx, d.wc, d.acc_end, d.anc_kind, d.anc_k, d.anc_state, d.anc_val,
+    void* ptrs[] = {d.data, d.nx, d.nx_end, d.start, d.cidx, d.gidx, d.wy, d.wk, d.acc_end, d.anc_kind, d.anc_k, d.anc_state, d.anc_val,
                     d.u[0], d.u[1], d.v[0], d.v[1], d.a[0], d.a[1], d.ctl, d.ring, d.partials, d.i_n, d.sq2,
                     d.cta_pending, d.regen_list, (void*)d.lr_pref, d.f_th, d.th_next, (void*)d.th_dinc, d.th_cnt,
                     d.th_list, d.th,
@@ -959,6 +938,10 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     d.s_k = classify_scale(d.k);
     d.s_kf = classify_scale(d.k_frame);
     d.s_im = classify_scale(d.inv_m);
+    d.f_dt = fq_s_factor(d.dt);
+    d.f_hdt = fq_s_factor(d.hdt);
+    d.f_hdt2 = fq_s_factor(d.hdt2);
+    d.f_me = fq_s_factor(d.me);
     h->lg = line_geometry(N);
     {
         /* small Line1d / Particles systems: whole runs in one thread-block cluster */
@@ -998,7 +981,8 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     ALLOC(d.start, sizeof(int64_t) * (size_t)N);
     ALLOC(d.cidx, sizeof(int32_t) * (size_t)N);
     ALLOC(d.gidx, sizeof(int64_t) * (size_t)N);
-    ALLOC(d.wc, sizeof(double4_32a) * (size_t)N);
+    ALLOC(d.wy, sizeof(double2) * (size_t)padded(N));
+    ALLOC(d.wk, sizeof(double2) * (size_t)padded(N));
     ALLOC(d.acc_end, nd);
     ALLOC(d.anc_kind, (size_t)N);
     ALLOC(d.anc_k, sizeof(int64_t) * (size_t)N);
@@ -1860,7 +1844,7 @@ extern "C" int fqsb_get_index(fqsb_system* h, int64_t* index_at_align, int64_t* 
         double* r = nullptr;
         CU(h, cudaMallocAsync((void**)&l, sizeof(double) * (size_t)N, h->stream));
         CU(h, cudaMallocAsync((void**)&r, sizeof(double) * (size_t)N, h->stream));
-        k_wc_lr<<<blocks_for(N, 256), 256, 0, h->stream>>>(h->d.wc, l, r, N);
+        k_well_lr<<<blocks_for(N, 256), 256, 0, h->stream>>>(h->d.wy, l, r, N);
         CU(h, cudaGetLastError());
         if (left_of_align) {
             CU(h, cudaMemcpyAsync(left_of_align, l, sizeof(double) * (size_t)N, cudaMemcpyDeviceToHost, h->stream));
@@ -1954,7 +1938,7 @@ __global__ void k_rewell(DevSys d)
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p < d.N) {
         const double* y = d.data + p * d.W + d.cidx[p];
-        d.wc[p] = make_wc(d, y[0], y[1]);
+        store_well(d, p, make_wc(d, y[0], y[1]));
     }
 }
 
@@ -1971,6 +1955,7 @@ extern "C" int fqsb_set_parameters(fqsb_system* h, double mu, double k_interacti
     h->cfg.eta = eta;
     h->d.s_mu = classify_scale(mu);
     h->d.s_k = classify_scale(k_interactions);
+    h->d.f_me = fq_s_factor(h->d.me);
     /* the cached well constants of SemiSmooth depend on mu */
     k_rewell<<<blocks_for(h->d.N, 256), 256, 0, h->stream>>>(h->d);
     CU(h, cudaGetLastError());

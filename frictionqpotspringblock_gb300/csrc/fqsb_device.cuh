@@ -27,6 +27,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "fq_math.h"
 #include "fq_soft64.h"
 
@@ -165,7 +167,30 @@ struct Scale {
     int mode; /* SCALE_* */
     int e;    /* c = 2^e when mode == SCALE_POW2 */
     double c;
+    fq_sfactor f; /* c for the integer-pipe multiplication */
 };
+
+/* How the kernels multiply by a parameter c: skip for 1, exponent add for a positive normal power of
+ * two, a multiplication otherwise (all three give x * c exactly as IEEE multiplication does). */
+inline Scale classify_scale(double c)
+{
+    Scale sc;
+    sc.c = c;
+    sc.e = 0;
+    sc.f = fq_s_factor(c);
+    sc.mode = SCALE_GENERAL;
+    if (c == 1.0) {
+        sc.mode = SCALE_ONE;
+        return sc;
+    }
+    int e = 0;
+    double m = std::frexp(c, &e);
+    if (c > 0.0 && m == 0.5 && std::isnormal(c)) {
+        sc.mode = SCALE_POW2;
+        sc.e = e - 1;
+    }
+    return sc;
+}
 
 struct DevSys {
     int64_t N, rows, cols;
@@ -177,6 +202,7 @@ struct DevSys {
     const double* lr_pref; /* LongRange1d: k / d^(alpha + 1) by ring distance d (0 at d = 0), host std::pow */
     int64_t lr_m;          /* LongRange1d: ring distances above lr_m wrap to N - d */
     Scale s_mu, s_k, s_kf, s_im; /* mu, k_interactions, k_frame, 1/m */
+    fq_sfactor f_dt, f_hdt, f_hdt2, f_me; /* dt, hdt, hdt2 and me for the integer-pipe multiplication */
     /* chunk */
     int64_t W, n0;
     int dist, npar;
@@ -190,7 +216,8 @@ struct DevSys {
     int64_t* start;
     int32_t* cidx;
     int64_t* gidx;
-    double4_32a* wc;
+    double2* wy; /* current well: (y_left, y_right) */
+    double2* wk; /* and its constants (make_wc): all that a Cuspy step reads of the well */
     double* acc_end;
     double* nx;      /* next-window buffer [N, W] of small systems (next_window_ready), or NULL */
     int64_t* nx_end; /* window end the buffer of particle p follows */
@@ -450,7 +477,12 @@ __device__ __forceinline__ void walker_next(const DevSys& s, Walker& w)
     w.k = k;
 }
 
-/* Refresh the cached well of particle p from its chunk row at chunk index li. */
+/*
+ * The cached well between yield positions yl and yr.  z, w: SemiSmooth u_l, u_r; Smooth centre and half
+ * width; Cuspy centre c and a width s with the guarantee that |RN(c - u)| < s puts u inside the well,
+ * yl <= u < yr: the half width less 2^-50 (|yl| + |yr|), which covers the roundings of c, of the half
+ * width and of c - u (together below 2^-51 (|yl| + |yr|)); 0 when nothing is left.
+ */
 __device__ __forceinline__ double4_32a make_wc(const DevSys& s, double yl, double yr)
 {
     double4_32a w;
@@ -464,15 +496,31 @@ __device__ __forceinline__ double4_32a make_wc(const DevSys& s, double yl, doubl
     }
     else {
         w.z = FQ_MUL(0.5, FQ_ADD(yl, yr)); /* well centre */
-        w.w = FQ_MUL(0.5, FQ_SUB(yr, yl)); /* half width (Smooth) */
+        w.w = FQ_MUL(0.5, FQ_SUB(yr, yl)); /* half width */
+        if (s.pot == POT_CUSPY) {
+            const double safe = FQ_SUB(w.w, FQ_MUL(0x1p-50, FQ_ADD(fabs(yl), fabs(yr))));
+            w.w = safe > 0.0 ? safe : 0.0;
+        }
     }
     return w;
+}
+
+__device__ __forceinline__ double4_32a load_well(const DevSys& s, int64_t p)
+{
+    const double2 y = s.wy[p], k = s.wk[p];
+    return make_double4_32a(y.x, y.y, k.x, k.y);
+}
+
+__device__ __forceinline__ void store_well(const DevSys& s, int64_t p, const double4_32a& w)
+{
+    s.wy[p] = make_double2(w.x, w.y);
+    s.wk[p] = make_double2(w.z, w.w);
 }
 
 /*
  * prrng align for particle p at target u: find i with y[i] <= u < y[i+1]; when i leaves
  * [min_margin, W - buffer) move the window so that the target sits at chunk index `margin`.
- * Updates start, cidx, gidx, wc, acc_end of the particle.  Returns false for a non-finite u
+ * Updates start, cidx, gidx, the cached well and acc_end of the particle.  Returns false for a non-finite u
  * (the index is then kept; the NaN is reported by the step's NaN check).
  */
 static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double u)
@@ -503,7 +551,7 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
         if (li >= s.min_margin && li < W - s.buffer) {
             s.cidx[p] = (int32_t)li;
             s.gidx[p] = start + li;
-            s.wc[p] = make_wc(s, y[li], y[li + 1]);
+            store_well(s, p, make_wc(s, y[li], y[li + 1]));
             return true;
         }
         gi = start + li;
@@ -618,7 +666,7 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
     li = s.margin;
     s.cidx[p] = (int32_t)li;
     s.gidx[p] = ns + li;
-    s.wc[p] = make_wc(s, y[li], y[li + 1]);
+    store_well(s, p, make_wc(s, y[li], y[li + 1]));
     return true;
 }
 
@@ -797,7 +845,7 @@ __device__ __forceinline__ void fwd_move_sum(const DevSys& s, const FwdMove& m)
     const int64_t li = s.margin;
     s.cidx[p] = (int32_t)li;
     s.gidx[p] = m.ns + li;
-    s.wc[p] = make_wc(s, y[li], y[li + 1]);
+    store_well(s, p, make_wc(s, y[li], y[li + 1]));
 }
 
 /*
@@ -879,7 +927,7 @@ __device__ __forceinline__ void fwd_move_finish(const DevSys& s, const FwdMove& 
     const int64_t li = s.margin;
     s.cidx[p] = (int32_t)li;
     s.gidx[p] = m.ns + li;
-    s.wc[p] = make_wc(s, y[li], y[li + 1]);
+    store_well(s, p, make_wc(s, y[li], y[li + 1]));
 }
 
 /* ------------------------------------------- exact integer-pipe helpers */
@@ -905,22 +953,24 @@ __device__ __forceinline__ bool in_well(double yl, double yr, double u)
  * Per-operation choice of unit.  Bit i of SOFT set: operation site i of the particle update runs on
  * the integer pipes (fq_soft64.h, bit-identical to the hardware instruction); clear: on the fp64
  * pipe.  Sites: 0 dt*v, 1 hdt2*a, 2 u+dt*v, 3 +hdt2*a (position); 4 u_frame-u', 5 c-u' (Cuspy),
- * 6 f_frame+f_pot, 7 uL-2u', 8 +uR, 9 +f_int (forces); 10 dt*a0, 11 v0+dt*a0, 12 -eta*v, 13 s+(-eta*v)
+ * 6 f_frame+f_pot, 7 and 8 the neighbours' sum, 9 +f_int (forces); 10 dt*a0, 11 v0+dt*a0, 12 -eta*v, 13 s+(-eta*v)
  * (first velocity update); 14 a0+a, 15 hdt*(a0+a), 16 v0+hdt*(..), 17 -eta*v, 18 s+(-eta*v) (second)
  * and 19..23 the same for the third.
  */
 #define S_ADD(bit, a, b) (((SOFT >> (bit)) & 1u) ? fq_sadd((a), (b)) : FQ_ADD((a), (b)))
 #define S_SUB(bit, a, b) (((SOFT >> (bit)) & 1u) ? fq_ssub((a), (b)) : FQ_SUB((a), (b)))
-#define S_MUL(bit, a, b) (((SOFT >> (bit)) & 1u) ? fq_smul((a), (b)) : FQ_MUL((a), (b)))
+/* c * x for a parameter c with its prepared factor f */
+#define S_MULC(bit, f, c, x) (((SOFT >> (bit)) & 1u) ? fq_smulc((x), (f)) : FQ_MUL((c), (x)))
 
 /*
- * The split the step kernels use: all eight multiplications and the two additions of the position
- * update on the integer pipes, the other fourteen additions on the fp64 pipe.  Measured on the
- * N = 2^22 flow workload against other splits (all multiplications only; also the velocity or the
- * force additions): 20.2 G particle-steps/s against 19.2-20.2 for the others and 14.8 with none.
+ * The split the step kernels use: the eight multiplications, the two additions of the position update and
+ * a0 + a of the last two velocity updates on the integer pipes, the other twelve additions on the fp64
+ * pipe.  Of the splits measured on the N = 2^22 flow step (159 us) the neighbours are: without 14 and
+ * 19 172 us; with 4 and 5 instead 161 us; with 4 as well 160 us; with 11 as well 162 us; with 4, 5 and
+ * 11 as well 169 us; the multiplications alone 180 us.
  */
-constexpr unsigned STEP_SOFT = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 10) | (1u << 12) | (1u << 15) |
-                               (1u << 17) | (1u << 20) | (1u << 22);
+constexpr unsigned STEP_SOFT = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 10) | (1u << 12) | (1u << 14) |
+                               (1u << 15) | (1u << 17) | (1u << 19) | (1u << 20) | (1u << 22);
 
 /* fp64 add / mul for work inside a run-time branch (residual and frame-force sums): volatile, so the
  * compiler cannot execute them speculatively before the branch, as it does with the plain forms. */
@@ -958,7 +1008,8 @@ __device__ __forceinline__ double scale_pow2(double x, int e, double c)
     return FQ_MUL(x, c);
 }
 
-/* x * c with c described by sc (c > 0 for the power-of-two forms). */
+/* x * c with c described by sc (c > 0 for the power-of-two forms); SOFT: a general c on the integer pipes. */
+template <bool SOFT = false>
 __device__ __forceinline__ double scale(double x, const Scale& sc)
 {
     if (sc.mode == SCALE_ONE) {
@@ -967,15 +1018,39 @@ __device__ __forceinline__ double scale(double x, const Scale& sc)
     if (sc.mode == SCALE_POW2) {
         return scale_pow2(x, sc.e, sc.c);
     }
-    return FQ_MUL(x, sc.c);
+    return SOFT ? fq_smulc(x, sc.f) : FQ_MUL(x, sc.c);
+}
+
+/* x * c + y with two roundings, as scale() followed by an addition.  A power of two scales exactly, so one
+ * fma does both (the fp64 pipe takes it in the cycles of the addition).  SOFT: general c on the integer pipes. */
+template <bool SOFT>
+__device__ __forceinline__ double scale_add(double x, const Scale& sc, double y)
+{
+    if (sc.mode != SCALE_GENERAL) {
+        return FQ_FMA(x, sc.c, y);
+    }
+    return FQ_ADD(SOFT ? fq_smulc(x, sc.f) : FQ_MUL(x, sc.c), y);
+}
+
+/* x + 0 (f_interactions of a system without interactions): only a -0 changes */
+__device__ __forceinline__ double add_zero(double x)
+{
+    return fq_s_hi(x) == 0x80000000u && fq_s_lo(x) == 0u ? 0.0 : x;
+}
+
+/* Whether u lies in the Cuspy well with constants k (make_wc), from d = RN(centre - u): the high words
+ * decide; false also when they cannot tell (within 2^-20 of the half width), and for a NaN. */
+__device__ __forceinline__ bool surely_in_well(const double2& k, double d)
+{
+    return (fq_s_hi(d) & 0x7fffffffu) < fq_s_hi(k.y);
 }
 
 /* Potential force, Cuspy detail.h:139-170 / SemiSmooth :236-277 / Smooth :379-409. */
-template <int POT, unsigned SOFT = 0u>
+template <int POT>
 __device__ __forceinline__ double pot_force(const DevSys& s, const double4_32a& w, double up)
 {
     if (POT == POT_CUSPY) {
-        return scale((SOFT >> 5) & 1u ? fq_ssub(w.z, up) : FQ_SUB(w.z, up), s.s_mu);
+        return scale(FQ_SUB(w.z, up), s.s_mu);
     }
     else if (POT == POT_SEMISMOOTH) {
         if (up < w.z) {
@@ -993,6 +1068,30 @@ __device__ __forceinline__ double pot_force(const DevSys& s, const double4_32a& 
     }
 }
 
+/* f = (sfi + f_damping) [+ f_thermal]: computeForce, detail.h:1321-1330 */
+template <bool TH>
+__device__ __forceinline__ double with_thermal(double f, double fth)
+{
+    return TH ? __dadd_rn(f, fth) : f;
+}
+
+/* velocity / acceleration updates of timeStep after the positions, detail.h:1552-1565 (TH: with the
+ * thermal force of RandomNormalForcing as the last term of each force sum) */
+template <unsigned SOFT = 0u, bool TH = false>
+__device__ __forceinline__ void verlet_velocity(const DevSys& s, double sfi, double v0, double a0, double& v, double& a,
+                                                double& f, double fth = 0.0)
+{
+    v = S_ADD(11, v0, S_MULC(10, s.f_dt, s.dt, a0));
+    f = with_thermal<TH>(S_ADD(13, sfi, S_MULC(12, s.f_me, s.me, v)), fth);
+    a = scale<SOFT != 0u>(f, s.s_im);
+    v = S_ADD(16, v0, S_MULC(15, s.f_hdt, s.hdt, S_ADD(14, a0, a)));
+    f = with_thermal<TH>(S_ADD(18, sfi, S_MULC(17, s.f_me, s.me, v)), fth);
+    a = scale<SOFT != 0u>(f, s.s_im);
+    v = S_ADD(21, v0, S_MULC(20, s.f_hdt, s.hdt, S_ADD(19, a0, a)));
+    f = with_thermal<TH>(S_ADD(23, sfi, S_MULC(22, s.f_me, s.me, v)), fth);
+    a = scale<SOFT != 0u>(f, s.s_im);
+}
+
 /* ------------------------------------------------ interactions */
 
 /*
@@ -1000,13 +1099,12 @@ __device__ __forceinline__ double pot_force(const DevSys& s, const double4_32a& 
  * Laplace1d detail.h:474-487 ((uL - 2u) + uR, then times k); Quartic1d :781-803
  * (a1 ((uL - 2u) + uR) + a2 ((dup dup) dup + (dun dun) dun), dup = uR - u, dun = uL - u);
  * QuarticGradient1d :636-650 (((uL - 2u) + uR) (k2 + (k4/4 du) du), du = uR - uL).
- * SOFT selects the integer-pipe forms of the Laplace1d operations (sites 7, 8).
  */
-template <int INTER, unsigned SOFT = 0u>
+template <int INTER>
 __device__ __forceinline__ double ring_force(const DevSys& s, double uL, double u, double uR)
 {
     if (INTER == INTER_LAPLACE1D) {
-        return scale(S_ADD(8, S_SUB(7, uL, scale_pow2(u, 1, 2.0)), uR), s.s_k);
+        return scale(FQ_ADD(FQ_SUB(uL, scale_pow2(u, 1, 2.0)), uR), s.s_k);
     }
     const double lap = FQ_ADD(FQ_SUB(uL, scale_pow2(u, 1, 2.0)), uR);
     if (INTER == INTER_QUARTIC1D) {
@@ -1016,6 +1114,18 @@ __device__ __forceinline__ double ring_force(const DevSys& s, double uL, double 
     }
     const double du = FQ_SUB(uR, uL);
     return FQ_MUL(lap, FQ_ADD(s.ia, FQ_MUL(FQ_MUL(s.k4_4, du), du)));
+}
+
+/* f + f_interactions on a ring, in the step's operations (sites 8, 9): 2 u and a power-of-two k are exact,
+ * so uL - 2 u and f + k (...) are one fma each (SOFT = 0, where latency counts: separately, so that 2 u is
+ * ready before uL arrives). */
+template <int INTER, unsigned SOFT>
+__device__ __forceinline__ double add_ring_force(const DevSys& s, double f, double uL, double u, double uR)
+{
+    if (INTER == INTER_LAPLACE1D && SOFT != 0u) {
+        return scale_add<true>(S_ADD(8, FQ_FMA(u, -2.0, uL), uR), s.s_k, f);
+    }
+    return S_ADD(9, f, ring_force<INTER>(s, uL, u, uR));
 }
 
 /*

@@ -27,14 +27,19 @@
  *
  * State is double buffered (u, v, a)[cur] -> (u, v, a)[cur ^ 1].  Arithmetic uses explicit
  * __dadd_rn / __dmul_rn in the reference's order (no fma contraction), so results equal the CPU
- * oracle bit for bit.  Only exact rewrites save fp64 issue slots (the fp64 pipe, ~1.6 instructions
- * per clock per SM on GB300, is the binding unit):
+ * oracle bit for bit.  Only exact rewrites save fp64 issue slots (the fp64 pipe, 1.68 operations per
+ * clock per SM on GB300, is the binding unit):
  *   - the partial sum f_frame + f_potential + f_interactions is formed once per step (it is the
  *     same in every computeForce of the step);
- *   - multiplications by parameters equal to 1 are skipped, and multiplications by powers of two
- *     (2 u, 4 u, and e.g. k_frame = 2^-22) are exponent adds on the integer pipe when the result
- *     stays normal;
- *   - the well test yl <= u < yr and the NaN test run on order-preserving integer keys.
+ *   - multiplications by parameters equal to 1 are skipped; a product by a power of two is exact, so where
+ *     it only feeds an addition (2 u, 4 u, and f_frame, f_interactions with k_frame or k a power of two)
+ *     one fma does both;
+ *   - the NaN test and, where it is needed at all, the well test yl <= u < yr run on order-preserving
+ *     integer keys; a Cuspy particle is first tested against its well's centre and half width, which
+ *     reads 16 bytes of the well instead of 32 and takes 2 instructions.
+ * Measured at N = 2^22 (Line1d Cuspy, kernel alone): 193 us per step with the sums formed separately, the
+ * well test on keys always and the previous integer-pipe operations, 159 us as it is; the 2048 x 2048
+ * grid 229 and 195 us.
  */
 #include "fqsb_internal.h"
 
@@ -57,40 +62,26 @@ template <unsigned SOFT = 0u>
 __device__ __forceinline__ double u_next(const DevSys& s, const double* u0, const double* v0, const double* a0,
                                          int64_t q)
 {
-    return S_ADD(3, S_ADD(2, u0[q], S_MUL(0, s.dt, v0[q])), S_MUL(1, s.hdt2, a0[q]));
+    return S_ADD(3, S_ADD(2, u0[q], S_MULC(0, s.f_dt, s.dt, v0[q])), S_MULC(1, s.f_hdt2, s.hdt2, a0[q]));
 }
 
-/* f = (sfi + f_damping) [+ f_thermal]: computeForce, detail.h:1321-1330 */
-template <bool TH>
-__device__ __forceinline__ double with_thermal(double f, double fth)
-{
-    return TH ? __dadd_rn(f, fth) : f;
-}
-
-/* velocity / acceleration updates of timeStep after the positions, detail.h:1552-1565 (TH: with the
- * thermal force of RandomNormalForcing as the last term of each force sum) */
-template <unsigned SOFT = 0u, bool TH = false>
-__device__ __forceinline__ void verlet_velocity(const DevSys& s, double sfi, double v0, double a0, double& v, double& a,
-                                                double& f, double fth = 0.0)
-{
-    v = S_ADD(11, v0, S_MUL(10, s.dt, a0));
-    f = with_thermal<TH>(S_ADD(13, sfi, S_MUL(12, s.me, v)), fth);
-    a = scale(f, s.s_im);
-    v = S_ADD(16, v0, S_MUL(15, s.hdt, S_ADD(14, a0, a)));
-    f = with_thermal<TH>(S_ADD(18, sfi, S_MUL(17, s.me, v)), fth);
-    a = scale(f, s.s_im);
-    v = S_ADD(21, v0, S_MUL(20, s.hdt, S_ADD(19, a0, a)));
-    f = with_thermal<TH>(S_ADD(23, sfi, S_MUL(22, s.me, v)), fth);
-    a = scale(f, s.s_im);
-}
-
-/* (f_frame + f_potential) of the force sum, and f_frame itself */
+/*
+ * The force sum of a particle without interactions and damping, f_frame + f_potential, and f_frame itself.
+ * d: centre - u of a Cuspy well (the others take w).  k_frame is most often a power of two or general:
+ * for a power of two f_frame is exact and one fma forms the sum (site 6; where f_frame is also needed and
+ * latency counts, SOFT = 0, the sum is formed from it).
+ */
 template <int POT, unsigned SOFT = 0u>
-__device__ __forceinline__ double frame_pot(const DevSys& s, const double4_32a& w, double up, double uf, double& ff)
+__device__ __forceinline__ double frame_pot(const DevSys& s, const double4_32a& w, double d, double up, double uf,
+                                            double& ff)
 {
-    double fp = pot_force<POT, SOFT>(s, w, up);
-    ff = scale(S_SUB(4, uf, up), s.s_kf);
-    return S_ADD(6, ff, fp);
+    const double fp = POT == POT_CUSPY ? scale<SOFT != 0u>(d, s.s_mu) : pot_force<POT>(s, w, up);
+    const double x = S_SUB(4, uf, up);
+    ff = scale<SOFT != 0u>(x, s.s_kf);
+    if (SOFT == 0u) {
+        return FQ_ADD(ff, fp);
+    }
+    return s.s_kf.mode != SCALE_GENERAL ? FQ_FMA(x, s.s_kf.c, fp) : S_ADD(6, ff, fp);
 }
 
 __device__ __forceinline__ long long absll(long long x)
@@ -332,7 +323,7 @@ __device__ __forceinline__ bool window_search(const DevSys& s, int64_t p, double
     s.cidx[p] = (int32_t)li;
     s.gidx[p] = s.start[p] + li;
     w = make_wc(s, y[li], y[li + 1]);
-    s.wc[p] = w;
+    store_well(s, p, w);
     return true;
 }
 
@@ -342,14 +333,32 @@ __device__ __forceinline__ bool non_finite(double x)
 }
 
 /*
- * Per-particle well check of the cached well w (particle p's record, loaded by the caller); returns the
- * (possibly refreshed) well cache.  `regen` is set when the particle's chunk window must move; the
- * pass-1 caller then marks its CTA pending.
+ * Well check of particle p at its new position un, from the constants wk of its cached well (loaded by the
+ * caller).  Cuspy: d = centre - un, which the force needs anyway, also tells that the particle stays in
+ * its well without reading the yield positions; only where it cannot tell is the exact test made (and
+ * un looked at for a NaN, which d carries).  The other potentials read the yield positions always.
+ * Returns the (possibly new) well, its yield positions unset where the Cuspy test sufficed.  `regen` is set
+ * when the chunk window must move; the pass-1 caller then marks its CTA pending.
  */
+template <int POT, unsigned SOFT = 0u>
 __device__ __forceinline__ double4_32a well_of(const DevSys& s, int64_t p, double un, bool act, StepShared& sh,
-                                               bool& regen, double4_32a w)
+                                               double2 wk, double& d, bool& regen)
 {
     regen = false;
+    double4_32a w = make_double4_32a(0.0, 0.0, wk.x, wk.y);
+    d = 0.0;
+    if (POT == POT_CUSPY) {
+        d = S_SUB(5, wk.x, un);
+        if (surely_in_well(wk, d)) {
+            return w;
+        }
+    }
+    const double2 wy = s.wy[p];
+    w.x = wy.x;
+    w.y = wy.y;
+    if (is_nan_bits(un)) {
+        sh.nan = 1;
+    }
     if (!in_well(w.x, w.y, un) && !non_finite(un)) {
         int64_t gold = s.gidx[p];
         if (window_search(s, p, un, w)) {
@@ -361,18 +370,15 @@ __device__ __forceinline__ double4_32a well_of(const DevSys& s, int64_t p, doubl
                 atomicAdd(&sh.ds, (unsigned long long)ds);
                 atomicAdd(&sh.da, (unsigned long long)da);
             }
+            if (POT == POT_CUSPY) {
+                d = FQ_SUB(w.z, un);
+            }
         }
         else {
             regen = true;
         }
     }
     return w;
-}
-
-__device__ __forceinline__ double4_32a well_of(const DevSys& s, int64_t p, double un, bool act, StepShared& sh,
-                                               bool& regen)
-{
-    return well_of(s, p, un, act, sh, regen, s.wc[p]);
 }
 
 /* Role of the CTA epilogue in the step's kernels. */
@@ -505,12 +511,10 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
     double un[PPT], vr[PPT], ar[PPT];
     /* the cached wells are loaded together with the state, so that their latency overlaps the
      * position update and the neighbour exchange instead of following them */
-    double4_32a wpre[PPT];
+    double2 wpre[PPT];
 #pragma unroll
     for (int j = 0; j < PPT; ++j) {
-        if (p0 + j < N) {
-            wpre[j] = s.wc[p0 + j];
-        }
+        wpre[j] = s.wk[p0 + j];
     }
     if (PPT == 2) {
         double2 uu = *reinterpret_cast<const double2*>(u0 + p0);
@@ -520,15 +524,16 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
         vr[PPT - 1] = vv.y;
         ar[0] = aa.x;
         ar[PPT - 1] = aa.y;
-        un[0] = S_ADD(3, S_ADD(2, uu.x, S_MUL(0, s.dt, vr[0])), S_MUL(1, s.hdt2, ar[0]));
-        un[PPT - 1] = S_ADD(3, S_ADD(2, uu.y, S_MUL(0, s.dt, vr[PPT - 1])), S_MUL(1, s.hdt2, ar[PPT - 1]));
+        un[0] = S_ADD(3, S_ADD(2, uu.x, S_MULC(0, s.f_dt, s.dt, vr[0])), S_MULC(1, s.f_hdt2, s.hdt2, ar[0]));
+        un[PPT - 1] = S_ADD(3, S_ADD(2, uu.y, S_MULC(0, s.f_dt, s.dt, vr[PPT - 1])),
+                            S_MULC(1, s.f_hdt2, s.hdt2, ar[PPT - 1]));
     }
     else {
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {
             vr[j] = v0[p0 + j];
             ar[j] = a0[p0 + j];
-            un[j] = S_ADD(3, S_ADD(2, u0[p0 + j], S_MUL(0, s.dt, vr[j])), S_MUL(1, s.hdt2, ar[j]));
+            un[j] = S_ADD(3, S_ADD(2, u0[p0 + j], S_MULC(0, s.f_dt, s.dt, vr[j])), S_MULC(1, s.f_hdt2, s.hdt2, ar[j]));
         }
     }
     if (inter_ring(INTER)) {
@@ -546,7 +551,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
         __syncthreads();
     }
     double rf = 0.0, rff = 0.0;
-    bool nan = false, pending = false;
+    bool pending = false;
     double vo[PPT], ao[PPT];
 #pragma unroll
     for (int j = 0; j < PPT; ++j) {
@@ -558,21 +563,22 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
         }
         double up = un[j];
         bool regen;
-        double4_32a w = well_of(s, p, up, act, sh, regen, wpre[j]);
+        double d;
+        double4_32a w = well_of<POT, SOFT>(s, p, up, act, sh, wpre[j], d, regen);
         pending |= regen;
         double ff;
-        double sfp = frame_pot<POT, SOFT>(s, w, up, uf, ff);
-        double fi = 0.0;
+        double sfi = frame_pot<POT, SOFT>(s, w, d, up, uf, ff);
         if (inter_ring(INTER)) {
             int li = threadIdx.x * PPT + j;
             double uL = li > 0 ? sh_un[li - 1] : sh_halo[0];
             double uR = (li + 1 < T * PPT && p + 1 < N) ? sh_un[li + 1] : sh_halo[1];
-            fi = ring_force<INTER, SOFT>(s, uL, up, uR);
+            sfi = add_ring_force<INTER, SOFT>(s, sfi, uL, up, uR);
         }
-        double sfi = S_ADD(9, sfp, fi);
+        else {
+            sfi = add_zero(sfi);
+        }
         double f;
         verlet_velocity<SOFT, TH>(s, sfi, vr[j], ar[j], vo[j], ao[j], f, TH ? s.f_th[p] : 0.0);
-        nan |= is_nan_bits(up);
         if (resid) {
             /* squares on the integer pipes (bit-identical), sums on the fp64 pipe */
             double f2 = fq_smul(f, f), ff2 = fq_smul(ff, ff);
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
             s.ctl->rec_u[o] = up;
             s.ctl->rec_v[o] = vo[j];
             s.ctl->rec_a[o] = ao[j];
-            s.ctl->rec_w[o] = w;
+            s.ctl->rec_w[o] = load_well(s, p);
         }
     }
     if (p0 < N) {
@@ -611,16 +617,13 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
             }
         }
     }
-    if (nan) {
-        sh.nan = 1;
-    }
     if (pending && !redo) {
         sh.pending = 1;
         for (int j = 0; j < PPT; ++j) {
             /* record the particles of this thread that need a new window */
             int64_t p = p0 + j;
             if (p < N) {
-                double4_32a w = s.wc[p];
+                double2 w = s.wy[p];
                 if (!in_well(w.x, w.y, un[j]) && !non_finite(un[j])) {
                     int k = atomicAdd(&s.ctl->n_regen, 1);
                     s.regen_list[k] = (int32_t)p;
@@ -678,10 +681,12 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s
     const double* a0 = s.a[cur];
     const int64_t p = i * C + jc;
     double up = 0.0, vr = 0.0, ar = 0.0;
+    double2 wk = make_double2(0.0, 0.0);
     if (valid) {
+        wk = s.wk[p];
         vr = v0[p];
         ar = a0[p];
-        up = S_ADD(3, S_ADD(2, u0[p], S_MUL(0, s.dt, vr)), S_MUL(1, s.hdt2, ar));
+        up = S_ADD(3, S_ADD(2, u0[p], S_MULC(0, s.f_dt, s.dt, vr)), S_MULC(1, s.f_hdt2, s.hdt2, ar));
         sh_un[1 + ty][1 + tx] = up;
     }
     {
@@ -719,7 +724,8 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s
     __syncthreads();
     if (valid) {
         bool regen;
-        double4_32a w = well_of(s, p, up, act, sh, regen);
+        double d;
+        double4_32a w = well_of<POT, SOFT>(s, p, up, act, sh, wk, d, regen);
         if (regen) {
             if (!redo) {
                 sh.pending = 1;
@@ -731,7 +737,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s
             }
         }
         double ff;
-        double sfp = frame_pot<POT, SOFT>(s, w, up, uf, ff);
+        double sfp = frame_pot<POT, SOFT>(s, w, d, up, uf, ff);
         double fi;
         if (INTER == INTER_LAPLACE2D) {
             const double uU = sh_un[ty][1 + tx];
@@ -751,9 +757,6 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s
         s.u[cur ^ 1][p] = up;
         s.v[cur ^ 1][p] = vv;
         s.a[cur ^ 1][p] = aa;
-        if (is_nan_bits(up)) {
-            sh.nan = 1;
-        }
         if (resid) {
             s.sq2[p] = make_double2(fq_smul(f, f), fq_smul(ff, ff));
         }
@@ -819,15 +822,18 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(DevSys 
     const double* v0 = s.v[cur];
     const double* a0 = s.a[cur];
     double up[2], vr[2], ar[2];
+    double2 wk[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int64_t i = i0 + q;
         up[q] = vr[q] = ar[q] = 0.0;
+        wk[q] = make_double2(0.0, 0.0);
         if (i < R && jc < C) {
             const int64_t p = i * C + jc;
+            wk[q] = s.wk[p];
             vr[q] = v0[p];
             ar[q] = a0[p];
-            up[q] = S_ADD(3, S_ADD(2, u0[p], S_MUL(0, s.dt, vr[q])), S_MUL(1, s.hdt2, ar[q]));
+            up[q] = S_ADD(3, S_ADD(2, u0[p], S_MULC(0, s.f_dt, s.dt, vr[q])), S_MULC(1, s.f_hdt2, s.hdt2, ar[q]));
             sh_un[1 + 2 * ty + q][1 + tx] = up[q];
         }
     }
@@ -854,7 +860,8 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(DevSys 
         const int64_t p = i * C + jc;
         const int r = 2 * ty + q;
         bool regen;
-        double4_32a w = well_of(s, p, up[q], act, sh, regen);
+        double d;
+        double4_32a w = well_of<POT, SOFT>(s, p, up[q], act, sh, wk[q], d, regen);
         if (regen) {
             if (!redo) {
                 sh.pending = 1;
@@ -866,21 +873,19 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(DevSys 
             }
         }
         double ff;
-        double sfp = frame_pot<POT, SOFT>(s, w, up[q], uf, ff);
+        double sfp = frame_pot<POT, SOFT>(s, w, d, up[q], uf, ff);
         const double uU = sh_un[r][1 + tx];
         const double uD = sh_un[r + 2][1 + tx];
         const double uL = sh_un[1 + r][tx];
         const double uR = sh_un[1 + r][tx + 2];
-        double fi = scale(FQ_SUB(FQ_ADD(FQ_ADD(FQ_ADD(uU, uD), uL), uR), scale_pow2(up[q], 2, 4.0)), s.s_k);
-        double sfi = S_ADD(9, sfp, fi);
+        /* 4 u is exact: the subtraction is one fma (as f + k (...), for a power of two k) */
+        const double lap = FQ_FMA(up[q], -4.0, S_ADD(7, S_ADD(8, FQ_ADD(uU, uD), uL), uR));
+        double sfi = scale_add<SOFT != 0u>(lap, s.s_k, sfp);
         double vv, aa, f;
         verlet_velocity<SOFT>(s, sfi, vr[q], ar[q], vv, aa, f);
         s.u[cur ^ 1][p] = up[q];
         s.v[cur ^ 1][p] = vv;
         s.a[cur ^ 1][p] = aa;
-        if (is_nan_bits(up[q])) {
-            sh.nan = 1;
-        }
         if (resid) {
             s.sq2[p] = make_double2(fq_smul(f, f), fq_smul(ff, ff));
         }
@@ -1320,7 +1325,7 @@ __global__ void __launch_bounds__(256) k_lr_step(DevSys s, int redo)
         }
     }
     double rf = 0.0, rff = 0.0;
-    bool nan = false, pending = false;
+    bool pending = false;
 #pragma unroll
     for (int j = 0; j < PPT; ++j) {
         const int64_t p = p0 + j;
@@ -1328,16 +1333,16 @@ __global__ void __launch_bounds__(256) k_lr_step(DevSys s, int redo)
             continue;
         }
         bool regen;
-        double4_32a w = well_of(s, p, up[j], act, sh, regen);
+        double d;
+        double4_32a w = well_of<POT>(s, p, up[j], act, sh, s.wk[p], d, regen);
         pending |= regen;
         double ff;
-        double sfp = frame_pot<POT>(s, w, up[j], uf, ff);
+        double sfp = frame_pot<POT>(s, w, d, up[j], uf, ff);
         double sfi = FQ_ADD(sfp, fi[j]);
         double vo, ao, f;
         verlet_velocity(s, sfi, s.v[cur][p], s.a[cur][p], vo, ao, f);
         s.v[cur ^ 1][p] = vo;
         s.a[cur ^ 1][p] = ao;
-        nan |= is_nan_bits(up[j]);
         if (resid) {
             double f2 = fq_smul(f, f), ff2 = fq_smul(ff, ff);
             if (j == 0) {
@@ -1350,15 +1355,12 @@ __global__ void __launch_bounds__(256) k_lr_step(DevSys s, int redo)
             }
         }
     }
-    if (nan) {
-        sh.nan = 1;
-    }
     if (pending && !redo) {
         sh.pending = 1;
         for (int j = 0; j < PPT; ++j) {
             const int64_t p = p0 + j;
             if (p < N) {
-                double4_32a w = s.wc[p];
+                double2 w = s.wy[p];
                 if (!in_well(w.x, w.y, up[j]) && !non_finite(up[j])) {
                     int k = atomicAdd(&s.ctl->n_regen, 1);
                     s.regen_list[k] = (int32_t)p;
@@ -1636,7 +1638,7 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
             u[j] = s.u[cur][p];
             v[j] = s.v[cur][p];
             a[j] = s.a[cur][p];
-            w[j] = s.wc[p];
+            w[j] = load_well(s, p);
         }
         else {
             u[j] = v[j] = a[j] = 0.0;
@@ -1660,7 +1662,7 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
         if (!ctrl) {
 #pragma unroll
             for (int j = 0; j < PPT; ++j) {
-                un[j] = S_ADD(3, S_ADD(2, u[j], S_MUL(0, s.dt, v[j])), S_MUL(1, s.hdt2, a[j]));
+                un[j] = S_ADD(3, S_ADD(2, u[j], S_MULC(0, s.f_dt, s.dt, v[j])), S_MULC(1, s.f_hdt2, s.hdt2, a[j]));
                 sh_un[buf][tid * PPT + j] = un[j];
             }
         }
@@ -1696,7 +1698,7 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
                         placed = true;
                     }
                     /* the well of the restored position (index, cached well) in the restored window */
-                    double4_32a ww = s.wc[p];
+                    double4_32a ww = load_well(s, p);
                     if ((placed || !in_well(ww.x, ww.y, u[j])) && !non_finite(u[j]) &&
                         !window_search(s, p, u[j], ww)) {
                         dev_align(s, p, u[j]);
@@ -1770,20 +1772,32 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
         int64_t gold[PPT];
         bool mv[PPT];
         bool any_mv = false;
+        double d[PPT]; /* Cuspy: centre - u (well_of) */
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {
             int64_t p = p0 + j;
             mv[j] = false;
+            d[j] = 0.0;
             if (p >= N) {
                 continue;
             }
             double up = un[j];
+            /* with one particle per thread the wait for d would be on the critical path (65 cycles of a
+             * step's ~6300): there the keys of un, which are ready, decide */
+            if (POT == POT_CUSPY && SOFT != 0u) {
+                d[j] = S_SUB(5, w[j].z, up);
+                if (surely_in_well(make_double2(w[j].z, w[j].w), d[j])) {
+                    continue;
+                }
+            }
+            nan |= is_nan_bits(up);
             double4_32a ww = w[j];
             if (!in_well(ww.x, ww.y, up) && !non_finite(up)) {
                 gold[j] = s.gidx[p];
                 if (window_search(s, p, up, ww)) {
                     count_move(p, gold[j], s.gidx[p]);
                     w[j] = ww;
+                    d[j] = FQ_SUB(ww.z, up);
                 }
                 else {
                     mv[j] = true;
@@ -1851,7 +1865,8 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
                         sh_walk = 1;
                     }
                 }
-                w[j] = s.wc[p];
+                w[j] = load_well(s, p);
+                d[j] = FQ_SUB(w[j].z, un[j]);
                 count_move(p, gold[j], s.gidx[p]);
             }
         }
@@ -1864,21 +1879,24 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
             double up = un[j];
             const double4_32a ww = w[j];
             double ff;
-            double sfp = frame_pot<POT, SOFT>(s, ww, up, uf, ff);
-            double fi = 0.0;
+            if (SOFT == 0u) {
+                d[j] = FQ_SUB(ww.z, up);
+            }
+            double sfi = frame_pot<POT, SOFT>(s, ww, d[j], up, uf, ff);
             if (inter_ring(INTER)) {
                 int li = tid * PPT + j;
                 double uL = li > 0 ? sh_un[buf][li - 1] : left[buf][il];
                 double uR = (li + 1 < tile && p + 1 < N) ? sh_un[buf][li + 1] : right[buf][ir];
-                fi = ring_force<INTER, SOFT>(s, uL, up, uR);
+                sfi = add_ring_force<INTER, SOFT>(s, sfi, uL, up, uR);
             }
-            double sfi = S_ADD(9, sfp, fi);
+            else {
+                sfi = add_zero(sfi);
+            }
             double vn, an, f;
             verlet_velocity<SOFT>(s, sfi, v[j], a[j], vn, an, f);
             u[j] = up;
             v[j] = vn;
             a[j] = an;
-            nan |= is_nan_bits(up);
             if (resid) {
                 double f2 = mul_nospec(f, f), ff2 = mul_nospec(ff, ff);
                 if (j == 0) {
