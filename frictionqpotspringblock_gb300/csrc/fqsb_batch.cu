@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                         s.gidx[g] = s.start[g] + li;
                         const double4_32a w = make_wc(s, y[li], y[li + 1]);
                         store_well(s, g, w);
-                        d = FQ_SUB(w.z, up);
+                        d = fq_s_hw_add(w.z, -up);
                         atomicAdd(&sh.ds, (unsigned long long)(s.gidx[g] - gold));
                         ok = true;
                     }

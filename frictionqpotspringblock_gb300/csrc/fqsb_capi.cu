@@ -37,6 +37,7 @@ struct fqsb_system {
     int device;
     bool is2d;
     LineGeom lg;
+    RunGeom rg;     /* resident run kernel (ctas = 0: none) */
     /* host mirrors of the run state */
     int cur;
     int64_t inc, qs_first, qs_last;
@@ -539,14 +540,14 @@ static int ensure_graph(fqsb_system* h, int mode = KMODE_GENERAL)
         if (!*g) {
             /* built from a copy: its conditional handles are its own kernels' arguments */
             DevSys d = h->d;
-            CU(h, build_run_graph(d, h->lg, g, mode));
+            CU(h, build_run_graph(d, h->lg, h->rg, g, mode));
         }
         return FQSB_OK;
     }
     if (h->graph) {
         return FQSB_OK;
     }
-    CU(h, build_run_graph(h->d, h->lg, &h->graph));
+    CU(h, build_run_graph(h->d, h->lg, h->rg, &h->graph));
     return FQSB_OK;
 }
 
@@ -609,9 +610,9 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     }
     bool use_small = np == nullptr && h->small_ok && io == nullptr && !(flags & (RF_SCHEDULE | RF_RECORD | RF_FFSUM)) &&
                      !((flags & RF_RESID) && niter_tol > SMALL_RING_MAX);
-    /* runs without activity, frame-force sums or recording take the specialised step kernels */
+    /* runs without activity, frame-force sums or recording take the specialised run kernels */
     int kmode = KMODE_GENERAL;
-    if (np == nullptr && plain_runs_apply(h->d) && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
+    if (np == nullptr && h->rg.ctas && h->use_graph && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
         kmode = (flags & RF_RESID) ? KMODE_RESID : KMODE_PLAIN;
     }
     if (np) {
@@ -716,7 +717,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
         }
         else {
             for (int i = 0; i < 64; ++i) {
-                CU(h, launch_iteration(h->d, h->lg, h->stream, kmode));
+                CU(h, launch_iteration(h->d, h->lg, h->stream));
             }
         }
         first_launch = false;
@@ -750,6 +751,9 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     }
     if (c->error == DERR_WALK) {
         return set_err(h, FQSB_ERR_TIMEOUT, "yield search exceeded its bound (position too far from the chunk)");
+    }
+    if (c->error == DERR_BARRIER) {
+        return set_err(h, FQSB_ERR_TIMEOUT, "a wait of the run kernel's CTAs for one another ran out");
     }
     return FQSB_OK;
 }
@@ -786,7 +790,7 @@ static void free_all(fqsb_system* h)
     DevSys& d = h->d;
     void* ptrs[] = {d.data, d.nx, d.nx_end, d.start, d.cidx, d.gidx, d.wy, d.wk, d.acc_end, d.anc_kind, d.anc_k, d.anc_state, d.anc_val,
                     d.u[0], d.u[1], d.v[0], d.v[1], d.a[0], d.a[1], d.ctl, d.ring, d.partials, d.i_n, d.sq2,
-                    d.cta_pending, d.regen_list, (void*)d.lr_pref, d.f_th, d.th_next, (void*)d.th_dinc, d.th_cnt,
+                    d.cta_pending, d.regen_list, d.sync, d.nodes, (void*)d.lr_pref, d.f_th, d.th_next, (void*)d.th_dinc, d.th_cnt,
                     d.th_list, d.th,
                     (void*)d.offp, h->scratch, h->red_partials, h->red_out, h->mkey, h->mflag, h->fs[0], h->fs[1],
                     h->fs[2], h->fs[3], h->fs[4], h->adj_sched, h->adj_ckpt, h->adj_ffsum, h->adj_final};
@@ -942,7 +946,8 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     d.f_hdt = fq_s_factor(d.hdt);
     d.f_hdt2 = fq_s_factor(d.hdt2);
     d.f_me = fq_s_factor(d.me);
-    h->lg = line_geometry(N);
+    h->rg = run_geometry(d);
+    h->lg = h->rg.ctas ? strip_geometry(N, h->rg.S) : line_geometry(N);
     {
         /* small Line1d / Particles systems: whole runs in one thread-block cluster */
         const char* ns = getenv("FQSB_NO_SMALL");
@@ -956,7 +961,11 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
                       !(ns && ns[0] == '1');
     }
     int64_t nsteps_cta = step_ctas(d, h->lg);
-    int64_t npart = h->is2d ? std::max(grid_reduce_ctas(N), nsteps_cta) : h->lg.grid;
+    if (!h->is2d) {
+        /* a RandomNormalForcing attached later takes the step kernel's own shape */
+        nsteps_cta = std::max(nsteps_cta, line_geometry(N).grid);
+    }
+    int64_t npart = h->is2d ? std::max(grid_reduce_ctas(N), nsteps_cta) : nsteps_cta;
     npart = std::max(npart, (int64_t)SMALL_MAX_CTAS); /* the one-cluster run kernel's CTA subtrees */
     d.npartials = npart;
 
@@ -995,6 +1004,8 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     }
     ALLOC(d.ctl, sizeof(Ctl));
     ALLOC(d.partials, sizeof(double2) * (size_t)npart);
+    ALLOC(d.sync, sizeof(RunSync));
+    ALLOC(d.nodes, sizeof(double2) * 2 * (size_t)RUN_NODES_MAX);
     if (d.inter == INTER_LONGRANGE1D) {
         /* LongRange1d constructor, detail.h:828-841: k / std::pow(d, alpha + 1) on the host */
         std::vector<double> pref((size_t)N);
@@ -1039,6 +1050,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     /* initSystem detail.h:1096-1139: zeros, disorder, refresh */
     cudaStream_t st = h->stream;
     bool ok = cudaMemsetAsync(d.ctl, 0, sizeof(Ctl), st) == cudaSuccess &&
+              cudaMemsetAsync(d.sync, 0, sizeof(RunSync), st) == cudaSuccess &&
               cudaMemsetAsync(d.cta_pending, 0, sizeof(int32_t) * (size_t)nsteps_cta, st) == cudaSuccess;
     for (int b = 0; b < 2 && ok; ++b) {
         ok = cudaMemsetAsync(d.u[b], 0, ndp, st) == cudaSuccess && cudaMemsetAsync(d.v[b], 0, ndp, st) == cudaSuccess &&
@@ -1546,7 +1558,9 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     d.th = th;
     d.th_mean = mean;
     d.th_sc = stddev * M_SQRT2; /* the association of the reference's normal transform */
-    /* the run graph's kernels take the new pointers; the one-cluster kernel has no thermal term */
+    /* the run graph's kernels take the new pointers; the one-cluster and run kernels have no thermal term */
+    h->rg = RunGeom{};
+    h->lg = line_geometry(N);
     if (h->graph) {
         cudaGraphExecDestroy(h->graph);
         h->graph = nullptr;

@@ -69,8 +69,8 @@ enum : int {
 
 /* termination codes of a stepping run (Ctl::done) */
 enum : int { RUN_ACTIVE = 0, RUN_CONVERGED = 1, RUN_MAXITER = 2, RUN_EVENT = 3, RUN_TRUNCATED = 4 };
-/* error codes (Ctl::error), equal to fqsb_status */
-enum : int { DERR_NONE = 0, DERR_NAN = 1, DERR_WALK = 5 };
+/* error codes (Ctl::error) */
+enum : int { DERR_NONE = 0, DERR_NAN = 1, DERR_WALK = 5, DERR_BARRIER = 6 };
 
 /* Upper bound on the draws one yield search may walk through; beyond it the search gives up
  * (flagging Ctl::walk_flag) instead of running for an unbounded time. */
@@ -140,6 +140,20 @@ struct Thermal {
     uint32_t pad;
 };
 
+/*
+ * Shared state of the resident run kernel's CTAs (fqsb_run.cu).  The slots alternate between even and odd
+ * steps of a launch; all but `base`, `arrived` and `failed` are zero between launches.
+ */
+struct RunSync {
+    unsigned long long arrived; /* arrivals at the grid barrier, over all launches */
+    unsigned long long base;    /* arrivals before the next launch */
+    int32_t failed;             /* a wait at the barrier ran out */
+    int32_t stop[2];            /* the run stops after the step before this one */
+    int32_t pending[2];         /* strips with a particle whose chunk window must move */
+    int32_t nan[2];
+    int64_t ds[2], da[2];       /* change of the plastic activity (Ctl::s_sum, Ctl::a_count) */
+};
+
 /* prrng pcg32(seed): the PCG seeding procedure on the default stream 0xda3e39cb94b95bdb */
 constexpr uint64_t PCG_DEFAULT_STREAM = 0xda3e39cb94b95bdbULL;
 
@@ -167,6 +181,7 @@ struct Scale {
     int mode; /* SCALE_* */
     int e;    /* c = 2^e when mode == SCALE_POW2 */
     double c;
+    double c_add; /* c where x * c is exact (1, a power of two), else 1 (scale_add) */
     fq_sfactor f; /* c for the integer-pipe multiplication */
 };
 
@@ -176,6 +191,7 @@ inline Scale classify_scale(double c)
 {
     Scale sc;
     sc.c = c;
+    sc.c_add = 1.0;
     sc.e = 0;
     sc.f = fq_s_factor(c);
     sc.mode = SCALE_GENERAL;
@@ -188,6 +204,7 @@ inline Scale classify_scale(double c)
     if (c > 0.0 && m == 0.5 && std::isnormal(c)) {
         sc.mode = SCALE_POW2;
         sc.e = e - 1;
+        sc.c_add = c;
     }
     return sc;
 }
@@ -236,6 +253,8 @@ struct DevSys {
     int64_t* i_n;
     double2* sq2;
     int64_t npartials;
+    RunSync* sync;  /* resident run kernel: shared state, and the sums of its nodes (2 x RUN_NODES_MAX) */
+    double2* nodes;
     int32_t* cta_pending; /* per CTA of the step grid */
     int32_t* regen_list;  /* particles whose chunk window must move (capacity N) */
     unsigned long long h_while; /* cudaGraphConditionalHandle of the run loop */
@@ -963,14 +982,14 @@ __device__ __forceinline__ bool in_well(double yl, double yr, double u)
 #define S_MULC(bit, f, c, x) (((SOFT >> (bit)) & 1u) ? fq_smulc((x), (f)) : FQ_MUL((c), (x)))
 
 /*
- * The split the step kernels use: the eight multiplications, the two additions of the position update and
- * a0 + a of the last two velocity updates on the integer pipes, the other twelve additions on the fp64
- * pipe.  Of the splits measured on the N = 2^22 flow step (159 us) the neighbours are: without 14 and
- * 19 172 us; with 4 and 5 instead 161 us; with 4 as well 160 us; with 11 as well 162 us; with 4, 5 and
- * 11 as well 169 us; the multiplications alone 180 us.
+ * The split the step kernels use: the eight multiplications, the two additions of the position update,
+ * u_frame - u' and a0 + a of the last two velocity updates on the integer pipes, the other eleven additions
+ * on the fp64 pipe.  Of the splits measured on the N = 2^22 flow (resident run kernel, 144 us per step) the
+ * neighbours are: without 4 149 us; without 4, 14 and 19 166 us; with 5 as well 152 us; with 11 as well 142
+ * us (but minimise 173 instead of 169 us); with 16 as well 142 us (minimise 173 us).
  */
-constexpr unsigned STEP_SOFT = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 10) | (1u << 12) | (1u << 14) |
-                               (1u << 15) | (1u << 17) | (1u << 19) | (1u << 20) | (1u << 22);
+constexpr unsigned STEP_SOFT = (1u << 0) | (1u << 1) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 10) | (1u << 12) |
+                               (1u << 14) | (1u << 15) | (1u << 17) | (1u << 19) | (1u << 20) | (1u << 22);
 
 /* fp64 add / mul for work inside a run-time branch (residual and frame-force sums): volatile, so the
  * compiler cannot execute them speculatively before the branch, as it does with the plain forms. */
@@ -992,8 +1011,11 @@ __device__ __forceinline__ bool is_nan_bits(double x)
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
 }
 
-/* x * 2^e for a positive power of two: an exponent add when the result stays a normal number, exact
- * like the fp64 multiplication; zeros pass through; other cases use the fp64 multiply. */
+/*
+ * x * 2^e for a positive power of two: an exponent add when the result stays a normal number, exact
+ * like the fp64 multiplication; zeros pass through; other cases use the fp64 multiply (a call: inlined,
+ * the compiler would predicate it, and a predicated fp64 instruction takes its pipe cycles all the same).
+ */
 __device__ __forceinline__ double scale_pow2(double x, int e, double c)
 {
     long long b = __double_as_longlong(x);
@@ -1005,31 +1027,45 @@ __device__ __forceinline__ double scale_pow2(double x, int e, double c)
     if ((b & 0x7fffffffffffffffLL) == 0) {
         return x;
     }
-    return FQ_MUL(x, c);
+    return fq_s_hw_mul(x, c);
 }
 
-/* x * c with c described by sc (c > 0 for the power-of-two forms); SOFT: a general c on the integer pipes. */
+/* x * c of scale() for c other than 1, general c on the integer pipes: out of line, for the same reason */
+static __device__ __noinline__ double scale_other(double x, const Scale& sc)
+{
+    return sc.mode == SCALE_POW2 ? scale_pow2(x, sc.e, sc.c) : fq_smulc(x, sc.f);
+}
+
+/* x * c with c described by sc (c > 0 for the power-of-two forms).  SOFT: for kernels bound by the fp64 pipe;
+ * else for those bound by latency, where a call would cost more than the predicated multiplication. */
 template <bool SOFT = false>
 __device__ __forceinline__ double scale(double x, const Scale& sc)
 {
     if (sc.mode == SCALE_ONE) {
         return x;
     }
-    if (sc.mode == SCALE_POW2) {
-        return scale_pow2(x, sc.e, sc.c);
+    if (SOFT) {
+        return scale_other(x, sc);
     }
-    return SOFT ? fq_smulc(x, sc.f) : FQ_MUL(x, sc.c);
+    if (sc.mode == SCALE_POW2) {
+        const long long b = __double_as_longlong(x);
+        const int ex = (int)((b >> 52) & 0x7ff), ne = ex + sc.e;
+        if (ex != 0 && ex != 0x7ff && ne >= 1 && ne <= 0x7fe) {
+            return __longlong_as_double(b + ((long long)sc.e << 52));
+        }
+    }
+    return FQ_MUL(x, sc.c);
 }
 
 /* x * c + y with two roundings, as scale() followed by an addition.  A power of two scales exactly, so one
- * fma does both (the fp64 pipe takes it in the cycles of the addition).  SOFT: general c on the integer pipes. */
-template <bool SOFT>
+ * fma does both (the fp64 pipe takes it in the cycles of the addition); a general c first multiplies on the
+ * integer pipes. */
 __device__ __forceinline__ double scale_add(double x, const Scale& sc, double y)
 {
-    if (sc.mode != SCALE_GENERAL) {
-        return FQ_FMA(x, sc.c, y);
+    if (sc.mode == SCALE_GENERAL) {
+        x = scale_other(x, sc);
     }
-    return FQ_ADD(SOFT ? fq_smulc(x, sc.f) : FQ_MUL(x, sc.c), y);
+    return FQ_FMA(x, sc.c_add, y);
 }
 
 /* x + 0 (f_interactions of a system without interactions): only a -0 changes */
@@ -1123,7 +1159,7 @@ template <int INTER, unsigned SOFT>
 __device__ __forceinline__ double add_ring_force(const DevSys& s, double f, double uL, double u, double uR)
 {
     if (INTER == INTER_LAPLACE1D && SOFT != 0u) {
-        return scale_add<true>(S_ADD(8, FQ_FMA(u, -2.0, uL), uR), s.s_k, f);
+        return scale_add(S_ADD(8, FQ_FMA(u, -2.0, uL), uR), s.s_k, f);
     }
     return S_ADD(9, f, ring_force<INTER>(s, uL, u, uR));
 }

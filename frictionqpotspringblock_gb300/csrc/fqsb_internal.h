@@ -22,6 +22,8 @@ struct LineGeom {
 };
 
 LineGeom line_geometry(int64_t N);
+/* The step kernel's launch shape beside the resident run kernel: one CTA per strip. */
+LineGeom strip_geometry(int64_t N, int S);
 
 /* Message returned by fqsb_last_error(NULL) (errors of calls that have no handle). */
 void set_global_error(const std::string& msg);
@@ -34,13 +36,24 @@ int64_t step_ctas(const DevSys& s, const LineGeom& g);
 
 /* The run graph: a device-side WHILE loop over fused steps, with the chunk-regeneration branch.
  * Writes the conditional handles into s (they are kernel arguments of the graph's nodes). */
-/* Step-kernel instantiations: the general one, and for athermal Line1d / Particles systems two
- * specialised ones -- runs without activity, residual, frame-force sums or recording (timeSteps /
- * flowSteps), and runs with the residual only (minimise) -- with the other code compiled out. */
+/* Run-kernel instantiations: the general one, and two specialised ones -- runs without activity, residual,
+ * frame-force sums or recording (timeSteps / flowSteps), and runs with the residual only (minimise) -- with
+ * the other code compiled out. */
 enum : int { KMODE_GENERAL = 0, KMODE_PLAIN = 1, KMODE_RESID = 2 };
-cudaError_t build_run_graph(DevSys& s, const LineGeom& g, cudaGraphExec_t* exec, int mode = KMODE_GENERAL);
-/* Whether the system has the specialised step kernels (athermal Line1d / Particles systems). */
-bool plain_runs_apply(const DevSys& s);
+struct RunGeom;
+cudaError_t build_run_graph(DevSys& s, const LineGeom& g, const RunGeom& rg, cudaGraphExec_t* exec,
+                            int mode = KMODE_GENERAL);
+
+/* Resident run kernel of Line1d / Particles systems (fqsb_run.cu): many steps in one cooperative launch. */
+static const int64_t RUN_NODES_MAX = 1216; /* 8 per SM: the control CTA sums them in one pass */
+struct RunGeom {
+    int S;               /* particles per strip: 32 .. 256, a power of two */
+    int threads, ctas;   /* launch shape (the last CTA is the control CTA); ctas = 0: not available */
+    int64_t nstrips, node_strips, nnodes;
+    size_t smem;
+};
+RunGeom run_geometry(const DevSys& s);
+const void* run_kernel(const DevSys& s, int mode);
 
 /* Small Line1d / Particles systems: a whole run in one launch of one thread-block cluster. */
 static const int SMALL_MAX_CTAS = 16;   /* cluster size limit (above 8 needs the non-portable opt-in) */
@@ -77,7 +90,7 @@ cudaError_t launch_thermal_draw(const DevSys& s, int from_ctl, int64_t inc, cuda
 int64_t thermal_tiles(int64_t N);
 
 /* One loop iteration launched kernel by kernel by the host (s.in_graph must be 0). */
-cudaError_t launch_iteration(const DevSys& s, const LineGeom& g, cudaStream_t st, int mode = KMODE_GENERAL);
+cudaError_t launch_iteration(const DevSys& s, const LineGeom& g, cudaStream_t st);
 
 /* NVTX range over one C-ABI call: each stepping / construction call shows as a named range on a
  * profiler timeline (header-only NVTX 3; a no-op unless a tool is attached). */

@@ -41,7 +41,7 @@
  * well test on keys always and the previous integer-pipe operations, 159 us as it is; the 2048 x 2048
  * grid 229 and 195 us.
  */
-#include "fqsb_internal.h"
+#include "fqsb_stepcore.cuh"
 
 #include <cooperative_groups.h>
 
@@ -57,175 +57,6 @@ template <int POT>
 struct StepOcc {
     static constexpr int value = POT == POT_SMOOTH ? 2 : 5;
 };
-
-template <unsigned SOFT = 0u>
-__device__ __forceinline__ double u_next(const DevSys& s, const double* u0, const double* v0, const double* a0,
-                                         int64_t q)
-{
-    return S_ADD(3, S_ADD(2, u0[q], S_MULC(0, s.f_dt, s.dt, v0[q])), S_MULC(1, s.f_hdt2, s.hdt2, a0[q]));
-}
-
-/*
- * The force sum of a particle without interactions and damping, f_frame + f_potential, and f_frame itself.
- * d: centre - u of a Cuspy well (the others take w).  k_frame is most often a power of two or general:
- * for a power of two f_frame is exact and one fma forms the sum (site 6; where f_frame is also needed and
- * latency counts, SOFT = 0, the sum is formed from it).
- */
-template <int POT, unsigned SOFT = 0u>
-__device__ __forceinline__ double frame_pot(const DevSys& s, const double4_32a& w, double d, double up, double uf,
-                                            double& ff)
-{
-    const double fp = POT == POT_CUSPY ? scale<SOFT != 0u>(d, s.s_mu) : pot_force<POT>(s, w, up);
-    const double x = S_SUB(4, uf, up);
-    ff = scale<SOFT != 0u>(x, s.s_kf);
-    if (SOFT == 0u) {
-        return FQ_ADD(ff, fp);
-    }
-    return s.s_kf.mode != SCALE_GENERAL ? FQ_FMA(x, s.s_kf.c, fp) : S_ADD(6, ff, fp);
-}
-
-__device__ __forceinline__ long long absll(long long x)
-{
-    return x < 0 ? -x : x;
-}
-
-__device__ __forceinline__ uint64_t globaltimer()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void set_loop(const DevSys& s, unsigned v)
-{
-    if (s.in_graph) {
-        cudaGraphSetConditional((cudaGraphConditionalHandle)s.h_while, v);
-    }
-}
-
-__device__ __forceinline__ void set_branch(const DevSys& s, unsigned v)
-{
-    if (s.in_graph) {
-        cudaGraphSetConditional((cudaGraphConditionalHandle)s.h_if, v);
-    }
-}
-
-/*
- * Bookkeeping and stop tests of one finished step on a run-control block c (global memory for the
- * graph path, shared memory for the one-cluster path) and its StopList window `ring`: step and
- * increment counters, frame position, plastic activity, NaN / yield-search errors, the StopList
- * residual test (GooseFEM::Iterate::StopList, detail.h:1780-1783), event, truncation and step limits.
- */
-template <typename CTL>
-__device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, double sf, double sff)
-{
-    int flags = c->flags;
-    c->ticket = 0;
-    c->ticket_redo = 0;
-    c->n_pending_cta = 0;
-    c->n_regen = 0;
-    if (flags & RF_FFSUM) {
-        c->rec_ffsum[c->step] = sf;
-    }
-    if (flags & RF_SCHEDULE) {
-        c->u_frame = uf;
-    }
-    c->step += 1;
-    if (!(flags & RF_NOINC)) {
-        c->inc += 1;
-    }
-    c->cur ^= 1;
-    if (flags & RF_FLOW) {
-        c->u_frame = uf;
-    }
-    uint64_t now = globaltimer();
-    if (c->launch_steps == 0) {
-        c->launch_t0 = now;
-    }
-    c->launch_steps += 1;
-    if (c->nan_flag) {
-        c->error = DERR_NAN;
-    }
-    else if (c->walk_flag) {
-        c->error = DERR_WALK;
-    }
-    else {
-        if (flags & (RF_ACT | RF_TRUNCATE)) {
-            long long sv = c->s_sum;
-            if (sv != c->s_n) {
-                if (c->init) {
-                    c->init = 0;
-                    c->qs_first = c->inc;
-                }
-                c->qs_last = c->inc;
-            }
-            c->s_n = sv;
-        }
-        if ((flags & RF_EVENT) && c->a_count != 0) {
-            c->done = RUN_EVENT;
-        }
-        if (!c->done && (flags & RF_RESID)) {
-            double r_fres = FQ_SQRT(sf);
-            double r_fext = FQ_SQRT(sff);
-            double r = r_fext != 0.0 ? FQ_DIV(r_fres, r_fext) : r_fres;
-            c->last_residual = r;
-            int64_t n = c->niter_tol;
-            if (n > 0) {
-                int64_t pos = c->sl_pos;
-                double old = ring[pos];
-                if (old >= c->tol) {
-                    c->sl_ge_tol -= 1;
-                }
-                if (old >= c->tol2) {
-                    c->sl_ge_tol2 -= 1;
-                }
-                if (n >= 2) {
-                    double second = ring[(pos + 1) % n];
-                    if (second > old) {
-                        c->sl_asc -= 1;
-                    }
-                    double newest = ring[(pos + n - 1) % n];
-                    if (r > newest) {
-                        c->sl_asc += 1;
-                    }
-                }
-                ring[pos] = r;
-                c->sl_pos = (pos + 1) % n;
-                if (r >= c->tol) {
-                    c->sl_ge_tol += 1;
-                }
-                if (r >= c->tol2) {
-                    c->sl_ge_tol2 += 1;
-                }
-            }
-            if ((c->sl_asc == 0 && c->sl_ge_tol == 0) || c->sl_ge_tol2 == 0) {
-                c->done = RUN_CONVERGED;
-            }
-        }
-        if (!c->done && (flags & RF_TRUNCATE)) {
-            if ((c->A_truncate > 0 && c->a_count >= c->A_truncate) ||
-                (c->S_truncate > 0 && c->s_sum >= c->S_truncate)) {
-                c->done = RUN_TRUNCATED;
-            }
-        }
-        if (!c->done && c->step >= c->max_steps) {
-            c->done = RUN_MAXITER;
-        }
-    }
-}
-
-/*
- * Stop tests of one finished step (thread 0 of the CTA that finishes the step last); sets the
- * run-loop condition.  sf / sff: sum of f^2 and of f_frame^2 over all particles.
- */
-__device__ void finalize_step(const DevSys& s, double uf, double sf, double sff)
-{
-    Ctl* c = s.ctl;
-    finalize_ctl(c, s.ring, uf, sf, sff);
-    bool more = !c->done && !c->error && (globaltimer() - c->launch_t0) < c->budget_ns;
-    __threadfence();
-    set_loop(s, more ? 1u : 0u);
-}
 
 /* Whole-CTA canonical tree over partials[0..G) (zero padded to a power of two). */
 static __device__ __noinline__ double2 tree_partials(const double2* partials, int64_t G, double* sh)
@@ -295,44 +126,6 @@ __device__ __forceinline__ bool step_prologue(const DevSys& s, StepShared& sh, b
 }
 
 /*
- * Searches particle p's current chunk window for the well of u (y[i] <= u < y[i+1], the prrng
- * align rule) and commits it when it lies inside the window's margins [min_margin, W - buffer).
- * Returns false when the window must move (then nothing is changed).
- */
-__device__ __forceinline__ bool window_search(const DevSys& s, int64_t p, double u, double4_32a& w)
-{
-    const int64_t W = s.W;
-    const double* y = s.data + p * W;
-    if (!(y[0] <= u && u < y[W - 1])) {
-        return false;
-    }
-    int64_t li = s.cidx[p];
-    if (y[li] <= u) {
-        while (li + 1 < W && y[li + 1] <= u) {
-            ++li;
-        }
-    }
-    else {
-        while (li > 0 && y[li] > u) {
-            --li;
-        }
-    }
-    if (li < s.min_margin || li >= W - s.buffer) {
-        return false;
-    }
-    s.cidx[p] = (int32_t)li;
-    s.gidx[p] = s.start[p] + li;
-    w = make_wc(s, y[li], y[li + 1]);
-    store_well(s, p, w);
-    return true;
-}
-
-__device__ __forceinline__ bool non_finite(double x)
-{
-    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) >= 0x7ff0000000000000LL;
-}
-
-/*
  * Well check of particle p at its new position un, from the constants wk of its cached well (loaded by the
  * caller).  Cuspy: d = centre - un, which the force needs anyway, also tells that the particle stays in
  * its well without reading the yield positions; only where it cannot tell is the exact test made (and
@@ -371,7 +164,7 @@ __device__ __forceinline__ double4_32a well_of(const DevSys& s, int64_t p, doubl
                 atomicAdd(&sh.da, (unsigned long long)da);
             }
             if (POT == POT_CUSPY) {
-                d = FQ_SUB(w.z, un);
+                d = fq_s_hw_add(w.z, -un); /* a call: not predicated into the path of the others */
             }
         }
         else {
@@ -469,8 +262,8 @@ __device__ __forceinline__ void step_epilogue(const DevSys& s, StepShared& sh, i
  * from the old state.  State arrays are padded to a multiple of 1024 entries.  redo = 1: only CTAs
  * marked pending run (after k_regen moved their particles' windows).
  */
-template <int POT, int INTER, int PPT, unsigned SOFT = STEP_SOFT, bool TH = false, int MODE = KMODE_GENERAL>
-__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s, int redo)
+template <int POT, int INTER, int PPT, unsigned SOFT = STEP_SOFT, bool TH = false>
+__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(const __grid_constant__ DevSys s, int redo)
 {
     __shared__ StepShared sh;
     __shared__ double sh_un[256 * PPT];
@@ -488,13 +281,10 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
         }
     }
     const int cur = sh.cur;
-    /* KMODE_PLAIN: the instantiation for runs without activity, residual, frame-force sums or recording
-     * (timeSteps / flowSteps); KMODE_RESID: with the residual only (minimise); the rest compiled out */
-    const bool general = MODE == KMODE_GENERAL;
-    const bool act = general && (sh.flags & (RF_ACT | RF_TRUNCATE | RF_EVENT)) != 0;
-    const bool resid = MODE == KMODE_RESID || (general && (sh.flags & RF_RESID) != 0);
-    const bool ffsum = general && (sh.flags & RF_FFSUM) != 0;
-    const bool record = general && (sh.flags & RF_RECORD) != 0;
+    const bool act = (sh.flags & (RF_ACT | RF_TRUNCATE | RF_EVENT)) != 0;
+    const bool resid = (sh.flags & RF_RESID) != 0;
+    const bool ffsum = (sh.flags & RF_FFSUM) != 0;
+    const bool record = (sh.flags & RF_RECORD) != 0;
     const int64_t rec_step = record ? ((volatile Ctl*)s.ctl)->step : 0;
     const double uf = sh.uf;
     const int64_t N = s.N;
@@ -645,7 +435,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(DevSys s
  * also finalises the step.
  */
 template <int POT, int INTER = INTER_LAPLACE2D, unsigned SOFT = STEP_SOFT>
-__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s, int redo)
+__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(const __grid_constant__ DevSys s, int redo)
 {
     __shared__ StepShared sh;
     /* the tile's new positions at [1 + row][1 + column], with the halo around its nr x nc valid
@@ -788,7 +578,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(DevSys s
  * row).  Per particle the same operations in the same order as k_step_grid, so the same results.
  */
 template <int POT, unsigned SOFT = STEP_SOFT>
-__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(DevSys s, int redo)
+__global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(const __grid_constant__ DevSys s, int redo)
 {
     __shared__ StepShared sh;
     /* the tile's new positions at [1 + row][1 + column], with the four halo lines around them: row 0
@@ -880,7 +670,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(DevSys 
         const double uR = sh_un[1 + r][tx + 2];
         /* 4 u is exact: the subtraction is one fma (as f + k (...), for a power of two k) */
         const double lap = FQ_FMA(up[q], -4.0, S_ADD(7, S_ADD(8, FQ_ADD(uU, uD), uL), uR));
-        double sfi = scale_add<SOFT != 0u>(lap, s.s_k, sfp);
+        double sfi = scale_add(lap, s.s_k, sfp);
         double vv, aa, f;
         verlet_velocity<SOFT>(s, sfi, vr[q], ar[q], vv, aa, f);
         s.u[cur ^ 1][p] = up[q];
@@ -1266,7 +1056,7 @@ __global__ void __launch_bounds__(256) k_lr_position(DevSys s)
 }
 
 template <int POT, int PPT>
-__global__ void __launch_bounds__(256) k_lr_step(DevSys s, int redo)
+__global__ void __launch_bounds__(256) k_lr_step(const __grid_constant__ DevSys s, int redo)
 {
     constexpr int LR_TILE = 1024;
     __shared__ StepShared sh;
@@ -1555,7 +1345,7 @@ __device__ __forceinline__ double2 particle_tree2(double x, double y, double* sh
 }
 
 template <int POT, int INTER, int PPT>
-__global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys s)
+__global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const __grid_constant__ DevSys s)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -1699,6 +1489,10 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(DevSys 
                     }
                     /* the well of the restored position (index, cached well) in the restored window */
                     double4_32a ww = load_well(s, p);
+                    if (placed) {
+                        /* not a well of the restored window: the search starts from its index alone */
+                        ww.x = ww.y = __longlong_as_double(0x7ff8000000000000LL);
+                    }
                     if ((placed || !in_well(ww.x, ww.y, u[j])) && !non_finite(u[j]) &&
                         !window_search(s, p, u[j], ww)) {
                         dev_align(s, p, u[j]);
@@ -2074,6 +1868,15 @@ LineGeom line_geometry(int64_t N)
     return g;
 }
 
+LineGeom strip_geometry(int64_t N, int S)
+{
+    LineGeom g;
+    g.ppt = 1;
+    g.threads = S;
+    g.grid = (N + S - 1) / S;
+    return g;
+}
+
 int64_t grid_reduce_ctas(int64_t N)
 {
     return (N + 1023) / 1024;
@@ -2089,40 +1892,14 @@ int64_t step_ctas(const DevSys& s, const LineGeom& g)
 
 /* ------------------------------------------------------------- run graph */
 
-template <int POT, int INTER, bool TH = false, int MODE = KMODE_GENERAL>
+template <int POT, int INTER, bool TH = false>
 static void* line_kernel_t(int ppt)
 {
-    return ppt == 2 ? (void*)k_step_line<POT, INTER, 2, STEP_SOFT, TH, MODE>
-                    : (void*)k_step_line<POT, INTER, 1, STEP_SOFT, TH, MODE>;
+    return ppt == 2 ? (void*)k_step_line<POT, INTER, 2, STEP_SOFT, TH> : (void*)k_step_line<POT, INTER, 1, STEP_SOFT, TH>;
 }
 
-template <int MODE>
-static void* special_kernel(const DevSys& s, const LineGeom& g)
+static void* step_kernel(const DevSys& s, const LineGeom& g)
 {
-    if (s.inter == INTER_LAPLACE1D) {
-        switch (s.pot) {
-            case POT_CUSPY: return line_kernel_t<POT_CUSPY, INTER_LAPLACE1D, false, MODE>(g.ppt);
-            case POT_SEMISMOOTH: return line_kernel_t<POT_SEMISMOOTH, INTER_LAPLACE1D, false, MODE>(g.ppt);
-            default: return line_kernel_t<POT_SMOOTH, INTER_LAPLACE1D, false, MODE>(g.ppt);
-        }
-    }
-    switch (s.pot) {
-        case POT_CUSPY: return line_kernel_t<POT_CUSPY, INTER_NONE, false, MODE>(g.ppt);
-        case POT_SEMISMOOTH: return line_kernel_t<POT_SEMISMOOTH, INTER_NONE, false, MODE>(g.ppt);
-        default: return line_kernel_t<POT_SMOOTH, INTER_NONE, false, MODE>(g.ppt);
-    }
-}
-
-bool plain_runs_apply(const DevSys& s)
-{
-    return !s.f_th && (s.inter == INTER_LAPLACE1D || s.inter == INTER_NONE);
-}
-
-static void* step_kernel(const DevSys& s, const LineGeom& g, int mode = KMODE_GENERAL)
-{
-    if (mode != KMODE_GENERAL && plain_runs_apply(s)) {
-        return mode == KMODE_PLAIN ? special_kernel<KMODE_PLAIN>(s, g) : special_kernel<KMODE_RESID>(s, g);
-    }
     if (s.f_th) {
         /* RandomNormalForcing systems: Cuspy with Laplace1d, Quartic1d or no interactions */
         switch (s.inter) {
@@ -2197,7 +1974,7 @@ static cudaError_t add_conditional(cudaGraphNode_t* node, cudaGraph_t graph, con
  * profile kernels inside conditional graphs): pass 1, the regeneration kernel and the redo are always
  * launched; the latter two do nothing when no CTA is pending.
  */
-cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t st, int mode)
+cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t st)
 {
     bool is2d = inter_grid(s.inter);
     dim3 grid, block;
@@ -2209,7 +1986,7 @@ cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t s
         grid = dim3((unsigned)g0.grid);
         block = dim3((unsigned)g0.threads);
     }
-    void* fstep = step_kernel(s, g0, mode);
+    void* fstep = step_kernel(s, g0);
     int pass1 = 0, pass2 = 1;
     void* args1[] = {(void*)&s, (void*)&pass1};
     void* args2[] = {(void*)&s, (void*)&pass2};
@@ -2246,10 +2023,10 @@ cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t s
     } while (0)
 
 /*
- * The run graph: WHILE(h_while) { step pass 1 ; IF(h_if) { regenerate windows ; redo pending CTAs } ;
- * [2d: reduce + finalise] }.  `s` is updated with the two conditional handles (kernel arguments).
+ * The run graph: WHILE(h_while) { step pass 1, or for Line1d / Particles systems the resident run kernel's
+ * many steps ; IF(h_if) { regenerate windows ; redo pending CTAs } ; [2d: reduce + finalise] }.  `s` is updated with the two conditional handles (kernel arguments).
  */
-cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, cudaGraphExec_t* exec, int mode)
+cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cudaGraphExec_t* exec, int mode)
 {
     cudaGraph_t g;
     cudaError_t e = cudaGraphCreate(&g, 0);
@@ -2276,7 +2053,7 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, cudaGraphExec_t* exec
         grid = dim3((unsigned)g0.grid);
         block = dim3((unsigned)g0.threads);
     }
-    void* fstep = step_kernel(s, g0, mode);
+    void* fstep = step_kernel(s, g0);
     int pass1 = 0, pass2 = 1;
     void* args1[] = {(void*)&s, (void*)&pass1};
     void* args2[] = {(void*)&s, (void*)&pass2};
@@ -2300,6 +2077,21 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, cudaGraphExec_t* exec
         GR(add_kernel(&npos, body, nullptr, 0, (void*)k_lr_position, dim3((unsigned)((s.N + 255) / 256)), dim3(256),
                       argsr));
         GR(add_kernel(&nstep, body, &npos, 1, fstep, grid, block, args1));
+    }
+    else if (rg.ctas) {
+        /* many steps per launch; its CTAs wait on one another, so all of them must be resident */
+        void* argsl[] = {(void*)&s, (void*)&rg};
+        cudaKernelNodeParams kp = {};
+        kp.func = const_cast<void*>(run_kernel(s, mode));
+        kp.gridDim = dim3((unsigned)rg.ctas);
+        kp.blockDim = dim3((unsigned)rg.threads);
+        kp.sharedMemBytes = (unsigned)rg.smem;
+        GR(cudaFuncSetAttribute(kp.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rg.smem));
+        kp.kernelParams = argsl;
+        GR(cudaGraphAddKernelNode(&nstep, body, nullptr, 0, &kp));
+        cudaKernelNodeAttrValue coop = {};
+        coop.cooperative = 1;
+        GR(cudaGraphKernelNodeSetAttribute(nstep, cudaLaunchAttributeCooperative, &coop));
     }
     else {
         GR(add_kernel(&nstep, body, nullptr, 0, fstep, grid, block, args1));

@@ -1,0 +1,261 @@
+/*
+ * Parts shared by the step kernels (fqsb_step.cu) and the resident run kernel (fqsb_run.cu): position
+ * update, force sum without interactions, the search of a chunk window, and the bookkeeping and stop
+ * tests of a finished step.
+ */
+#ifndef FQSB_STEPCORE_CUH
+#define FQSB_STEPCORE_CUH
+
+#include "fqsb_internal.h"
+
+namespace fqsb {
+
+template <unsigned SOFT = 0u>
+__device__ __forceinline__ double u_next(const DevSys& s, const double* u0, const double* v0, const double* a0,
+                                         int64_t q)
+{
+    return S_ADD(3, S_ADD(2, u0[q], S_MULC(0, s.f_dt, s.dt, v0[q])), S_MULC(1, s.f_hdt2, s.hdt2, a0[q]));
+}
+
+/*
+ * The force sum of a particle without interactions and damping, f_frame + f_potential, and f_frame itself.
+ * d: centre - u of a Cuspy well (the others take w).  k_frame is most often a power of two or general:
+ * for a power of two f_frame is exact and one fma forms the sum (site 6; where f_frame is also needed and
+ * latency counts, SOFT = 0, the sum is formed from it).
+ */
+template <int POT, unsigned SOFT = 0u>
+__device__ __forceinline__ double frame_pot(const DevSys& s, const double4_32a& w, double d, double up, double uf,
+                                            double& ff)
+{
+    const double fp = POT == POT_CUSPY ? scale<SOFT != 0u>(d, s.s_mu) : pot_force<POT>(s, w, up);
+    double x = S_SUB(4, uf, up);
+    if (SOFT == 0u) {
+        ff = scale(x, s.s_kf);
+        return FQ_ADD(ff, fp);
+    }
+    if (s.s_kf.mode == SCALE_GENERAL) {
+        x = fq_smulc(x, s.s_kf.f);
+        ff = x;
+    }
+    else {
+        ff = scale(x, s.s_kf); /* read for the residual and frame-force sums only */
+    }
+    return FQ_FMA(x, s.s_kf.c_add, fp);
+}
+
+__device__ __forceinline__ long long absll(long long x)
+{
+    return x < 0 ? -x : x;
+}
+
+__device__ __forceinline__ uint64_t globaltimer()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ void set_loop(const DevSys& s, unsigned v)
+{
+    if (s.in_graph) {
+        cudaGraphSetConditional((cudaGraphConditionalHandle)s.h_while, v);
+    }
+}
+
+__device__ __forceinline__ void set_branch(const DevSys& s, unsigned v)
+{
+    if (s.in_graph) {
+        cudaGraphSetConditional((cudaGraphConditionalHandle)s.h_if, v);
+    }
+}
+
+/*
+ * Bookkeeping and stop tests of one finished step on a run-control block c (global memory for the
+ * graph path, shared memory for the one-cluster path) and its StopList window `ring`: step and
+ * increment counters, frame position, plastic activity, NaN / yield-search errors, the StopList
+ * residual test (GooseFEM::Iterate::StopList, detail.h:1780-1783), event, truncation and step limits.
+ */
+template <typename CTL>
+__device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, double sf, double sff)
+{
+    int flags = c->flags;
+    c->ticket = 0;
+    c->ticket_redo = 0;
+    c->n_pending_cta = 0;
+    c->n_regen = 0;
+    if (flags & RF_FFSUM) {
+        c->rec_ffsum[c->step] = sf;
+    }
+    if (flags & RF_SCHEDULE) {
+        c->u_frame = uf;
+    }
+    c->step += 1;
+    if (!(flags & RF_NOINC)) {
+        c->inc += 1;
+    }
+    c->cur ^= 1;
+    if (flags & RF_FLOW) {
+        c->u_frame = uf;
+    }
+    uint64_t now = globaltimer();
+    if (c->launch_steps == 0) {
+        c->launch_t0 = now;
+    }
+    c->launch_steps += 1;
+    if (c->nan_flag) {
+        c->error = DERR_NAN;
+    }
+    else if (c->walk_flag) {
+        c->error = DERR_WALK;
+    }
+    else {
+        if (flags & (RF_ACT | RF_TRUNCATE)) {
+            long long sv = c->s_sum;
+            if (sv != c->s_n) {
+                if (c->init) {
+                    c->init = 0;
+                    c->qs_first = c->inc;
+                }
+                c->qs_last = c->inc;
+            }
+            c->s_n = sv;
+        }
+        if ((flags & RF_EVENT) && c->a_count != 0) {
+            c->done = RUN_EVENT;
+        }
+        if (!c->done && (flags & RF_RESID)) {
+            double r_fres = FQ_SQRT(sf);
+            double r_fext = FQ_SQRT(sff);
+            double r = r_fext != 0.0 ? FQ_DIV(r_fres, r_fext) : r_fres;
+            c->last_residual = r;
+            int64_t n = c->niter_tol;
+            if (n > 0) {
+                int64_t pos = c->sl_pos;
+                double old = ring[pos];
+                if (old >= c->tol) {
+                    c->sl_ge_tol -= 1;
+                }
+                if (old >= c->tol2) {
+                    c->sl_ge_tol2 -= 1;
+                }
+                if (n >= 2) {
+                    double second = ring[(pos + 1) % n];
+                    if (second > old) {
+                        c->sl_asc -= 1;
+                    }
+                    double newest = ring[(pos + n - 1) % n];
+                    if (r > newest) {
+                        c->sl_asc += 1;
+                    }
+                }
+                ring[pos] = r;
+                c->sl_pos = (pos + 1) % n;
+                if (r >= c->tol) {
+                    c->sl_ge_tol += 1;
+                }
+                if (r >= c->tol2) {
+                    c->sl_ge_tol2 += 1;
+                }
+            }
+            if ((c->sl_asc == 0 && c->sl_ge_tol == 0) || c->sl_ge_tol2 == 0) {
+                c->done = RUN_CONVERGED;
+            }
+        }
+        if (!c->done && (flags & RF_TRUNCATE)) {
+            if ((c->A_truncate > 0 && c->a_count >= c->A_truncate) ||
+                (c->S_truncate > 0 && c->s_sum >= c->S_truncate)) {
+                c->done = RUN_TRUNCATED;
+            }
+        }
+        if (!c->done && c->step >= c->max_steps) {
+            c->done = RUN_MAXITER;
+        }
+    }
+}
+
+/*
+ * Stop tests of one finished step (thread 0 of the CTA that finishes the step last); sets the
+ * run-loop condition.  sf / sff: sum of f^2 and of f_frame^2 over all particles.
+ */
+static __device__ __forceinline__ void finalize_step(const DevSys& s, double uf, double sf, double sff)
+{
+    Ctl* c = s.ctl;
+    finalize_ctl(c, s.ring, uf, sf, sff);
+    bool more = !c->done && !c->error && (globaltimer() - c->launch_t0) < c->budget_ns;
+    __threadfence();
+    set_loop(s, more ? 1u : 0u);
+}
+
+/* Commits well li of particle p, between yield positions yl and yr, in the window that starts at `start`. */
+__device__ __forceinline__ void commit_well(const DevSys& s, int64_t p, int64_t start, int64_t li, double yl, double yr,
+                                            double4_32a& w)
+{
+    s.cidx[p] = (int32_t)li;
+    s.gidx[p] = start + li;
+    w = make_wc(s, yl, yr);
+    store_well(s, p, w);
+}
+
+/*
+ * Searches particle p's current chunk window for the well of u (y[i] <= u < y[i+1], the prrng
+ * align rule) and commits it when it lies inside the window's margins [min_margin, W - buffer).
+ * Returns false when the window must move (then nothing is changed).  On entry w holds the yield
+ * positions of the particle's present well (chunk index cidx), which u has left, or NaNs where they
+ * are not known.
+ *
+ * Nearly always u is in the next well on one side: its far yield position is the only load that waits for
+ * another one.  (The general search reads the window's ends, the index, and the positions one after the
+ * other; a warp waits for whichever lane leaves its well.)
+ */
+__device__ __forceinline__ bool window_search(const DevSys& s, int64_t p, double u, double4_32a& w)
+{
+    const int64_t W = s.W;
+    const double* y = s.data + p * W;
+    int64_t li = s.cidx[p];
+    const int64_t start = s.start[p];
+    if (w.y <= u) {
+        if (li + 2 < W && li + 1 >= s.min_margin && li + 1 < W - s.buffer) {
+            const double yr = y[li + 2];
+            if (u < yr) {
+                commit_well(s, p, start, li + 1, w.y, yr, w);
+                return true;
+            }
+        }
+    }
+    else if (u < w.x) {
+        if (li - 1 >= s.min_margin && li - 1 < W - s.buffer) {
+            const double yl = y[li - 1];
+            if (yl <= u) {
+                commit_well(s, p, start, li - 1, yl, w.x, w);
+                return true;
+            }
+        }
+    }
+    if (!(y[0] <= u && u < y[W - 1])) {
+        return false;
+    }
+    if (y[li] <= u) {
+        while (li + 1 < W && y[li + 1] <= u) {
+            ++li;
+        }
+    }
+    else {
+        while (li > 0 && y[li] > u) {
+            --li;
+        }
+    }
+    if (li < s.min_margin || li >= W - s.buffer) {
+        return false;
+    }
+    commit_well(s, p, start, li, y[li], y[li + 1], w);
+    return true;
+}
+
+__device__ __forceinline__ bool non_finite(double x)
+{
+    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) >= 0x7ff0000000000000LL;
+}
+
+} // namespace fqsb
+
+#endif
