@@ -988,6 +988,7 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     for (int i = 0; i < 4; ++i) {
         d.par[i] = i < c->n_parameters ? c->parameters[i] : 0.0;
     }
+    d.ipar0 = 1.0 / (d.npar > 0 ? d.par[0] : 1.0);
     d.offset = c->offset;
     d.buffer = 2;
     d.margin = 30;

@@ -932,6 +932,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     for (int i = 0; i < 4; ++i) {
         d.par[i] = i < cfg->n_parameters ? cfg->parameters[i] : 0.0;
     }
+    d.ipar0 = 1.0 / (d.npar > 0 ? d.par[0] : 1.0);
     d.offset = cfg->offset;
     d.seed = cfg->seed;
     d.buffer = 2;

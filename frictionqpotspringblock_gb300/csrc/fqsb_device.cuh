@@ -224,6 +224,7 @@ struct DevSys {
     int64_t W, n0;
     int dist, npar;
     double par[4];
+    double ipar0; /* 1 / par[0] (1 without parameters), as the power, Pareto and Weibull transforms form it */
     double offset;
     const double* offp;
     uint64_t seed;
@@ -325,12 +326,12 @@ __device__ __forceinline__ double dev_transform_inl(const DevSys& s, uint32_t r3
         case DIST_EXPONENTIAL:
             return FQ_ADD(FQ_MUL(-fq_log(FQ_SUB(1.0, r)), par_or(s, 0, 1.0)), par_or(s, 1, 0.0));
         case DIST_POWER:
-            return FQ_ADD(fq_pow(r, FQ_DIV(1.0, par_or(s, 0, 1.0))), par_or(s, 1, 0.0));
+            return FQ_ADD(fq_pow(r, s.ipar0), par_or(s, 1, 0.0));
         case DIST_PARETO:
-            return FQ_ADD(FQ_DIV(par_or(s, 1, 1.0), fq_pow(FQ_SUB(1.0, r), FQ_DIV(1.0, par_or(s, 0, 1.0)))),
+            return FQ_ADD(FQ_DIV(par_or(s, 1, 1.0), fq_pow(FQ_SUB(1.0, r), s.ipar0)),
                           par_or(s, 2, 0.0));
         case DIST_WEIBULL:
-            return FQ_ADD(FQ_MUL(par_or(s, 1, 1.0), fq_pow(-fq_log(FQ_SUB(1.0, r)), FQ_DIV(1.0, par_or(s, 0, 1.0)))),
+            return FQ_ADD(FQ_MUL(par_or(s, 1, 1.0), fq_pow(-fq_log(FQ_SUB(1.0, r)), s.ipar0)),
                           par_or(s, 2, 0.0));
         default:
             return __longlong_as_double(0x7ff8000000000000LL);
