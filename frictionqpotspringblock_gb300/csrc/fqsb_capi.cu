@@ -612,7 +612,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
                      !((flags & RF_RESID) && niter_tol > SMALL_RING_MAX);
     /* runs without activity, frame-force sums or recording take the specialised run kernels */
     int kmode = KMODE_GENERAL;
-    if (np == nullptr && h->rg.ctas && h->use_graph && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
+    if (np == nullptr && h->rg.ctas && h->use_graph && !h->d.f_th && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
         kmode = (flags & RF_RESID) ? KMODE_RESID : KMODE_PLAIN;
     }
     if (np) {
@@ -695,7 +695,18 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
                 CU(h, launch_next_window(h->d, h->stream));
                 h->nx_dirty = false;
             }
-            cudaError_t le = launch_small_run(h->d, h->sg, h->stream);
+            cudaError_t le = cudaSuccess;
+            /* with thermal forcing a launch takes the planned steps: several plans and launches per wait */
+            const int64_t launches = h->d.f_th ? std::min((int64_t)16, (max_steps - c->step + h->d.th_K - 1) / h->d.th_K) : 1;
+            for (int64_t k = 0; k < launches && le == cudaSuccess; ++k) {
+                if (h->d.f_th) {
+                    CU(h, launch_thermal_plan(h->d, h->d.th_K, TH_FROM_RUN, 0, h->stream));
+                }
+                le = launch_small_run(h->d, h->sg, h->stream);
+                if (h->d.f_th && le == cudaSuccess) {
+                    CU(h, launch_thermal_commit(h->d, TH_COMMIT_RUN, h->stream));
+                }
+            }
             if (first_launch && (le == cudaErrorInvalidClusterSize || le == cudaErrorLaunchOutOfResources)) {
                 /* the cluster could not be scheduled now (nothing ran): this handle uses the graph path */
                 cudaGetLastError();
@@ -791,7 +802,7 @@ static void free_all(fqsb_system* h)
     void* ptrs[] = {d.data, d.nx, d.nx_end, d.start, d.cidx, d.gidx, d.wy, d.wk, d.acc_end, d.anc_kind, d.anc_k, d.anc_state, d.anc_val,
                     d.u[0], d.u[1], d.v[0], d.v[1], d.a[0], d.a[1], d.ctl, d.ring, d.partials, d.i_n, d.sq2,
                     d.cta_pending, d.regen_list, d.sync, d.nodes, (void*)d.lr_pref, d.f_th, d.th_next, (void*)d.th_dinc, d.th_cnt,
-                    d.th_list, d.th,
+                    d.th_cum, d.th_mask, d.th_val, d.th_w[0], d.th_w[1], d.th_list, d.th,
                     (void*)d.offp, h->scratch, h->red_partials, h->red_out, h->mkey, h->mflag, h->fs[0], h->fs[1],
                     h->fs[2], h->fs[3], h->fs[4], h->adj_sched, h->adj_ckpt, h->adj_ffsum, h->adj_final};
     for (void* p : ptrs) {
@@ -1454,7 +1465,8 @@ static int updated_inc(fqsb_system* h)
     if (!h->d.f_th) {
         return FQSB_OK;
     }
-    CU(h, launch_thermal_draw(h->d, 0, h->inc, h->stream));
+    CU(h, launch_thermal_plan(h->d, 1, TH_AT_INC, h->inc, h->stream));
+    CU(h, launch_thermal_commit(h->d, TH_COMMIT_NOW, h->stream));
     if (h->stored) {
         /* f from the stored components (f_damping is -eta v in the store) and the new f_thermal */
         k_store_damp<<<blocks_for(h->d.N, 128), 128, 0, h->stream>>>(h->d, cur_v(h), h->fs[0], h->fs[1], h->fs[2],
@@ -1496,12 +1508,23 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
                        "interactions");
     }
     const int64_t N = d.N;
-    const int64_t G = thermal_tiles(N);
-    double* f_th = nullptr;
-    int64_t *next = nullptr, *di = nullptr, *cnt = nullptr;
-    int32_t* list = nullptr;
+    /* steps planned ahead: bounded by the memory of their draws (2^24 values), one at least */
+    const int64_t K = std::max((int64_t)1, std::min(TH_STEPS_MAX, ((int64_t)1 << 24) / N));
+    const int64_t words = (N + 31) / 32;
+    double *f_th = nullptr, *val = nullptr, *w0 = nullptr, *w1 = nullptr;
+    int64_t *next = nullptr, *di = nullptr, *cnt = nullptr, *cum = nullptr, *list = nullptr;
+    uint32_t* mask = nullptr;
     Thermal* th = nullptr;
     cudaError_t e = cudaMalloc(&f_th, sizeof(double) * (size_t)padded(N));
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&w0, sizeof(double) * (size_t)N);
+    }
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&w1, sizeof(double) * (size_t)N);
+    }
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&val, sizeof(double) * (size_t)(K * N));
+    }
     if (e == cudaSuccess) {
         e = cudaMalloc(&next, sizeof(int64_t) * (size_t)N);
     }
@@ -1509,13 +1532,22 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         e = cudaMalloc(&di, sizeof(int64_t) * (size_t)N);
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&cnt, sizeof(int64_t) * (size_t)G);
+        e = cudaMalloc(&cnt, sizeof(int64_t) * (size_t)K);
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&list, sizeof(int32_t) * (size_t)N);
+        e = cudaMalloc(&cum, sizeof(int64_t) * (size_t)(K + 1));
+    }
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&list, sizeof(int64_t) * (size_t)(K * N));
+    }
+    if (e == cudaSuccess) {
+        e = cudaMalloc(&mask, sizeof(uint32_t) * (size_t)((K + 2) * words));
     }
     if (e == cudaSuccess) {
         e = cudaMalloc(&th, sizeof(Thermal));
+    }
+    if (e == cudaSuccess) {
+        e = cudaMemsetAsync(mask, 0, sizeof(uint32_t) * (size_t)((K + 2) * words), h->stream);
     }
     /* prrng pcg32(seed): the PCG seeding procedure on the default stream */
     Thermal t0;
@@ -1524,7 +1556,6 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     t0.state = t0.state * PCG_MULT + t0.inc;
     t0.state += seed;
     t0.state = t0.state * PCG_MULT + t0.inc;
-    t0.base = t0.state;
     t0.total = 0;
     t0.ticket = 0u;
     t0.pad = 0u;
@@ -1544,7 +1575,8 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         e = cudaStreamSynchronize(h->stream);
     }
     if (e != cudaSuccess) {
-        for (void* q : {(void*)f_th, (void*)next, (void*)di, (void*)cnt, (void*)list, (void*)th}) {
+        for (void* q : {(void*)f_th, (void*)w0, (void*)w1, (void*)val, (void*)next, (void*)di, (void*)cnt, (void*)cum,
+                        (void*)list, (void*)mask, (void*)th}) {
             if (q) {
                 cudaFree(q);
             }
@@ -1556,12 +1588,21 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     d.th_dinc = di;
     d.th_cnt = cnt;
     d.th_list = list;
+    d.th_cum = cum;
+    d.th_mask = mask;
+    d.th_val = val;
+    d.th_w[0] = w0;
+    d.th_w[1] = w1;
+    d.th_K = K;
+    d.th_words = words;
     d.th = th;
     d.th_mean = mean;
     d.th_sc = stddev * M_SQRT2; /* the association of the reference's normal transform */
-    /* the run graph's kernels take the new pointers; the one-cluster and run kernels have no thermal term */
-    h->rg = RunGeom{};
-    h->lg = line_geometry(N);
+    /* the run graph's kernels take the new pointers; few planned steps are not worth a launch of the run kernel */
+    if (K < 8) {
+        h->rg = RunGeom{};
+        h->lg = line_geometry(N);
+    }
     if (h->graph) {
         cudaGraphExecDestroy(h->graph);
         h->graph = nullptr;
@@ -1574,7 +1615,7 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         cudaGraphExecDestroy(h->graph_resid);
         h->graph_resid = nullptr;
     }
-    h->small_ok = false;
+    h->small_ok = h->small_ok && (h->sg.ctas <= 8 || small_cluster_fits(d, h->sg));
     int rc = updated_inc(h); /* the constructor's refresh */
     return rc ? rc : sync(h);
 }

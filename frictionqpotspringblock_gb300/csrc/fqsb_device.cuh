@@ -124,18 +124,18 @@ struct Ctl {
     double *rec_u, *rec_v, *rec_a;
     double4_32a* rec_w;
     double* rec_ffsum;
+    int64_t th_commit; /* steps of the plan of thermal draws that the launch has taken */
 };
 
 /*
  * RandomNormalForcing (detail.h:881-1000): the pcg32 stream all draws come from, in particle order
- * (prrng's pcg32 m_state / m_inc), and the bookkeeping of one draw: the state before it (base) and
- * the ticket of its counting kernel.
+ * (prrng's pcg32 m_state / m_inc), and the bookkeeping of a plan of draws: their number and the ticket
+ * of its counting kernel.
  */
 struct Thermal {
-    uint64_t state;
+    uint64_t state; /* before the planned draws */
     uint64_t inc;
-    uint64_t base;  /* state before the current draw */
-    int64_t total;  /* draws of the current draw */
+    int64_t total;  /* planned draws */
     uint32_t ticket;
     uint32_t pad;
 };
@@ -265,8 +265,14 @@ struct DevSys {
     double* f_th;       /* f_thermal [N] */
     int64_t* th_next;   /* next increment at which particle p redraws */
     const int64_t* th_dinc;
-    int64_t* th_cnt;    /* per 1024-particle tile: draws, then their exclusive prefix */
-    int32_t* th_list;   /* the drawing particles in flat order (capacity N) */
+    /* the draws of the next th_K steps (fqsb_thermal.cu); th_words = ceil(N / 32) words per step */
+    int64_t th_K, th_words;
+    uint32_t* th_mask;  /* [th_K + 2][th_words]: which particles draw; the last two rows stay 0 */
+    int64_t* th_cnt;    /* [th_K] draws per step */
+    int64_t* th_cum;    /* [th_K + 1] draws before a step */
+    int64_t* th_list;   /* the draws in order: step * N + particle (capacity th_K * N) */
+    double* th_val;     /* [th_K][N] the drawn forces */
+    double* th_w[2];    /* the run kernel's f_thermal after even and odd steps of a launch */
     Thermal* th;
     double th_mean, th_sc; /* mean and stddev * sqrt(2) (rounded as the reference's normal transform) */
 };

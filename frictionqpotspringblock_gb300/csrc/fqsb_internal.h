@@ -84,10 +84,21 @@ static const int NOPASS_MAX_REALIGN = 1 << 20; /* bound on one particle's well u
 cudaError_t build_nopass_graph(const DevSys& s, const LineGeom& g, const NopassArgs& A, cudaGraphExec_t* exec);
 cudaError_t launch_nopass_iteration(const DevSys& s, const LineGeom& g, const NopassArgs& A, cudaStream_t st);
 
-/* RandomNormalForcing draw (updated_inc): from_ctl = 1 for the step a run is about to make (inside
- * the run loop), else at increment `inc`.  thermal_tiles: size of DevSys::th_cnt. */
-cudaError_t launch_thermal_draw(const DevSys& s, int from_ctl, int64_t inc, cudaStream_t st);
-int64_t thermal_tiles(int64_t N);
+/*
+ * RandomNormalForcing (fqsb_thermal.cu).  A plan holds the draws of the next K steps, the first at the step a run
+ * is about to make (TH_FROM_RUN) or at increment `inc` (TH_AT_INC); it changes nothing of the system's state.
+ * Committing its first steps (all of a one-step plan; those that the launch has taken, Ctl::th_commit) updates
+ * f_thermal, the next increments and the stream.
+ */
+enum : int { TH_AT_INC = 0, TH_FROM_RUN = 1 };
+enum : int { TH_COMMIT_NOW = 0, TH_COMMIT_ONE = 1, TH_COMMIT_RUN = 2 };
+static const int64_t TH_STEPS_MAX = 256;
+cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, int from, int64_t inc, cudaStream_t st);
+cudaError_t launch_thermal_commit(const DevSys& s, int what, cudaStream_t st);
+/* the same as nodes of a graph: the plan first in `body` (its last node in *node), the commit after *dep */
+cudaError_t add_thermal_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K);
+cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s,
+                               int what);
 
 /* One loop iteration launched kernel by kernel by the host (s.in_graph must be 0). */
 cudaError_t launch_iteration(const DevSys& s, const LineGeom& g, cudaStream_t st);

@@ -196,11 +196,13 @@ struct Strip {
  * One time step of the strip of particles p0 .. p0 + n - 1 (n <= S) by one warp; returns the strip's sums
  * of f^2 and f_frame^2 (or of f_frame) in lane 0.
  */
-template <int POT, int INTER, int MODE>
+template <int POT, int INTER, int MODE, bool TH>
 __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, int64_t p0, int n, int cur, double uf,
                                               int flags, int64_t step, int64_t t, bool& pending, int64_t* moved)
 {
-    constexpr unsigned SOFT = STEP_SOFT;
+    /* one more addition on the integer pipes where they do not also square the residual: at N = 2^22 142 us per
+     * step instead of 144 us, but 173 us instead of 169 us with the squares */
+    constexpr unsigned SOFT = MODE == KMODE_PLAIN ? STEP_SOFT | (1u << 11) : STEP_SOFT;
     const int lane = threadIdx.x & 31;
     const bool general = MODE == KMODE_GENERAL;
     const bool act = general && (flags & (RF_ACT | RF_TRUNCATE | RF_EVENT)) != 0;
@@ -309,7 +311,15 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
             sfi = add_zero(sfi);
         }
         double vn, an, f;
-        verlet_velocity<SOFT>(s, sfi, st.v[k], a, vn, an, f);
+        double fth = 0.0;
+        if (TH && k < n) {
+            /* the planned draw of step t, or the force of the step before */
+            const uint32_t draw = __ldcg(s.th_mask + t * s.th_words + (p >> 5));
+            fth = draw >> (p & 31) & 1u ? __ldcg(s.th_val + t * N + p)
+                                        : __ldcg((t == 0 ? s.f_th : s.th_w[(t - 1) & 1]) + p);
+            s.th_w[t & 1][p] = fth;
+        }
+        verlet_velocity<SOFT, TH>(s, sfi, st.v[k], a, vn, an, f, fth);
         if (k < n) {
             v1[p] = vn;
             a1[p] = an;
@@ -340,6 +350,13 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
     return sum;
 }
 
+/* Steps that a launch takes at most: those the run has left, and with thermal forcing those planned */
+__device__ __forceinline__ int64_t steps_of_launch(const DevSys& s)
+{
+    const int64_t left = s.ctl->max_steps - s.ctl->step;
+    return s.f_th && s.th_K < left ? s.th_K : left;
+}
+
 /* The CTA without strips: sums and stop tests of each step, one step behind the others */
 static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& g)
 {
@@ -353,7 +370,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     const int flags = s.ctl->flags;
     const bool tree = (flags & (RF_RESID | RF_FFSUM)) != 0;
     const unsigned long long base = y->base;
-    const int64_t left = s.ctl->max_steps - s.ctl->step, step0 = s.ctl->step;
+    const int64_t left = steps_of_launch(s), step0 = s.ctl->step;
     const double vdt = s.ctl->vdt;
     const int64_t nring = (flags & RF_RESID) ? s.ctl->niter_tol : 0;
     const bool shared_ring = nring <= RUN_RING;
@@ -461,6 +478,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
             vy->da[k] = 0;
         }
         vy->base = base + (unsigned long long)(t + 1) * gridDim.x;
+        sc.th_commit = how == END_BARRIER ? 0 : how == END_STOPPED ? t : t + 1;
         *s.ctl = sc;
         const bool more = !sc.done && !sc.error && (sc.launch_steps == 0 || globaltimer() - sc.launch_t0 < sc.budget_ns);
         __threadfence();
@@ -469,7 +487,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     }
 }
 
-template <int POT, int INTER, int MODE>
+template <int POT, int INTER, int MODE, bool TH>
 __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     k_run_line(const __grid_constant__ DevSys s, const __grid_constant__ RunGeom g)
 {
@@ -478,6 +496,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     __shared__ int64_t moved_sh; /* 1 + the last step in which a particle of this CTA changed its well */
     if (s.ctl->done || s.ctl->error) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
+            s.ctl->th_commit = 0;
             set_branch(s, 0u);
             set_loop(s, 0u);
         }
@@ -499,7 +518,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     const unsigned long long base = y->base;
     const int flags = s.ctl->flags;
     const int cur0 = s.ctl->cur;
-    const int64_t step0 = s.ctl->step, left = s.ctl->max_steps - step0;
+    const int64_t step0 = s.ctl->step, left = steps_of_launch(s);
     const double vdt = s.ctl->vdt;
     const double* sched = s.ctl->sched;
     const bool tree = MODE == KMODE_RESID || (MODE == KMODE_GENERAL && (flags & (RF_RESID | RF_FFSUM)) != 0);
@@ -530,7 +549,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
         for (int64_t k = s0 + wid; k < s1;) {
             const int64_t p0 = k * S;
             bool pending;
-            const double2 sum = strip_step<POT, INTER, MODE>(s, st, p0, (int)(s.N - p0 < S ? s.N - p0 : S), cur0 ^ q, uf,
+            const double2 sum = strip_step<POT, INTER, MODE, TH>(s, st, p0, (int)(s.N - p0 < S ? s.N - p0 : S), cur0 ^ q, uf,
                                                              flags, step0 + t, t, pending, &moved_sh);
             if (lane == 0) {
                 if (tree) {
@@ -592,13 +611,21 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
 template <int POT, int INTER>
 static const void* run_kernel_t(int mode)
 {
-    return mode == KMODE_PLAIN   ? (const void*)k_run_line<POT, INTER, KMODE_PLAIN>
-           : mode == KMODE_RESID ? (const void*)k_run_line<POT, INTER, KMODE_RESID>
-                                 : (const void*)k_run_line<POT, INTER, KMODE_GENERAL>;
+    return mode == KMODE_PLAIN   ? (const void*)k_run_line<POT, INTER, KMODE_PLAIN, false>
+           : mode == KMODE_RESID ? (const void*)k_run_line<POT, INTER, KMODE_RESID, false>
+                                 : (const void*)k_run_line<POT, INTER, KMODE_GENERAL, false>;
 }
 
 const void* run_kernel(const DevSys& s, int mode)
 {
+    if (s.f_th) {
+        /* RandomNormalForcing systems: Cuspy with Laplace1d, Quartic1d or no interactions */
+        switch (s.inter) {
+            case INTER_LAPLACE1D: return (const void*)k_run_line<POT_CUSPY, INTER_LAPLACE1D, KMODE_GENERAL, true>;
+            case INTER_QUARTIC1D: return (const void*)k_run_line<POT_CUSPY, INTER_QUARTIC1D, KMODE_GENERAL, true>;
+            default: return (const void*)k_run_line<POT_CUSPY, INTER_NONE, KMODE_GENERAL, true>;
+        }
+    }
     switch (s.inter) {
         case INTER_QUARTIC1D: return run_kernel_t<POT_CUSPY, INTER_QUARTIC1D>(mode);
         case INTER_QUARTICGRAD1D: return run_kernel_t<POT_CUSPY, INTER_QUARTICGRAD1D>(mode);
@@ -616,7 +643,7 @@ const void* run_kernel(const DevSys& s, int mode)
 RunGeom run_geometry(const DevSys& s)
 {
     RunGeom g = {};
-    if (!(inter_ring(s.inter) || s.inter == INTER_NONE) || s.f_th) {
+    if (!(inter_ring(s.inter) || s.inter == INTER_NONE)) {
         return g;
     }
     int dev = 0, sms = 0, coop = 0;

@@ -850,187 +850,6 @@ cudaError_t launch_next_window(const DevSys& s, cudaStream_t st)
     return cudaGetLastError();
 }
 
-/* ------------------------------------------------------------- thermal forcing */
-
-/*
- * RandomNormalForcing::force (detail.h:930-942), run by updated_inc at the start of every time step
- * (timeStep :1540-1544) and by refresh / set_inc: in particle order, every particle with inc >= next[p]
- * takes the next draw of one pcg32 stream, f_thermal[p] = mean + (stddev sqrt 2) erfinv(2 r - 1)
- * (r = u32 2^-32), and next[p] += dinc[p].  The draws are numbered by an exclusive scan over the flat
- * index: k_th_count counts each 1024-particle tile's draws and its last CTA turns the counts into
- * tile offsets and jumps the stream past the whole draw; k_th_list writes each drawing particle to
- * its rank in a compact list; k_th_eval gives list entry k the k-th output after the old state (a
- * jump-ahead per entry) with one thread per draw, so the erfinv work is dense whatever the fraction
- * of particles that draw, and the result equals the reference's sequential loop.
- *
- * from_ctl = 1: inside a run, for the step about to run (inc = Ctl::inc + 1); nothing happens once the
- * run is over or when the run's iterations are not time steps.  from_ctl = 0: at inc = inc_arg.
- */
-constexpr int TH_TILE = 1024; /* particles per CTA of the draw kernels: 256 threads x 4 */
-
-__device__ __forceinline__ bool th_draw_inc(const DevSys& s, int from_ctl, int64_t inc_arg, int64_t& inc)
-{
-    if (!from_ctl) {
-        inc = inc_arg;
-        return true;
-    }
-    volatile Ctl* c = s.ctl;
-    if (c->done || c->error || (c->flags & RF_NOINC)) {
-        return false;
-    }
-    inc = c->inc + 1;
-    return true;
-}
-
-/* Exclusive prefix of x over the CTA's 256 threads (8 warps); *total gets the CTA's sum. */
-__device__ __forceinline__ int64_t cta_exclusive_scan256(int64_t x, int64_t* sh8, int64_t* total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) {
-            incl += y;
-        }
-    }
-    if (lane == 31) {
-        sh8[warp] = incl;
-    }
-    __syncthreads();
-    int64_t before = 0, all = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        int64_t t = sh8[w];
-        before += w < warp ? t : 0;
-        all += t;
-    }
-    __syncthreads();
-    *total = all;
-    return before + incl - x;
-}
-
-__global__ void __launch_bounds__(256) k_th_count(DevSys s, int from_ctl, int64_t inc_arg)
-{
-    __shared__ int64_t sh8[8];
-    __shared__ int sh_last;
-    int64_t inc;
-    if (!th_draw_inc(s, from_ctl, inc_arg, inc)) {
-        return;
-    }
-    const int64_t p0 = (int64_t)blockIdx.x * TH_TILE + (int64_t)threadIdx.x * 4;
-    int64_t n = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        int64_t p = p0 + j;
-        n += (p < s.N && inc >= s.th_next[p]) ? 1 : 0;
-    }
-    int64_t tile_total;
-    cta_exclusive_scan256(n, sh8, &tile_total);
-    if (threadIdx.x == 0) {
-        s.th_cnt[blockIdx.x] = tile_total;
-        __threadfence();
-        unsigned t = atomicAdd(&s.th->ticket, 1u);
-        sh_last = (t == gridDim.x - 1u) ? 1 : 0;
-    }
-    __syncthreads();
-    if (!sh_last) {
-        return;
-    }
-    /* last CTA: tile counts -> exclusive tile offsets (in place), the stream jumps past all draws */
-    __threadfence();
-    const int64_t G = gridDim.x;
-    const int64_t per = (G + 255) / 256;
-    const int64_t lo = (int64_t)threadIdx.x * per;
-    const int64_t hi = lo + per < G ? lo + per : G;
-    int64_t sum = 0;
-    for (int64_t i = lo; i < hi; ++i) {
-        sum += __ldcg(s.th_cnt + i);
-    }
-    int64_t all;
-    int64_t run = cta_exclusive_scan256(sum, sh8, &all);
-    for (int64_t i = lo; i < hi; ++i) {
-        int64_t x = __ldcg(s.th_cnt + i);
-        s.th_cnt[i] = run;
-        run += x;
-    }
-    if (threadIdx.x == 0) {
-        Thermal* th = s.th;
-        uint64_t base = th->state;
-        th->base = base;
-        th->total = all;
-        th->state = pcg_advance_inc(base, (uint64_t)all, th->inc);
-        th->ticket = 0u;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_th_list(DevSys s, int from_ctl, int64_t inc_arg)
-{
-    __shared__ int64_t sh8[8];
-    int64_t inc;
-    if (!th_draw_inc(s, from_ctl, inc_arg, inc)) {
-        return;
-    }
-    const int64_t p0 = (int64_t)blockIdx.x * TH_TILE + (int64_t)threadIdx.x * 4;
-    bool draw[4];
-    int64_t n = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        int64_t p = p0 + j;
-        draw[j] = p < s.N && inc >= s.th_next[p];
-        n += draw[j] ? 1 : 0;
-    }
-    int64_t tile_total;
-    int64_t k = s.th_cnt[blockIdx.x] + cta_exclusive_scan256(n, sh8, &tile_total);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if (draw[j]) {
-            s.th_list[k++] = (int32_t)(p0 + j);
-        }
-    }
-}
-
-/* One thread per draw: entry k of the list takes output k of the stream after the old state. */
-__global__ void __launch_bounds__(128) k_th_eval(DevSys s, int from_ctl, int64_t inc_arg)
-{
-    int64_t inc;
-    if (!th_draw_inc(s, from_ctl, inc_arg, inc)) {
-        return;
-    }
-    const int64_t total = s.th->total;
-    const uint64_t base = s.th->base, sinc = s.th->inc;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t p = s.th_list[k];
-        const uint32_t u32 = pcg_output(pcg_advance_inc(base, (uint64_t)k, sinc));
-        const double r = FQ_MUL((double)u32, 0x1p-32);
-        const double z = fq_erfinv(FQ_SUB(FQ_MUL(2.0, r), 1.0));
-        s.f_th[p] = FQ_ADD(s.th_mean, FQ_MUL(s.th_sc, z));
-        s.th_next[p] += s.th_dinc[p];
-    }
-}
-
-/* CTAs of k_th_eval (72 registers, 128 threads): 4 per SM, 78 k draws per pass, grid-stride beyond */
-constexpr unsigned TH_EVAL_CTAS = 4 * 152;
-
-cudaError_t launch_thermal_draw(const DevSys& s, int from_ctl, int64_t inc, cudaStream_t st)
-{
-    unsigned G = (unsigned)((s.N + TH_TILE - 1) / TH_TILE);
-    void* args[] = {(void*)&s, (void*)&from_ctl, (void*)&inc};
-    cudaError_t e = cudaLaunchKernel((void*)k_th_count, dim3(G), dim3(256), args, 0, st);
-    if (e == cudaSuccess) {
-        e = cudaLaunchKernel((void*)k_th_list, dim3(G), dim3(256), args, 0, st);
-    }
-    if (e == cudaSuccess) {
-        e = cudaLaunchKernel((void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), args, 0, st);
-    }
-    return e;
-}
-
-int64_t thermal_tiles(int64_t N)
-{
-    return (N + TH_TILE - 1) / TH_TILE;
-}
-
 /* ------------------------------------------------------------- long-range interactions */
 
 /*
@@ -1344,7 +1163,7 @@ __device__ __forceinline__ double2 particle_tree2(double x, double y, double* sh
     return make_double2(x, y);
 }
 
-template <int POT, int INTER, int PPT>
+template <int POT, int INTER, int PPT, bool TH>
 __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const __grid_constant__ DevSys s)
 {
     namespace cg = cooperative_groups;
@@ -1366,6 +1185,13 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
     __shared__ FwdMove sh_moves[SMALL_MOVES];
     __shared__ int sh_nmove;
 
+    if (TH && (s.ctl->done || s.ctl->error)) {
+        /* launched beside others that ended the run (no CTA writes the control block before all have read it) */
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            s.ctl->th_commit = 0;
+        }
+        return;
+    }
     const unsigned rank = cluster.block_rank();
     const unsigned G = cluster.num_blocks();
     const int tid = threadIdx.x;
@@ -1439,12 +1265,27 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
         pa[j] = a[j];
         pstart[j] = 0;
     }
+    /* thermal forces: the values in use, and what step t + 1 draws, loaded a step ahead (planned draws) */
+    double fth[PPT], fnew[PPT];
+    uint32_t draw = 0u, draw_next = 0u;
+    const uint32_t* th_mask = TH ? s.th_mask + (p0 < N ? p0 >> 5 : 0) : nullptr;
+    if (TH && !ctrl) {
+        draw = p0 < N ? th_mask[0] : 0u;
+        draw_next = p0 < N ? th_mask[s.th_words] : 0u;
+#pragma unroll
+        for (int j = 0; j < PPT; ++j) {
+            const int64_t p = p0 + j;
+            fth[j] = p < N ? s.f_th[p] : 0.0;
+            fnew[j] = p < N && (draw >> (p & 31) & 1u) ? s.th_val[p] : 0.0;
+        }
+    }
     /* one particle per thread: latency bound, all fp64 on the fp64 pipe; more: throughput bound, split */
     constexpr unsigned SOFT = PPT >= 2 ? STEP_SOFT : 0u;
     /* pcg32 stride of pt steps, x -> mv_a x + mv_c, for the shared draws of window moves */
     const uint64_t mv_c = pcg_advance(0ULL, (uint64_t)pt);
     const uint64_t mv_a = pcg_advance(1ULL, (uint64_t)pt) - mv_c;
     int buf = 0;
+    int64_t steps_taken = 0;
     double uf_prev = uf;
     for (int64_t t = 0;; ++t) {
         const double uf_t = (flags & RF_FLOW) ? FQ_ADD(uf, vdt) : uf;
@@ -1468,6 +1309,7 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
         cluster.sync();
         if (t >= 2 && sl_stop0[t & 1]) {
             /* stopped after step t - 2: restore the state before step t - 1 */
+            steps_taken = t - 1;
             if (!ctrl) {
 #pragma unroll
                 for (int j = 0; j < PPT; ++j) {
@@ -1534,7 +1376,10 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
                     sl_nan[q] = 0;
                     sl_walk[q] = 0;
                     finalize_ctl(&sc, sring, uf_last, tx, ty);
-                    sl_stop[q] = (sc.done || sc.error || (globaltimer() - sc.launch_t0) >= sc.budget_ns) ? 1 : 0;
+                    sl_stop[q] = (sc.done || sc.error || (globaltimer() - sc.launch_t0) >= sc.budget_ns ||
+                                  (TH && t >= s.th_K))
+                                     ? 1
+                                     : 0;
                 }
             }
             buf ^= 1;
@@ -1687,7 +1532,16 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
                 sfi = add_zero(sfi);
             }
             double vn, an, f;
-            verlet_velocity<SOFT>(s, sfi, v[j], a[j], vn, an, f);
+            if (TH) {
+                /* step t's draw, then the loads for step t + 1 (row th_K of the plan is empty) */
+                if (draw >> (p & 31) & 1u) {
+                    fth[j] = fnew[j];
+                }
+                if (draw_next >> (p & 31) & 1u) {
+                    fnew[j] = s.th_val[(t + 1) * N + p];
+                }
+            }
+            verlet_velocity<SOFT, TH>(s, sfi, v[j], a[j], vn, an, f, TH ? fth[j] : 0.0);
             u[j] = up;
             v[j] = vn;
             a[j] = an;
@@ -1702,6 +1556,10 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
                     rff = add_nospec(rff, ff2);
                 }
             }
+        }
+        if (TH) {
+            draw = draw_next;
+            draw_next = p0 < N ? th_mask[(t + 2 < s.th_K ? t + 2 : s.th_K) * s.th_words] : 0u;
         }
         if (nan) {
             sh_nan = 1;
@@ -1749,6 +1607,9 @@ __global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const _
             s.ring[i] = sring[i];
         }
         if (tid == 0) {
+            if (TH) {
+                sc.th_commit = steps_taken;
+            }
             *s.ctl = sc;
         }
     }
@@ -1771,18 +1632,26 @@ SmallGeom small_geometry(int64_t N, int max_ctas)
     return g;
 }
 
-template <int POT, int INTER>
+template <int POT, int INTER, bool TH = false>
 static const void* small_kernel_t(int ppt)
 {
     switch (ppt) {
-        case 1: return (const void*)k_run_small<POT, INTER, 1>;
-        case 2: return (const void*)k_run_small<POT, INTER, 2>;
-        default: return (const void*)k_run_small<POT, INTER, 4>;
+        case 1: return (const void*)k_run_small<POT, INTER, 1, TH>;
+        case 2: return (const void*)k_run_small<POT, INTER, 2, TH>;
+        default: return (const void*)k_run_small<POT, INTER, 4, TH>;
     }
 }
 
 static const void* small_kernel(const DevSys& s, const SmallGeom& g)
 {
+    if (s.f_th) {
+        /* RandomNormalForcing systems: Cuspy with Laplace1d, Quartic1d or no interactions */
+        switch (s.inter) {
+            case INTER_LAPLACE1D: return small_kernel_t<POT_CUSPY, INTER_LAPLACE1D, true>(g.ppt);
+            case INTER_QUARTIC1D: return small_kernel_t<POT_CUSPY, INTER_QUARTIC1D, true>(g.ppt);
+            default: return small_kernel_t<POT_CUSPY, INTER_NONE, true>(g.ppt);
+        }
+    }
     /* the Quartic interactions exist with the Cuspy potential only (Line1d.h:428, :562) */
     if (s.inter == INTER_QUARTIC1D) {
         return small_kernel_t<POT_CUSPY, INTER_QUARTIC1D>(g.ppt);
@@ -1993,7 +1862,10 @@ cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t s
     void* argsr[] = {(void*)&s};
     cudaError_t e = cudaSuccess;
     if (s.f_th) {
-        e = launch_thermal_draw(s, 1, 0, st);
+        e = launch_thermal_plan(s, 1, TH_FROM_RUN, 0, st);
+        if (e == cudaSuccess) {
+            e = launch_thermal_commit(s, TH_COMMIT_ONE, st);
+        }
     }
     if (e == cudaSuccess && s.inter == INTER_LONGRANGE1D) {
         e = cudaLaunchKernel((void*)k_lr_position, dim3((unsigned)((s.N + 255) / 256)), dim3(256), argsr, 0, st);
@@ -2059,17 +1931,12 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
     void* args2[] = {(void*)&s, (void*)&pass2};
     void* argsr[] = {(void*)&s};
     cudaGraphNode_t nstep, nif;
-    int th_from_ctl = 1;
-    int64_t th_inc = 0;
-    void* argst[] = {(void*)&s, (void*)&th_from_ctl, (void*)&th_inc};
-    if (s.f_th) {
+    if (s.f_th && !rg.ctas) {
         /* updated_inc of the step: thermal draws before the step's forces */
-        cudaGraphNode_t ncount, nlist, neval;
-        dim3 gth((unsigned)thermal_tiles(s.N));
-        GR(add_kernel(&ncount, body, nullptr, 0, (void*)k_th_count, gth, dim3(256), argst));
-        GR(add_kernel(&nlist, body, &ncount, 1, (void*)k_th_list, gth, dim3(256), argst));
-        GR(add_kernel(&neval, body, &nlist, 1, (void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), argst));
-        GR(add_kernel(&nstep, body, &neval, 1, fstep, grid, block, args1));
+        cudaGraphNode_t ndraw;
+        GR(add_thermal_plan(&ndraw, body, s, 1));
+        GR(add_thermal_commit(&ndraw, body, &ndraw, s, TH_COMMIT_ONE));
+        GR(add_kernel(&nstep, body, &ndraw, 1, fstep, grid, block, args1));
     }
     else if (s.inter == INTER_LONGRANGE1D) {
         /* all new positions before the all-pairs interaction */
@@ -2088,10 +1955,18 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
         kp.sharedMemBytes = (unsigned)rg.smem;
         GR(cudaFuncSetAttribute(kp.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rg.smem));
         kp.kernelParams = argsl;
-        GR(cudaGraphAddKernelNode(&nstep, body, nullptr, 0, &kp));
+        cudaGraphNode_t nplan;
+        if (s.f_th) {
+            /* the thermal draws of the launch's steps ahead of it */
+            GR(add_thermal_plan(&nplan, body, s, s.th_K));
+        }
+        GR(cudaGraphAddKernelNode(&nstep, body, s.f_th ? &nplan : nullptr, s.f_th ? 1 : 0, &kp));
         cudaKernelNodeAttrValue coop = {};
         coop.cooperative = 1;
         GR(cudaGraphKernelNodeSetAttribute(nstep, cudaLaunchAttributeCooperative, &coop));
+        if (s.f_th) {
+            GR(add_thermal_commit(&nstep, body, &nstep, s, TH_COMMIT_RUN));
+        }
     }
     else {
         GR(add_kernel(&nstep, body, nullptr, 0, fstep, grid, block, args1));

@@ -1,0 +1,269 @@
+/*
+ * RandomNormalForcing::force (detail.h:930-942), run by updated_inc at the start of every time step
+ * (timeStep :1540-1544) and by refresh / set_inc: in particle order, every particle with inc >= next[p]
+ * takes the next draw of one pcg32 stream, f_thermal[p] = mean + (stddev sqrt 2) erfinv(2 r - 1)
+ * (r = u32 2^-32), and next[p] += dinc[p].
+ *
+ * Which particles draw when does not depend on the dynamics, so the draws of many steps are made ahead of
+ * them (a plan): k_th_mask marks who draws in each step, k_th_count numbers the draws (step by step, in
+ * particle order), k_th_list lists them, and k_th_eval computes one per thread from the stream's state
+ * jumped ahead, so that the erfinv work (600 fp64 operations, one after the other) is dense and not in the
+ * path of a step.  The run kernels then only read the drawn forces.  k_th_commit makes the steps that a
+ * launch has taken the system's state (f_thermal, next, the stream); a step that the launch dropped is
+ * planned again.  Per time step of 1000 particles, each redrawn every 100 steps: 46.4 us with the draws
+ * of each step made before it (four launches in the run graph's loop), 3.1 us planned for 256 steps and
+ * taken by the one-cluster kernel.
+ */
+#include "fqsb_stepcore.cuh"
+
+namespace fqsb {
+
+/* The increment of the plan's first step, and in K its steps (no more than the run has left); false when the
+ * run is over or takes no time steps. */
+__device__ __forceinline__ bool th_first_inc(const DevSys& s, int from, int64_t inc_arg, int64_t& inc, int& K)
+{
+    if (from == TH_AT_INC) {
+        inc = inc_arg;
+        return true;
+    }
+    const volatile Ctl* c = s.ctl;
+    if (c->done || c->error || (c->flags & RF_NOINC)) {
+        return false;
+    }
+    inc = c->inc + 1;
+    const int64_t left = c->max_steps - c->step;
+    K = left < K ? (int)left : K;
+    return true;
+}
+
+__global__ void __launch_bounds__(256) k_th_mask(const __grid_constant__ DevSys s, int K, int from, int64_t inc_arg)
+{
+    int64_t inc;
+    if (!th_first_inc(s, from, inc_arg, inc, K)) {
+        return;
+    }
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t next = 0, dinc = 0;
+    if (p < s.N) {
+        next = s.th_next[p];
+        dinc = s.th_dinc[p];
+    }
+    for (int k = 0; k < K; ++k) {
+        const bool draw = p < s.N && inc + k >= next;
+        next += draw ? dinc : 0;
+        const unsigned word = __ballot_sync(0xffffffffu, draw);
+        if ((threadIdx.x & 31) == 0 && p < s.N) {
+            s.th_mask[(int64_t)k * s.th_words + (p >> 5)] = word;
+        }
+    }
+}
+
+/* Exclusive prefix of x over the CTA's 256 threads (8 warps); *total gets the CTA's sum. */
+__device__ __forceinline__ int64_t cta_exclusive_scan256(int64_t x, int64_t* sh8, int64_t* total)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) {
+            incl += y;
+        }
+    }
+    if (lane == 31) {
+        sh8[warp] = incl;
+    }
+    __syncthreads();
+    int64_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        int64_t t = sh8[w];
+        before += w < warp ? t : 0;
+        all += t;
+    }
+    __syncthreads();
+    *total = all;
+    return before + incl - x;
+}
+
+/* One CTA per planned step counts its draws; the last one turns the counts into the draws before each step. */
+__global__ void __launch_bounds__(256) k_th_count(const __grid_constant__ DevSys s, int K, int from, int64_t inc_arg)
+{
+    __shared__ int64_t sh8[8];
+    __shared__ int sh_last;
+    int64_t inc;
+    if (!th_first_inc(s, from, inc_arg, inc, K)) {
+        return;
+    }
+    const uint32_t* row = s.th_mask + (int64_t)blockIdx.x * s.th_words;
+    int64_t n = 0, total;
+    for (int64_t i = threadIdx.x; (int)blockIdx.x < K && i < s.th_words; i += 256) {
+        n += __popc(row[i]);
+    }
+    cta_exclusive_scan256(n, sh8, &total);
+    if (threadIdx.x == 0) {
+        s.th_cnt[blockIdx.x] = total;
+        __threadfence();
+        sh_last = atomicAdd(&s.th->ticket, 1u) == gridDim.x - 1u ? 1 : 0;
+    }
+    __syncthreads();
+    if (!sh_last) {
+        return;
+    }
+    __threadfence();
+    const int64_t x = (int)threadIdx.x < K ? __ldcg(s.th_cnt + threadIdx.x) : 0;
+    const int64_t before = cta_exclusive_scan256(x, sh8, &total);
+    if ((int)threadIdx.x < K) {
+        s.th_cum[threadIdx.x] = before;
+    }
+    if (threadIdx.x == 0) {
+        s.th_cum[K] = total;
+        s.th->total = total;
+        s.th->ticket = 0u;
+    }
+}
+
+/* One CTA per planned step lists its draws in particle order. */
+__global__ void __launch_bounds__(256) k_th_list(const __grid_constant__ DevSys s, int K, int from, int64_t inc_arg)
+{
+    __shared__ int64_t sh8[8];
+    int64_t inc;
+    if (!th_first_inc(s, from, inc_arg, inc, K)) {
+        return;
+    }
+    if ((int)blockIdx.x >= K) {
+        return;
+    }
+    const uint32_t* row = s.th_mask + (int64_t)blockIdx.x * s.th_words;
+    int64_t base = s.th_cum[blockIdx.x];
+    for (int64_t w0 = 0; w0 < s.th_words; w0 += 256) {
+        const int64_t w = w0 + threadIdx.x;
+        uint32_t word = w < s.th_words ? row[w] : 0u;
+        int64_t total;
+        int64_t k = base + cta_exclusive_scan256(__popc(word), sh8, &total);
+        for (; word; word &= word - 1u) {
+            s.th_list[k++] = (int64_t)blockIdx.x * s.N + 32 * w + (__ffs((int)word) - 1);
+        }
+        base += total;
+    }
+}
+
+/* One thread per draw: entry k of the list takes output k of the stream. */
+__global__ void __launch_bounds__(128) k_th_eval(const __grid_constant__ DevSys s, int from, int64_t inc_arg)
+{
+    int64_t inc;
+    int K = 0;
+    if (!th_first_inc(s, from, inc_arg, inc, K)) {
+        return;
+    }
+    const int64_t total = s.th->total;
+    const uint64_t state = s.th->state, sinc = s.th->inc;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t u32 = pcg_output(pcg_advance_inc(state, (uint64_t)k, sinc));
+        const double r = FQ_MUL((double)u32, 0x1p-32);
+        const double z = fq_erfinv(FQ_SUB(FQ_MUL(2.0, r), 1.0));
+        s.th_val[s.th_list[k]] = FQ_ADD(s.th_mean, FQ_MUL(s.th_sc, z));
+    }
+}
+
+__global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSys s, int what)
+{
+    const volatile Ctl* c = s.ctl;
+    int64_t steps = 1;
+    if (what == TH_COMMIT_RUN) {
+        steps = c->th_commit;
+    }
+    else if (what == TH_COMMIT_ONE && (c->done || c->error || (c->flags & RF_NOINC))) {
+        steps = 0;
+    }
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < s.N) {
+        int64_t draws = 0, last = -1;
+        for (int64_t k = 0; k < steps; ++k) {
+            if (s.th_mask[k * s.th_words + (p >> 5)] >> (p & 31) & 1u) {
+                ++draws;
+                last = k;
+            }
+        }
+        if (draws) {
+            s.f_th[p] = s.th_val[last * s.N + p];
+            s.th_next[p] += draws * s.th_dinc[p];
+        }
+    }
+    if (p == 0 && steps > 0) {
+        Thermal* th = s.th;
+        th->state = pcg_advance_inc(th->state, (uint64_t)s.th_cum[steps], th->inc);
+    }
+}
+
+/* CTAs of k_th_eval (72 registers, 128 threads): 4 per SM, 78 k draws per pass, grid-stride beyond */
+constexpr unsigned TH_EVAL_CTAS = 4 * 152;
+
+struct ThLaunch {
+    void* f;
+    dim3 grid, block;
+    void** args;
+};
+
+template <class F>
+static cudaError_t for_plan(const DevSys& s, int64_t K, int from, int64_t inc, F launch)
+{
+    int k = (int)K;
+    void* args[] = {(void*)&s, (void*)&k, (void*)&from, (void*)&inc};
+    void* args_eval[] = {(void*)&s, (void*)&from, (void*)&inc};
+    const dim3 parts((unsigned)((s.N + 255) / 256)), steps((unsigned)K);
+    const ThLaunch all[4] = {{(void*)k_th_mask, parts, dim3(256), args},
+                             {(void*)k_th_count, steps, dim3(256), args},
+                             {(void*)k_th_list, steps, dim3(256), args},
+                             {(void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), args_eval}};
+    for (const ThLaunch& l : all) {
+        const cudaError_t e = launch(l);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, int from, int64_t inc, cudaStream_t st)
+{
+    return for_plan(s, K, from, inc, [&](const ThLaunch& l) { return cudaLaunchKernel(l.f, l.grid, l.block, l.args, 0, st); });
+}
+
+cudaError_t launch_thermal_commit(const DevSys& s, int what, cudaStream_t st)
+{
+    k_th_commit<<<(unsigned)((s.N + 255) / 256), 256, 0, st>>>(s, what);
+    return cudaGetLastError();
+}
+
+static cudaError_t add_node(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const ThLaunch& l)
+{
+    cudaKernelNodeParams kp = {};
+    kp.func = l.f;
+    kp.gridDim = l.grid;
+    kp.blockDim = l.block;
+    kp.kernelParams = l.args;
+    cudaGraphNode_t n;
+    const cudaError_t e = cudaGraphAddKernelNode(&n, body, dep, dep ? 1 : 0, &kp);
+    *node = n;
+    return e;
+}
+
+cudaError_t add_thermal_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K)
+{
+    bool first = true;
+    return for_plan(s, K, TH_FROM_RUN, 0, [&](const ThLaunch& l) {
+        const cudaError_t e = add_node(node, body, first ? nullptr : node, l);
+        first = false;
+        return e;
+    });
+}
+
+cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s,
+                               int what)
+{
+    void* args[] = {(void*)&s, (void*)&what};
+    return add_node(node, body, dep, {(void*)k_th_commit, dim3((unsigned)((s.N + 255) / 256)), dim3(256), args});
+}
+
+} // namespace fqsb
