@@ -240,18 +240,17 @@ __device__ static const double fq_log_tab_dev[FQ_LOG_N][4] = FQ_LOG_TABLE_INIT;
 static const double fq_log_tab_host[FQ_LOG_N][4] = FQ_LOG_TABLE_INIT;
 
 /*
- * Quick phases.  log and sin below first compute a double-double hi + lo of relative error below
- * FQ_QUICK_ERR in a fraction of the operations of the full evaluation, and round it when every value
- * within that error rounds alike (Ziv, "Fast evaluation of elementary mathematical functions with
- * correctly rounded last bit", 1991); else (about once in 2^10) they evaluate in full.  The full
- * evaluation's own error is far smaller, so where the quick phase rounds, it rounds to the same double.
+ * Quick phases.  log and sin below first compute a double-double hi + lo of a known relative error in a
+ * fraction of the operations of the full evaluation, and round it when every value within that error
+ * rounds alike (Ziv, "Fast evaluation of elementary mathematical functions with correctly rounded last
+ * bit", 1991); else they evaluate in full.  The bounds cover the full evaluation's own error as well, so where
+ * the quick phase rounds, it rounds to the same double.
  */
-#define FQ_QUICK_ERR 0x1p-64
 
-/* hi + lo rounded, if certain */
-FQ_HD int fq_quick_round(double hi, double lo, double* y)
+/* hi + lo rounded, if certain with a relative error below eps */
+FQ_HD int fq_quick_round(double hi, double lo, double eps, double* y)
 {
-    const double e = FQ_MUL(hi, FQ_QUICK_ERR);
+    const double e = FQ_MUL(hi, eps);
     const double y0 = FQ_ADD(hi, FQ_SUB(lo, e)), y1 = FQ_ADD(hi, FQ_ADD(lo, e));
     *y = y0;
     return y0 == y1;
@@ -261,7 +260,7 @@ FQ_HD int fq_quick_round(double hi, double lo, double* y)
  * Quick phase of log for 0 < x < infinity, x normal, of at most 33 significant bits (the yield distances'
  * 1 - u32 2^-32): x = 2^E m, z = m c - 1 exactly (c of 20 bits from the table, |z| < 2^-7),
  * log x = E ln 2 - log c + z - z^2/2 + z^3 (1/3 - z/4 + ... - z^7/10).  About 35 operations without a division,
- * against 200 and one of the full evaluation.  (Over all 2^32 arguments of a yield distance 0.07% need the full
+ * against 200 and one of the full evaluation.  (Of all 2^32 arguments of a yield distance 0.02% need the full
  * evaluation.)  Construction of 16384 x 1000 yield positions and a drive over 2250 more: 42.3 ms without the
  * quick phase, 14.0 ms with it.
  */
@@ -297,7 +296,8 @@ FQ_HD int fq_log_quick(double x, double* y)
     double lo = FQ_ADD(FQ_ADD(s1.lo, s2.lo), FQ_ADD(s3.lo, FQ_FMA(-0.5, z2l, t[2])));
     lo = FQ_FMA(E, FQ_LOG_LN2_LO, lo);
     lo = FQ_FMA(FQ_MUL(z, z2), p, lo);
-    return fq_quick_round(s3.hi, lo, y);
+    /* largest error: the cube's term beside a logarithm of about z, in the two rows with c = 1 (2^-67) */
+    return fq_quick_round(s3.hi, lo, 0x1p-66, y);
 }
 
 FQ_HD_OUT double fq_log_full(double x)
@@ -441,11 +441,11 @@ FQ_HD double fq_pow(double x, double y)
 }
 
 /*
- * Quick phase of sin for 2^-30 <= |x - n pi| and |x| <= 12.5: r = x - n pi in [-pi/2, pi/2] as a double-double (x minus
+ * Quick phase of sin for 2^-20 <= |x - n pi| and |x| <= 12.5: r = x - n pi in [-pi/2, pi/2] as a double-double (x minus
  * n times pi's leading double is exact there), sin r = r (1 + r^2 (c1 + r^2 (c2 + ...))) with c1 .. c4 and their
  * sums in double-double.  One series for all quadrants (a warp holds all of them), about 75 operations
  * against 330.  Adjoint of 200 steps at N = 65536 (forward with recording and backward): 43.6 ms without the
- * quick phase, 21.1 ms with it.
+ * quick phase, 18 ms with it.
  */
 FQ_HD int fq_sin_quick(double x, double* y)
 {
@@ -455,7 +455,7 @@ FQ_HD int fq_sin_quick(double x, double* y)
     const double nf = FQ_SUB(FQ_ADD(FQ_MUL(x, 0x1.45f306dc9c883p-2), 0x1.8p52), 0x1.8p52);
     const double t = FQ_FMA(-nf, 0x1.921fb54442d18p+1, x);
     const double a = t < 0.0 ? -t : t;
-    if (a < 0x1p-30) {
+    if (a < 0x1p-20) {
         return 0;
     }
     const double w = FQ_MUL(nf, 0x1.1a62633145c07p-53);
@@ -486,7 +486,12 @@ FQ_HD int fq_sin_quick(double x, double* y)
 #undef FQ_SIN_STEP
     const double hi = FQ_MUL(rh, c.hi);
     const double lo = FQ_FMA(rl, c.hi, FQ_FMA(rh, c.lo, FQ_FMA(rh, c.hi, -hi)));
-    if (!fq_quick_round(hi, lo, y)) {
+    /* errors: the roundings of the terms from c5 on, 2^-69.2 at r = pi/2 and falling as r^10; the full
+     * evaluation's truncated series, 2^-72.3 at r = pi/4; the others (pi as a double-double at 2^-20 from its
+     * multiple) stay below 2^-80.  A full evaluation holds up its warp for 10 us, and with it a whole step of
+     * a small system, so the bound follows r: it is needed once in 10^5. */
+    const double q2 = FQ_MUL(q, q), q5 = FQ_MUL(FQ_MUL(q2, q2), q);
+    if (!fq_quick_round(hi, lo, FQ_FMA(q5, 0x1p-74, 0x1p-71), y)) {
         return 0;
     }
     if ((int)nf & 1) {
