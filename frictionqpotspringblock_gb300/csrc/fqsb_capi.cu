@@ -965,9 +965,9 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
         const char* ns = getenv("FQSB_NO_SMALL");
         const char* nc = getenv("FQSB_SMALL_CTAS");
         int max_ctas = nc ? atoi(nc) : SMALL_MAX_CTAS;
-        h->sg = small_geometry(N, max_ctas);
+        h->sg = small_geometry(N, d.pot, max_ctas);
         if (h->sg.ok && h->sg.ctas > 8 && !small_cluster_fits(d, h->sg)) {
-            h->sg = small_geometry(N, 8); /* the GPU cannot co-schedule a cluster of 16 */
+            h->sg = small_geometry(N, d.pot, 8); /* the GPU cannot co-schedule a cluster of 16 */
         }
         h->small_ok = h->sg.ok && !inter_grid(cfg->interactions) && cfg->interactions != FQSB_LONGRANGE1D &&
                       !(ns && ns[0] == '1');

@@ -63,11 +63,10 @@ static const int64_t NX_MAX_VALUES = (int64_t)1 << 25;
 static const int SMALL_THREADS_MAX = 256; /* particle threads per CTA (each CTA adds one control warp) */
 struct SmallGeom {
     int threads; /* per CTA, power of two in [32, 256] */
-    int ppt;     /* particles per thread: 1, 2 or 4 */
     int ctas;    /* CTAs of the cluster */
-    bool ok;     /* N fits: N <= max_ctas * 1024 */
+    bool ok;     /* N fits and gains from it */
 };
-SmallGeom small_geometry(int64_t N, int max_ctas);
+SmallGeom small_geometry(int64_t N, int pot, int max_ctas);
 cudaError_t launch_small_run(const DevSys& s, const SmallGeom& g, cudaStream_t st);
 /* refreshes the next-window buffers of a small system (no-op when it has none) */
 cudaError_t launch_next_window(const DevSys& s, cudaStream_t st);

@@ -90,44 +90,6 @@ __device__ __forceinline__ int barrier_after(RunSync* y, unsigned long long base
     return last ? END_LAST : END_NOT;
 }
 
-/* Pairwise sums of x and of y over the 32 lanes (fixed order; both sums share instructions as in
- * cta_tree2): lane 0 gets both. */
-__device__ __forceinline__ double2 warp_tree2(double x, double y)
-{
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    double v;
-    {
-        const double xa = __shfl_sync(full, x, (2 * lane) & 31), xb = __shfl_sync(full, x, (2 * lane + 1) & 31);
-        const double ya = __shfl_sync(full, y, (2 * lane) & 31), yb = __shfl_sync(full, y, (2 * lane + 1) & 31);
-        v = add_nospec(lane < 16 ? xa : ya, lane < 16 ? xb : yb);
-    }
-#pragma unroll
-    for (int h = 16; h >= 2; h >>= 1) {
-        const double a = __shfl_sync(full, v, (2 * lane) & 31), b = __shfl_sync(full, v, (2 * lane + 1) & 31);
-        if (lane < h) {
-            v = add_nospec(a, b);
-        }
-    }
-    return make_double2(v, __shfl_sync(full, v, 1));
-}
-
-/* Pairwise sum of n = 1, 2, 4 or 8 consecutive values */
-__device__ __forceinline__ double sum_consecutive(const double* x, int n)
-{
-    double r = x[0];
-    if (n >= 2) {
-        r = add_nospec(r, x[1]);
-    }
-    if (n >= 4) {
-        r = add_nospec(r, add_nospec(x[2], x[3]));
-    }
-    if (n >= 8) {
-        r = add_nospec(r, add_nospec(add_nospec(x[4], x[5]), add_nospec(x[6], x[7])));
-    }
-    return r;
-}
-
 /*
  * Particle p at its new position un, which may have left its well: searches its window, counts the change
  * in the slot of step t (act) and commits the new well; d becomes centre - un (Cuspy).  Returns whether
@@ -417,7 +379,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
             if (vy->nan[q]) {
                 sc.nan_flag = 1;
             }
-            finalize_ctl(&sc, shared_ring ? ring : s.ring, ufk, tot.x, tot.y);
+            finalize_ctl(&sc, shared_ring ? ring : s.ring, ufk, tot.x, residual_of(flags, tot.x, tot.y), globaltimer());
         }
     };
 

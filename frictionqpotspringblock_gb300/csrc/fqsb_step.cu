@@ -43,8 +43,6 @@
  */
 #include "fqsb_stepcore.cuh"
 
-#include <cooperative_groups.h>
-
 namespace fqsb {
 
 /*
@@ -1082,643 +1080,6 @@ cudaError_t launch_nopass_iteration(const DevSys& s, const LineGeom& g, const No
     k_nopass_update<<<(unsigned)g.grid, (unsigned)g.threads, 0, st>>>(s, A);
     k_nopass_force<<<(unsigned)g.grid, (unsigned)g.threads, 0, st>>>(s, A);
     return cudaGetLastError();
-}
-
-/* ------------------------------------------------------------- small systems: one cluster */
-
-/*
- * A whole run of a small Line1d / Particles system in one launch of one thread-block cluster (up to
- * 16 CTAs on 16 SMs).  For small N the graph path is bound by its per-step launch and node overhead
- * (about 18 us per time step at N = 1024, no faster than one CPU core); here the state stays in
- * registers for the whole run, the new positions at tile edges cross CTA boundaries through
- * distributed shared memory, and one cluster barrier per time step replaces the per-step launches.
- *
- * Every CTA has its particle threads and one control warp (the last warp).  Time step t:
- *   position update -> cluster barrier A_t -> wells, forces, velocities, the CTA's residual subtree
- *   and counters, published to CTA 0's slot t % 2 -> position update of step t + 1 -> A_{t+1} ...
- * Meanwhile, after A_{t+1}, CTA 0's control warp sums step t's subtrees, applies its counters and
- * runs the same stop tests as the graph path (finalize_ctl); its decision is read by every thread
- * after A_{t+2}.  The decision thus comes two barriers late: when it says stop after step t, the
- * threads have already taken step t + 1, and they restore the state from before that step (positions,
- * velocities, accelerations, and the well and chunk window as they were) -- the step's counters were
- * never applied.  The stop tests therefore leave the critical path, and one barrier per step remains.
- * Arithmetic, the residual tree (aligned power-of-two tiles) and the stop tests are those of
- * k_step_line, and chunk windows move as k_regen moves them, so the results equal the graph path's
- * bit for bit.  Runs that record a trajectory (adjoint) use the graph path.
- */
-
-/* Named barrier 1 over the particle threads of the CTA (the control warp is not in it). */
-__device__ __forceinline__ void particle_bar(int n)
-{
-    asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
-}
-
-/* particle_bar that also returns whether any particle thread passed a non-zero flag */
-__device__ __forceinline__ int particle_bar_or(int n, int flag)
-{
-    int r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\t"
-                 "selp.s32 %0, 1, 0, q;\n\t}"
-                 : "=r"(r)
-                 : "r"(flag), "r"(n)
-                 : "memory");
-    return r;
-}
-
-/* cta_tree2 over the first nt threads of the CTA (nt a multiple of 32), with the named barrier */
-__device__ __forceinline__ double2 particle_tree2(double x, double y, double* sh, int nt)
-{
-#pragma unroll
-    for (int m = 1; m < 32; m <<= 1) {
-        double xo = __shfl_down_sync(0xffffffffu, x, m);
-        double yo = __shfl_down_sync(0xffffffffu, y, m);
-        if ((threadIdx.x & (2 * m - 1)) == 0) {
-            x = add_nospec(x, xo);
-            y = add_nospec(y, yo);
-        }
-    }
-    int nw = nt >> 5;
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    particle_bar(nt);
-    if (lane == 0) {
-        sh[wid] = x;
-        sh[32 + wid] = y;
-    }
-    particle_bar(nt);
-    if (wid == 0) {
-        double a = lane < nw ? sh[lane] : 0.0;
-        double b = lane < nw ? sh[32 + lane] : 0.0;
-#pragma unroll
-        for (int m = 1; m < 32; m <<= 1) {
-            double ao = __shfl_down_sync(0xffffffffu, a, m);
-            double bo = __shfl_down_sync(0xffffffffu, b, m);
-            if ((threadIdx.x & (2 * m - 1)) == 0) {
-                a = add_nospec(a, ao);
-                b = add_nospec(b, bo);
-            }
-        }
-        x = a;
-        y = b;
-    }
-    return make_double2(x, y);
-}
-
-template <int POT, int INTER, int PPT, bool TH>
-__global__ void __launch_bounds__(SMALL_THREADS_MAX + 32, 1) k_run_small(const __grid_constant__ DevSys s)
-{
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    __shared__ double sh_un[2][SMALL_THREADS_MAX * PPT];
-    __shared__ double red[64];
-    /* CTA 0 keeps the run-control block and the StopList window, and per step parity the CTAs'
-     * residual subtrees and counters, and the stop decision */
-    __shared__ Ctl sc;
-    __shared__ double sring[SMALL_RING_MAX];
-    __shared__ double2 spart[2][SMALL_MAX_CTAS];
-    __shared__ unsigned long long sl_ds[2], sl_da[2];
-    __shared__ int sl_nan[2], sl_walk[2], sl_stop[2];
-    /* this CTA's counters of the current step */
-    __shared__ int sh_nan, sh_walk;
-    __shared__ unsigned long long sh_ds, sh_da;
-    /* window moves of this step shared by the CTA's particle threads (fwd_move_*) */
-    constexpr int SMALL_MOVES = 64;
-    __shared__ FwdMove sh_moves[SMALL_MOVES];
-    __shared__ int sh_nmove;
-
-    if (TH && (s.ctl->done || s.ctl->error)) {
-        /* launched beside others that ended the run (no CTA writes the control block before all have read it) */
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            s.ctl->th_commit = 0;
-        }
-        return;
-    }
-    const unsigned rank = cluster.block_rank();
-    const unsigned G = cluster.num_blocks();
-    const int tid = threadIdx.x;
-    const int pt = (int)blockDim.x - 32; /* particle threads; the last warp is the control warp */
-    const bool ctrl = tid >= pt;
-    const int64_t N = s.N;
-    const int64_t tile = (int64_t)pt * PPT;
-    const int64_t base = (int64_t)rank * tile;
-    const int64_t p0 = base + (int64_t)tid * PPT;
-    const Ctl* gc = s.ctl;
-    const int flags = gc->flags;
-    const bool act = (flags & (RF_ACT | RF_TRUNCATE | RF_EVENT)) != 0;
-    const bool resid = (flags & RF_RESID) != 0;
-    const double vdt = gc->vdt;
-    double uf = gc->u_frame;
-    int cur = gc->cur;
-    const int64_t nring = (resid && gc->niter_tol > 0) ? gc->niter_tol : 0;
-    if (rank == 0) {
-        if (tid == 0) {
-            sc = *gc;
-        }
-        for (int64_t i = tid; i < nring; i += blockDim.x) {
-            sring[i] = s.ring[i];
-        }
-        if (tid < 2) {
-            sl_ds[tid] = 0ull;
-            sl_da[tid] = 0ull;
-            sl_nan[tid] = 0;
-            sl_walk[tid] = 0;
-            sl_stop[tid] = 0;
-        }
-    }
-
-    /* ring neighbours of the tile's first and last particle: (CTA rank, index in its tile) */
-    const int64_t plast = (base + tile < N ? base + tile : N) - 1;
-    const int64_t pl = base == 0 ? N - 1 : base - 1;
-    const int64_t pr = plast + 1 == N ? 0 : plast + 1;
-    const int il = (int)(pl % tile), ir = (int)(pr % tile);
-    const double* left[2] = {cluster.map_shared_rank(&sh_un[0][0], (unsigned)(pl / tile)),
-                             cluster.map_shared_rank(&sh_un[1][0], (unsigned)(pl / tile))};
-    const double* right[2] = {cluster.map_shared_rank(&sh_un[0][0], (unsigned)(pr / tile)),
-                              cluster.map_shared_rank(&sh_un[1][0], (unsigned)(pr / tile))};
-    Ctl* sc0 = cluster.map_shared_rank(&sc, 0);
-    double2* spart0 = cluster.map_shared_rank(&spart[0][0], 0);
-    unsigned long long* sl_ds0 = cluster.map_shared_rank(&sl_ds[0], 0);
-    unsigned long long* sl_da0 = cluster.map_shared_rank(&sl_da[0], 0);
-    int* sl_nan0 = cluster.map_shared_rank(&sl_nan[0], 0);
-    int* sl_walk0 = cluster.map_shared_rank(&sl_walk[0], 0);
-    const int* sl_stop0 = cluster.map_shared_rank(&sl_stop[0], 0);
-
-    double u[PPT], v[PPT], a[PPT];
-    double4_32a w[PPT];
-    /* the state before the latest step, kept for the rollback of a step taken after the stop */
-    double pu[PPT], pv[PPT], pa[PPT];
-    int64_t pstart[PPT];
-#pragma unroll
-    for (int j = 0; j < PPT; ++j) {
-        int64_t p = p0 + j;
-        if (!ctrl && p < N) {
-            u[j] = s.u[cur][p];
-            v[j] = s.v[cur][p];
-            a[j] = s.a[cur][p];
-            w[j] = load_well(s, p);
-        }
-        else {
-            u[j] = v[j] = a[j] = 0.0;
-            w[j] = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-        }
-        pu[j] = u[j];
-        pv[j] = v[j];
-        pa[j] = a[j];
-        pstart[j] = 0;
-    }
-    /* thermal forces: the values in use, and what step t + 1 draws, loaded a step ahead (planned draws) */
-    double fth[PPT], fnew[PPT];
-    uint32_t draw = 0u, draw_next = 0u;
-    const uint32_t* th_mask = TH ? s.th_mask + (p0 < N ? p0 >> 5 : 0) : nullptr;
-    if (TH && !ctrl) {
-        draw = p0 < N ? th_mask[0] : 0u;
-        draw_next = p0 < N ? th_mask[s.th_words] : 0u;
-#pragma unroll
-        for (int j = 0; j < PPT; ++j) {
-            const int64_t p = p0 + j;
-            fth[j] = p < N ? s.f_th[p] : 0.0;
-            fnew[j] = p < N && (draw >> (p & 31) & 1u) ? s.th_val[p] : 0.0;
-        }
-    }
-    /* one particle per thread: latency bound, all fp64 on the fp64 pipe; more: throughput bound, split */
-    constexpr unsigned SOFT = PPT >= 2 ? STEP_SOFT : 0u;
-    /* pcg32 stride of pt steps, x -> mv_a x + mv_c, for the shared draws of window moves */
-    const uint64_t mv_c = pcg_advance(0ULL, (uint64_t)pt);
-    const uint64_t mv_a = pcg_advance(1ULL, (uint64_t)pt) - mv_c;
-    int buf = 0;
-    int64_t steps_taken = 0;
-    double uf_prev = uf;
-    for (int64_t t = 0;; ++t) {
-        const double uf_t = (flags & RF_FLOW) ? FQ_ADD(uf, vdt) : uf;
-        double un[PPT];
-        if (!ctrl) {
-#pragma unroll
-            for (int j = 0; j < PPT; ++j) {
-                un[j] = S_ADD(3, S_ADD(2, u[j], S_MULC(0, s.f_dt, s.dt, v[j])), S_MULC(1, s.f_hdt2, s.hdt2, a[j]));
-                sh_un[buf][tid * PPT + j] = un[j];
-            }
-        }
-        if (tid == 0) {
-            sh_ds = 0ull;
-            sh_da = 0ull;
-            sh_nan = 0;
-            sh_walk = 0;
-            sh_nmove = 0;
-        }
-        /* A_t: every tile's new positions, the subtrees and counters of step t - 1, and the decision
-         * after step t - 2 (slot t % 2) */
-        cluster.sync();
-        if (t >= 2 && sl_stop0[t & 1]) {
-            /* stopped after step t - 2: restore the state before step t - 1 */
-            steps_taken = t - 1;
-            if (!ctrl) {
-#pragma unroll
-                for (int j = 0; j < PPT; ++j) {
-                    int64_t p = p0 + j;
-                    u[j] = pu[j];
-                    v[j] = pv[j];
-                    a[j] = pa[j];
-                    if (p >= N) {
-                        continue;
-                    }
-                    bool placed = false;
-                    if (s.start[p] != pstart[j]) {
-                        /* the window moved in the step taken after the stop: put it back */
-                        double acc;
-                        seq_fill(s, p, pstart[j], s.W, s.data + p * s.W, &acc);
-                        s.start[p] = pstart[j];
-                        s.acc_end[p] = acc;
-                        placed = true;
-                    }
-                    /* the well of the restored position (index, cached well) in the restored window */
-                    double4_32a ww = load_well(s, p);
-                    if (placed) {
-                        /* not a well of the restored window: the search starts from its index alone */
-                        ww.x = ww.y = __longlong_as_double(0x7ff8000000000000LL);
-                    }
-                    if ((placed || !in_well(ww.x, ww.y, u[j])) && !non_finite(u[j]) &&
-                        !window_search(s, p, u[j], ww)) {
-                        dev_align(s, p, u[j]);
-                    }
-                }
-            }
-            break;
-        }
-        const double uf_last = uf_prev; /* u_frame of step t - 1, for its stop tests */
-        uf_prev = uf_t;
-        uf = uf_t;
-        if (ctrl) {
-            if (rank == 0 && t >= 1) {
-                /* the decision after step t - 1 */
-                const int q = (int)((t - 1) & 1);
-                const int lane = tid - pt;
-                double tx = 0.0, ty = 0.0;
-                if (resid) {
-                    /* the canonical tree over the CTA subtrees, zero padded (as tree_partials): G <= 32 */
-                    double x = 0.0, y = 0.0;
-                    if ((unsigned)lane < G) {
-                        x = spart[q][lane].x;
-                        y = spart[q][lane].y;
-                    }
-                    tx = warp_tree(x);
-                    ty = warp_tree(y);
-                }
-                if (lane == 0) {
-                    sc.s_sum = (long long)((unsigned long long)sc.s_sum + sl_ds[q]);
-                    sc.a_count = (long long)((unsigned long long)sc.a_count + sl_da[q]);
-                    if (sl_nan[q]) {
-                        sc.nan_flag = 1;
-                    }
-                    if (sl_walk[q]) {
-                        sc.walk_flag = 1;
-                    }
-                    sl_ds[q] = 0ull;
-                    sl_da[q] = 0ull;
-                    sl_nan[q] = 0;
-                    sl_walk[q] = 0;
-                    finalize_ctl(&sc, sring, uf_last, tx, ty);
-                    sl_stop[q] = (sc.done || sc.error || (globaltimer() - sc.launch_t0) >= sc.budget_ns ||
-                                  (TH && t >= s.th_K))
-                                     ? 1
-                                     : 0;
-                }
-            }
-            buf ^= 1;
-            continue;
-        }
-        /* the particle threads take step t */
-#pragma unroll
-        for (int j = 0; j < PPT; ++j) {
-            pu[j] = u[j];
-            pv[j] = v[j];
-            pa[j] = a[j];
-            if (p0 + j < N) {
-                pstart[j] = s.start[p0 + j];
-            }
-        }
-        double rf = 0.0, rff = 0.0;
-        bool nan = false;
-        /* plastic activity of a particle whose well index went from gold to gnew */
-        auto count_move = [&](int64_t p, int64_t gold, int64_t gnew) {
-            if (act && gnew != gold) {
-                int64_t ref = s.i_n[p];
-                long long ds = absll(gnew - ref) - absll(gold - ref);
-                long long da = (long long)(gnew != ref) - (long long)(gold != ref);
-                atomicAdd(&sh_ds, (unsigned long long)ds);
-                atomicAdd(&sh_da, (unsigned long long)da);
-            }
-        };
-        /* wells: a search inside the chunk window, or a window move */
-        int64_t gold[PPT];
-        bool mv[PPT];
-        bool any_mv = false;
-        double d[PPT]; /* Cuspy: centre - u (well_of) */
-#pragma unroll
-        for (int j = 0; j < PPT; ++j) {
-            int64_t p = p0 + j;
-            mv[j] = false;
-            d[j] = 0.0;
-            if (p >= N) {
-                continue;
-            }
-            double up = un[j];
-            /* with one particle per thread the wait for d would be on the critical path (65 cycles of a
-             * step's ~6300): there the keys of un, which are ready, decide */
-            if (POT == POT_CUSPY && SOFT != 0u) {
-                d[j] = S_SUB(5, w[j].z, up);
-                if (surely_in_well(make_double2(w[j].z, w[j].w), d[j])) {
-                    continue;
-                }
-            }
-            nan |= is_nan_bits(up);
-            double4_32a ww = w[j];
-            if (!in_well(ww.x, ww.y, up) && !non_finite(up)) {
-                gold[j] = s.gidx[p];
-                if (window_search(s, p, up, ww)) {
-                    count_move(p, gold[j], s.gidx[p]);
-                    w[j] = ww;
-                    d[j] = FQ_SUB(ww.z, up);
-                }
-                else {
-                    mv[j] = true;
-                    any_mv = true;
-                }
-            }
-        }
-        if (particle_bar_or(pt, any_mv ? 1 : 0)) {
-            /* moves planned here are drawn by all particle threads of the CTA, then summed by their
-             * owners; the others (more than SMALL_MOVES, or not a forward move) go through dev_align */
-            int slot[PPT];
-#pragma unroll
-            for (int j = 0; j < PPT; ++j) {
-                slot[j] = -1;
-                if (mv[j]) {
-                    int k = atomicAdd(&sh_nmove, 1);
-                    if (k < SMALL_MOVES) {
-                        FwdMove m;
-                        const bool ready = next_window_ready(s, p0 + j);
-                        if (fwd_move_plan(s, p0 + j, un[j], m)) {
-                            m.next = ready ? 1 : 0;
-                            sh_moves[k] = m;
-                            slot[j] = k;
-                        }
-                        else {
-                            sh_moves[k].p = -1;
-                        }
-                    }
-                }
-            }
-            if (tid == 0) {
-                /* the moved windows' next-window buffers are out of date after this run */
-                atomicOr(&sc0->nx_stale, 1);
-            }
-            particle_bar(pt);
-            const int nm = sh_nmove < SMALL_MOVES ? sh_nmove : SMALL_MOVES;
-            for (int k = 0; k < nm; ++k) {
-                if (sh_moves[k].p >= 0) {
-                    if (sh_moves[k].next) {
-                        fwd_move_copy(s, sh_moves[k], tid, pt);
-                    }
-                    else {
-                        fwd_move_draws(s, sh_moves[k], tid, pt, mv_a, mv_c);
-                    }
-                }
-            }
-            particle_bar(pt);
-#pragma unroll
-            for (int j = 0; j < PPT; ++j) {
-                if (!mv[j]) {
-                    continue;
-                }
-                int64_t p = p0 + j;
-                if (slot[j] >= 0) {
-                    if (sh_moves[slot[j]].next) {
-                        fwd_move_finish(s, sh_moves[slot[j]]);
-                    }
-                    else {
-                        fwd_move_sum(s, sh_moves[slot[j]]);
-                    }
-                }
-                else {
-                    dev_align(s, p, un[j]); /* moves the chunk window; a failed search sets walk_flag */
-                    if (((volatile Ctl*)s.ctl)->walk_flag) {
-                        sh_walk = 1;
-                    }
-                }
-                w[j] = load_well(s, p);
-                d[j] = FQ_SUB(w[j].z, un[j]);
-                count_move(p, gold[j], s.gidx[p]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < PPT; ++j) {
-            int64_t p = p0 + j;
-            if (p >= N) {
-                continue;
-            }
-            double up = un[j];
-            const double4_32a ww = w[j];
-            double ff;
-            if (SOFT == 0u) {
-                d[j] = FQ_SUB(ww.z, up);
-            }
-            double sfi = frame_pot<POT, SOFT>(s, ww, d[j], up, uf, ff);
-            if (inter_ring(INTER)) {
-                int li = tid * PPT + j;
-                double uL = li > 0 ? sh_un[buf][li - 1] : left[buf][il];
-                double uR = (li + 1 < tile && p + 1 < N) ? sh_un[buf][li + 1] : right[buf][ir];
-                sfi = add_ring_force<INTER, SOFT>(s, sfi, uL, up, uR);
-            }
-            else {
-                sfi = add_zero(sfi);
-            }
-            double vn, an, f;
-            if (TH) {
-                /* step t's draw, then the loads for step t + 1 (row th_K of the plan is empty) */
-                if (draw >> (p & 31) & 1u) {
-                    fth[j] = fnew[j];
-                }
-                if (draw_next >> (p & 31) & 1u) {
-                    fnew[j] = s.th_val[(t + 1) * N + p];
-                }
-            }
-            verlet_velocity<SOFT, TH>(s, sfi, v[j], a[j], vn, an, f, TH ? fth[j] : 0.0);
-            u[j] = up;
-            v[j] = vn;
-            a[j] = an;
-            if (resid) {
-                double f2 = mul_nospec(f, f), ff2 = mul_nospec(ff, ff);
-                if (j == 0) {
-                    rf = f2;
-                    rff = ff2;
-                }
-                else {
-                    rf = add_nospec(rf, f2);
-                    rff = add_nospec(rff, ff2);
-                }
-            }
-        }
-        if (TH) {
-            draw = draw_next;
-            draw_next = p0 < N ? th_mask[(t + 2 < s.th_K ? t + 2 : s.th_K) * s.th_words] : 0u;
-        }
-        if (nan) {
-            sh_nan = 1;
-        }
-        double2 sfs = make_double2(0.0, 0.0);
-        if (resid) {
-            sfs = particle_tree2(rf, rff, red, pt);
-        }
-        particle_bar(pt);
-        if (tid == 0) {
-            /* publish step t to CTA 0's slot t % 2 */
-            const int q = (int)(t & 1);
-            if (resid) {
-                spart0[q * SMALL_MAX_CTAS + rank] = sfs;
-            }
-            if (sh_ds) {
-                atomicAdd(sl_ds0 + q, sh_ds);
-            }
-            if (sh_da) {
-                atomicAdd(sl_da0 + q, sh_da);
-            }
-            if (sh_nan) {
-                atomicOr(sl_nan0 + q, 1);
-            }
-            if (sh_walk) {
-                atomicOr(sl_walk0 + q, 1);
-            }
-        }
-        buf ^= 1;
-    }
-    cur = sc0->cur;
-    if (!ctrl) {
-#pragma unroll
-        for (int j = 0; j < PPT; ++j) {
-            int64_t p = p0 + j;
-            if (p < N) {
-                s.u[cur][p] = u[j];
-                s.v[cur][p] = v[j];
-                s.a[cur][p] = a[j];
-            }
-        }
-    }
-    if (rank == 0) {
-        for (int64_t i = tid; i < nring; i += blockDim.x) {
-            s.ring[i] = sring[i];
-        }
-        if (tid == 0) {
-            if (TH) {
-                sc.th_commit = steps_taken;
-            }
-            *s.ctl = sc;
-        }
-    }
-    /* no CTA may exit while others still read its shared memory */
-    cluster.sync();
-}
-
-SmallGeom small_geometry(int64_t N, int max_ctas)
-{
-    SmallGeom g;
-    int64_t per = (N + max_ctas - 1) / max_ctas;
-    int64_t tile = 32;
-    while (tile < per) {
-        tile <<= 1;
-    }
-    g.threads = (int)(tile < 256 ? tile : 256);
-    g.ppt = (int)(tile / g.threads);
-    g.ctas = (int)((N + tile - 1) / tile);
-    g.ok = N >= 1 && tile <= 1024 && max_ctas <= SMALL_MAX_CTAS;
-    return g;
-}
-
-template <int POT, int INTER, bool TH = false>
-static const void* small_kernel_t(int ppt)
-{
-    switch (ppt) {
-        case 1: return (const void*)k_run_small<POT, INTER, 1, TH>;
-        case 2: return (const void*)k_run_small<POT, INTER, 2, TH>;
-        default: return (const void*)k_run_small<POT, INTER, 4, TH>;
-    }
-}
-
-static const void* small_kernel(const DevSys& s, const SmallGeom& g)
-{
-    if (s.f_th) {
-        /* RandomNormalForcing systems: Cuspy with Laplace1d, Quartic1d or no interactions */
-        switch (s.inter) {
-            case INTER_LAPLACE1D: return small_kernel_t<POT_CUSPY, INTER_LAPLACE1D, true>(g.ppt);
-            case INTER_QUARTIC1D: return small_kernel_t<POT_CUSPY, INTER_QUARTIC1D, true>(g.ppt);
-            default: return small_kernel_t<POT_CUSPY, INTER_NONE, true>(g.ppt);
-        }
-    }
-    /* the Quartic interactions exist with the Cuspy potential only (Line1d.h:428, :562) */
-    if (s.inter == INTER_QUARTIC1D) {
-        return small_kernel_t<POT_CUSPY, INTER_QUARTIC1D>(g.ppt);
-    }
-    if (s.inter == INTER_QUARTICGRAD1D) {
-        return small_kernel_t<POT_CUSPY, INTER_QUARTICGRAD1D>(g.ppt);
-    }
-    if (s.inter == INTER_LAPLACE1D) {
-        return s.pot == POT_CUSPY ? small_kernel_t<POT_CUSPY, INTER_LAPLACE1D>(g.ppt)
-               : s.pot == POT_SEMISMOOTH ? small_kernel_t<POT_SEMISMOOTH, INTER_LAPLACE1D>(g.ppt)
-                                         : small_kernel_t<POT_SMOOTH, INTER_LAPLACE1D>(g.ppt);
-    }
-    return s.pot == POT_CUSPY ? small_kernel_t<POT_CUSPY, INTER_NONE>(g.ppt)
-           : s.pot == POT_SEMISMOOTH ? small_kernel_t<POT_SEMISMOOTH, INTER_NONE>(g.ppt)
-                                     : small_kernel_t<POT_SMOOTH, INTER_NONE>(g.ppt);
-}
-
-static void small_launch_config(const SmallGeom& g, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr)
-{
-    cfg = {};
-    cfg.gridDim = dim3((unsigned)g.ctas);
-    cfg.blockDim = dim3((unsigned)g.threads + 32u); /* particle threads and the control warp */
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)g.ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-}
-
-bool small_cluster_fits(const DevSys& s, const SmallGeom& g)
-{
-    const void* f = small_kernel(s, g);
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    small_launch_config(g, nullptr, cfg, attr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return n >= 1;
-}
-
-cudaError_t launch_small_run(const DevSys& s, const SmallGeom& g, cudaStream_t st)
-{
-    const void* f = small_kernel(s, g);
-    if (g.ctas > 8) {
-        /* clusters above the portable size of 8 must be allowed per kernel */
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) {
-            return e;
-        }
-    }
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    small_launch_config(g, st, cfg, attr);
-    DevSys arg = s;
-    arg.in_graph = 0; /* not inside the run graph: no conditional handles to set */
-    void* args[] = {(void*)&arg};
-    return cudaLaunchKernelExC(&cfg, f, args);
 }
 
 /* ------------------------------------------------------------- geometry */

@@ -69,14 +69,25 @@ __device__ __forceinline__ void set_branch(const DevSys& s, unsigned v)
     }
 }
 
+/* The residual of a step (residual, detail.h:1512-1520) from its sums of f^2 and f_frame^2, if the run asks for it */
+__device__ __forceinline__ double residual_of(int flags, double sf, double sff)
+{
+    if (!(flags & RF_RESID)) {
+        return 0.0;
+    }
+    const double r_fres = FQ_SQRT(sf), r_fext = FQ_SQRT(sff);
+    return r_fext != 0.0 ? FQ_DIV(r_fres, r_fext) : r_fres;
+}
+
 /*
  * Bookkeeping and stop tests of one finished step on a run-control block c (global memory for the
  * graph path, shared memory for the one-cluster path) and its StopList window `ring`: step and
  * increment counters, frame position, plastic activity, NaN / yield-search errors, the StopList
  * residual test (GooseFEM::Iterate::StopList, detail.h:1780-1783), event, truncation and step limits.
+ * sf: the sum of f_frame (RF_FFSUM); r: the residual; now: the time, for the start of a launch.
  */
 template <typename CTL>
-__device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, double sf, double sff)
+__device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, double sf, double r, uint64_t now)
 {
     int flags = c->flags;
     c->ticket = 0;
@@ -97,7 +108,6 @@ __device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, do
     if (flags & RF_FLOW) {
         c->u_frame = uf;
     }
-    uint64_t now = globaltimer();
     if (c->launch_steps == 0) {
         c->launch_t0 = now;
     }
@@ -124,9 +134,6 @@ __device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, do
             c->done = RUN_EVENT;
         }
         if (!c->done && (flags & RF_RESID)) {
-            double r_fres = FQ_SQRT(sf);
-            double r_fext = FQ_SQRT(sff);
-            double r = r_fext != 0.0 ? FQ_DIV(r_fres, r_fext) : r_fres;
             c->last_residual = r;
             int64_t n = c->niter_tol;
             if (n > 0) {
@@ -139,17 +146,17 @@ __device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, do
                     c->sl_ge_tol2 -= 1;
                 }
                 if (n >= 2) {
-                    double second = ring[(pos + 1) % n];
+                    double second = ring[pos + 1 < n ? pos + 1 : 0];
                     if (second > old) {
                         c->sl_asc -= 1;
                     }
-                    double newest = ring[(pos + n - 1) % n];
+                    double newest = ring[pos > 0 ? pos - 1 : n - 1];
                     if (r > newest) {
                         c->sl_asc += 1;
                     }
                 }
                 ring[pos] = r;
-                c->sl_pos = (pos + 1) % n;
+                c->sl_pos = pos + 1 < n ? pos + 1 : 0;
                 if (r >= c->tol) {
                     c->sl_ge_tol += 1;
                 }
@@ -180,7 +187,7 @@ __device__ __forceinline__ void finalize_ctl(CTL* c, double* ring, double uf, do
 static __device__ __forceinline__ void finalize_step(const DevSys& s, double uf, double sf, double sff)
 {
     Ctl* c = s.ctl;
-    finalize_ctl(c, s.ring, uf, sf, sff);
+    finalize_ctl(c, s.ring, uf, sf, residual_of(c->flags, sf, sff), globaltimer());
     bool more = !c->done && !c->error && (globaltimer() - c->launch_t0) < c->budget_ns;
     __threadfence();
     set_loop(s, more ? 1u : 0u);
@@ -254,6 +261,44 @@ __device__ __forceinline__ bool window_search(const DevSys& s, int64_t p, double
 __device__ __forceinline__ bool non_finite(double x)
 {
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) >= 0x7ff0000000000000LL;
+}
+
+/* Pairwise sums of x and of y over the 32 lanes (fixed order; both sums share instructions as in
+ * cta_tree2): lane 0 gets both. */
+__device__ __forceinline__ double2 warp_tree2(double x, double y)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    double v;
+    {
+        const double xa = __shfl_sync(full, x, (2 * lane) & 31), xb = __shfl_sync(full, x, (2 * lane + 1) & 31);
+        const double ya = __shfl_sync(full, y, (2 * lane) & 31), yb = __shfl_sync(full, y, (2 * lane + 1) & 31);
+        v = add_nospec(lane < 16 ? xa : ya, lane < 16 ? xb : yb);
+    }
+#pragma unroll
+    for (int h = 16; h >= 2; h >>= 1) {
+        const double a = __shfl_sync(full, v, (2 * lane) & 31), b = __shfl_sync(full, v, (2 * lane + 1) & 31);
+        if (lane < h) {
+            v = add_nospec(a, b);
+        }
+    }
+    return make_double2(v, __shfl_sync(full, v, 1));
+}
+
+/* Pairwise sum of n = 1, 2, 4 or 8 consecutive values */
+__device__ __forceinline__ double sum_consecutive(const double* x, int n)
+{
+    double r = x[0];
+    if (n >= 2) {
+        r = add_nospec(r, x[1]);
+    }
+    if (n >= 4) {
+        r = add_nospec(r, add_nospec(x[2], x[3]));
+    }
+    if (n >= 8) {
+        r = add_nospec(r, add_nospec(add_nospec(x[4], x[5]), add_nospec(x[6], x[7])));
+    }
+    return r;
 }
 
 } // namespace fqsb
