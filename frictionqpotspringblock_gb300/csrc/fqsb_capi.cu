@@ -56,6 +56,7 @@ struct fqsb_system {
     int64_t ring_cap;
     cudaGraphExec_t graph;
     cudaGraphExec_t graph_plain; /* the run graph of runs without activity, residual or recording */
+    cudaGraphExec_t graph_one;   /* the run graph of single steps of a grid */
     cudaGraphExec_t graph_resid; /* the run graph of runs with the residual only (minimise) */
     cudaGraphExec_t graph_np; /* the no-passing minimiser's run graph */
     int graph_k;
@@ -535,6 +536,13 @@ static int ensure_graph(fqsb_system* h, int mode = KMODE_GENERAL)
         h->d.in_graph = 0;
         return FQSB_OK;
     }
+    if (mode == KMODE_ONE) {
+        if (!h->graph_one) {
+            DevSys d = h->d;
+            CU(h, build_run_graph(d, h->lg, RunGeom{}, &h->graph_one));
+        }
+        return FQSB_OK;
+    }
     if (mode != KMODE_GENERAL) {
         cudaGraphExec_t* g = mode == KMODE_PLAIN ? &h->graph_plain : &h->graph_resid;
         if (!*g) {
@@ -603,6 +611,10 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
             cudaGraphExecDestroy(h->graph_resid);
             h->graph_resid = nullptr;
         }
+        if (h->graph_one) {
+            cudaGraphExecDestroy(h->graph_one);
+            h->graph_one = nullptr;
+        }
         if (h->graph_np) {
             cudaGraphExecDestroy(h->graph_np);
             h->graph_np = nullptr;
@@ -614,6 +626,9 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     int kmode = KMODE_GENERAL;
     if (np == nullptr && h->rg.ctas && h->use_graph && !h->d.f_th && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
         kmode = (flags & RF_RESID) ? KMODE_RESID : KMODE_PLAIN;
+    }
+    if (np == nullptr && h->rg.ctas && h->use_graph && h->is2d && max_steps == 1) {
+        kmode = KMODE_ONE;
     }
     if (np) {
         if (h->use_graph && !h->graph_np) {
@@ -723,6 +738,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
         else if (h->use_graph) {
             CU(h, cudaGraphLaunch(kmode == KMODE_PLAIN ? h->graph_plain
                                   : kmode == KMODE_RESID ? h->graph_resid
+                                  : kmode == KMODE_ONE   ? h->graph_one
                                                          : h->graph,
                                   h->stream));
         }
@@ -819,6 +835,9 @@ static void free_all(fqsb_system* h)
     if (h->graph_resid) {
         cudaGraphExecDestroy(h->graph_resid);
     }
+    if (h->graph_one) {
+        cudaGraphExecDestroy(h->graph_one);
+    }
     if (h->graph_np) {
         cudaGraphExecDestroy(h->graph_np);
     }
@@ -884,6 +903,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     h->graph = nullptr;
     h->graph_plain = nullptr;
     h->graph_resid = nullptr;
+    h->graph_one = nullptr;
     h->graph_np = nullptr;
     h->graph_k = 0;
     {
@@ -972,7 +992,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
         h->small_ok = h->sg.ok && !inter_grid(cfg->interactions) && cfg->interactions != FQSB_LONGRANGE1D &&
                       !(ns && ns[0] == '1');
     }
-    int64_t nsteps_cta = step_ctas(d, h->lg);
+    int64_t nsteps_cta = std::max(step_ctas(d, h->lg), h->rg.nstrips);
     if (!h->is2d) {
         /* a RandomNormalForcing attached later takes the step kernel's own shape */
         nsteps_cta = std::max(nsteps_cta, line_geometry(N).grid);
@@ -1040,6 +1060,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     h->ring_cap = RING_MIN;
     if (h->is2d) {
         ALLOC(d.sq2, sizeof(double2) * (size_t)N);
+        d.ahead = reinterpret_cast<double*>(d.sq2);
     }
     ALLOC(h->scratch, nd);
     ALLOC(h->red_out, sizeof(double2));
@@ -1615,6 +1636,10 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         cudaGraphExecDestroy(h->graph_resid);
         h->graph_resid = nullptr;
     }
+    if (h->graph_one) {
+        cudaGraphExecDestroy(h->graph_one);
+        h->graph_one = nullptr;
+    }
     h->small_ok = h->small_ok && (h->sg.ctas <= 8 || small_cluster_fits(d, h->sg));
     int rc = updated_inc(h); /* the constructor's refresh */
     return rc ? rc : sync(h);
@@ -2030,6 +2055,10 @@ extern "C" int fqsb_set_parameters(fqsb_system* h, double mu, double k_interacti
     if (h->graph_resid) {
         cudaGraphExecDestroy(h->graph_resid);
         h->graph_resid = nullptr;
+    }
+    if (h->graph_one) {
+        cudaGraphExecDestroy(h->graph_one);
+        h->graph_one = nullptr;
     }
     h->stored = false;
     return sync(h);

@@ -253,6 +253,7 @@ struct DevSys {
     double2* partials;
     int64_t* i_n;
     double2* sq2;
+    double* ahead; /* 2 x N, Laplace2d in the run kernel: every particle's position one step ahead (in sq2's memory) */
     int64_t npartials;
     RunSync* sync;  /* resident run kernel: shared state, and the sums of its nodes (2 x RUN_NODES_MAX) */
     double2* nodes;

@@ -38,13 +38,15 @@ int64_t step_ctas(const DevSys& s, const LineGeom& g);
  * Writes the conditional handles into s (they are kernel arguments of the graph's nodes). */
 /* Run-kernel instantiations: the general one, and two specialised ones -- runs without activity, residual,
  * frame-force sums or recording (timeSteps / flowSteps), and runs with the residual only (minimise) -- with
- * the other code compiled out. */
-enum : int { KMODE_GENERAL = 0, KMODE_PLAIN = 1, KMODE_RESID = 2 };
+ * the other code compiled out.  KMODE_ONE: runs of one step on a grid, by tiles (k_step_grid2): the run kernel's pass
+ * for the first positions is not worth one step (N = 4194304, a call of timeStep: 192 us by tiles, 334 us with the first
+ * step's positions recomputed where they are read). */
+enum : int { KMODE_GENERAL = 0, KMODE_PLAIN = 1, KMODE_RESID = 2, KMODE_ONE = 3 };
 struct RunGeom;
 cudaError_t build_run_graph(DevSys& s, const LineGeom& g, const RunGeom& rg, cudaGraphExec_t* exec,
                             int mode = KMODE_GENERAL);
 
-/* Resident run kernel of Line1d / Particles systems (fqsb_run.cu): many steps in one cooperative launch. */
+/* Resident run kernel of Line1d / Particles / Laplace2d systems (fqsb_run.cu): many steps in one cooperative launch. */
 static const int64_t RUN_NODES_MAX = 1216; /* 8 per SM: the control CTA sums them in one pass */
 struct RunGeom {
     int S;               /* particles per strip: 32 .. 256, a power of two */

@@ -1,5 +1,5 @@
 /*
- * Resident run kernel of Line1d and Particles systems (sm_103a, FP64): many time steps
+ * Resident run kernel of Line1d, Particles and Laplace2d systems (sm_103a, FP64): many time steps
  * (System::timeStep, include/FrictionQPotSpringBlock/detail.h:1539-1570) in one cooperative launch.
  *
  * Why.  With one kernel per time step inside the run graph's WHILE loop every step pays the loop's
@@ -57,28 +57,34 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
-/*
- * Grid barrier after step t, for thread 0 of a CTA (the others wait at a CTA barrier on both sides);
- * returns how the launch goes on.
- */
-__device__ __forceinline__ int barrier_after(RunSync* y, unsigned long long base, int64_t t, bool last)
+/* Grid barrier up to `want` arrivals, for thread 0 of a CTA (the others wait at a CTA barrier on both sides);
+ * false when it ran out. */
+__device__ __forceinline__ bool grid_barrier(RunSync* y, unsigned long long want)
 {
     __threadfence();
     atomicAdd(&y->arrived, 1ull);
-    const unsigned long long want = base + (unsigned long long)(t + 1) * gridDim.x;
     uint64_t t0 = 0;
     for (unsigned k = 1; load_acquire(&y->arrived) < want; ++k) {
         if ((k & 255u) == 0u) {
             if (((volatile RunSync*)y)->failed) {
-                return END_BARRIER;
+                return false;
             }
             const uint64_t now = globaltimer();
             t0 = t0 == 0 ? now : t0;
             if (now - t0 > BARRIER_NS) {
                 atomicOr(&y->failed, 1);
-                return END_BARRIER;
+                return false;
             }
         }
+    }
+    return true;
+}
+
+/* The barrier after step t; returns how the launch goes on. */
+__device__ __forceinline__ int barrier_after(RunSync* y, unsigned long long base, int64_t t, bool last)
+{
+    if (!grid_barrier(y, base + (unsigned long long)(t + 1) * gridDim.x)) {
+        return END_BARRIER;
     }
     const volatile RunSync* vy = y;
     if (vy->stop[t & 1]) {
@@ -157,6 +163,13 @@ struct Strip {
 /*
  * One time step of the strip of particles p0 .. p0 + n - 1 (n <= S) by one warp; returns the strip's sums
  * of f^2 and f_frame^2 (or of f_frame) in lane 0.
+ *
+ * A grid (Laplace2d) is taken in the order of its flat index, so a strip has most of its particles' left and
+ * right neighbours; those above and below are in other strips.  Their positions are read, not recomputed: every step
+ * leaves its particles' next positions in s.ahead (for the first step of a launch a pass of its own does).
+ * That is 8 B more written per particle and step, but no position is updated twice (a tile of 16 x 32 updates 96 of
+ * its neighbours' besides its own 512), and no launches: flow, us per step, by tiles in the run graph and here:
+ * 301 x 257 21.1 and 6.7, 1024 x 1024 51.6 and 40.0, 2048 x 2048 173 and 163, 4096 x 3000 480 and 446.
  */
 template <int POT, int INTER, int MODE, bool TH>
 __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, int64_t p0, int n, int cur, double uf,
@@ -177,7 +190,11 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
 
     /* positions: pass i < G the strip's particles, pass G its two neighbours outside (lanes 0 and 1); the
      * loads of a pass are issued a pass ahead */
-    const int passes = inter_ring(INTER) ? G + 1 : G;
+    constexpr bool GRID = inter_grid(INTER);
+    const int passes = inter_ring(INTER) || GRID ? G + 1 : G;
+    /* grid: positions of this step by the step before, and where this step leaves those of the next */
+    const double* ahead = GRID ? s.ahead + (t & 1 ? 0 : N) : nullptr;
+    double* ahead_next = GRID ? s.ahead + (t & 1 ? N : 0) : nullptr;
     auto index = [&](int i) -> int64_t {
         if (i < G) {
             return p0 + i * 32 + lane;
@@ -188,9 +205,16 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
     double2 wl = __ldcg((POT == POT_CUSPY ? s.wk : s.wy) + p0 + lane);
     {
         const int64_t p = index(0);
-        ul = __ldcg(u0 + p);
-        vl = __ldcg(v0 + p);
-        al = __ldcg(a0 + p);
+        if (GRID) {
+            ul = lane < n ? __ldcg(ahead + p) : 0.0;
+            vl = __ldcg(v0 + p);
+            al = 0.0;
+        }
+        else {
+            ul = __ldcg(u0 + p);
+            vl = __ldcg(v0 + p);
+            al = __ldcg(a0 + p);
+        }
     }
     int leaving = 0;
 #pragma unroll 1
@@ -200,14 +224,20 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
         const int64_t p = index(i);
         if (i + 1 < passes) {
             const int64_t pn = index(i + 1);
-            ul = __ldcg(u0 + pn);
+            if (GRID) {
+                ul = (i + 1 < G ? (i + 1) * 32 + lane < n : lane < 2) ? __ldcg(ahead + pn) : 0.0;
+            }
+            else {
+                ul = __ldcg(u0 + pn);
+                al = __ldcg(a0 + pn);
+            }
             vl = __ldcg(v0 + pn);
-            al = __ldcg(a0 + pn);
             if (i + 1 < G) {
                 wl = __ldcg((POT == POT_CUSPY ? s.wk : s.wy) + pn);
             }
         }
-        const double un = S_ADD(3, S_ADD(2, u, S_MULC(0, s.f_dt, s.dt, v)), S_MULC(1, s.f_hdt2, s.hdt2, a));
+        const double un =
+            GRID ? u : S_ADD(3, S_ADD(2, u, S_MULC(0, s.f_dt, s.dt, v)), S_MULC(1, s.f_hdt2, s.hdt2, a));
         if (i < G) {
             const int k = i * 32 + lane;
             st.v[k] = v;
@@ -250,13 +280,31 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
 
     /* wells, forces and velocities */
     al = __ldcg(a0 + p0 + lane);
+    /* grid: column of the lane's particle, the positions above and below it (loaded a pass ahead) */
+    int64_t col = 0, col_step = 0;
+    double upper = 0.0, lower = 0.0;
+    auto above = [&](int64_t p) { return __ldcg(ahead + (p >= s.cols ? p - s.cols : p + (N - s.cols))); };
+    auto below = [&](int64_t p) { return __ldcg(ahead + (p < N - s.cols ? p + s.cols : p - (N - s.cols))); };
+    if (GRID) {
+        col = (p0 + lane) % s.cols;
+        col_step = 32 % s.cols;
+        if (lane < n) {
+            upper = above(p0 + lane);
+            lower = below(p0 + lane);
+        }
+    }
 #pragma unroll 1
     for (int i = 0; i < G; ++i) {
         const int k = i * 32 + lane;
         const int64_t p = p0 + k;
         const double a = al;
+        const double uU = upper, uD = lower;
         if (i + 1 < G) {
             al = __ldcg(a0 + p + 32);
+            if (GRID && k + 32 < n) {
+                upper = above(p + 32);
+                lower = below(p + 32);
+            }
         }
         const double up = st.un[1 + k], d = POT == POT_CUSPY ? st.d[k] : 0.0;
         double4_32a w = make_double4_32a(0.0, 0.0, 0.0, 0.0);
@@ -268,6 +316,18 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
         double sfi = frame_pot<POT, SOFT>(s, w, d, up, uf, ff);
         if (inter_ring(INTER)) {
             sfi = add_ring_force<INTER, SOFT>(s, sfi, st.un[k], up, st.un[2 + k]);
+        }
+        else if (GRID) {
+            double uL = st.un[k], uR = st.un[2 + k];
+            if (k < n && col == 0) {
+                uL = __ldcg(ahead + p + s.cols - 1);
+            }
+            if (k < n && col == s.cols - 1) {
+                uR = __ldcg(ahead + p - (s.cols - 1));
+            }
+            col += col_step;
+            col -= col >= s.cols ? s.cols : 0;
+            sfi = grid_force<SOFT>(s, sfi, uU, uD, uL, up, uR);
         }
         else {
             sfi = add_zero(sfi);
@@ -285,6 +345,9 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
         if (k < n) {
             v1[p] = vn;
             a1[p] = an;
+            if (GRID) {
+                ahead_next[p] = S_ADD(3, S_ADD(2, up, S_MULC(0, s.f_dt, s.dt, vn)), S_MULC(1, s.f_hdt2, s.hdt2, an));
+            }
         }
         if (resid) {
             st.v[k] = k < n ? fq_smul(f, f) : 0.0;
@@ -331,7 +394,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     RunSync* y = s.sync;
     const int flags = s.ctl->flags;
     const bool tree = (flags & (RF_RESID | RF_FFSUM)) != 0;
-    const unsigned long long base = y->base;
+    unsigned long long base = y->base;
     const int64_t left = steps_of_launch(s), step0 = s.ctl->step;
     const double vdt = s.ctl->vdt;
     const int64_t nring = (flags & RF_RESID) ? s.ctl->niter_tol : 0;
@@ -345,6 +408,12 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     }
     for (int64_t i = tid; shared_ring && i < nring; i += blockDim.x) {
         ring[i] = s.ring[i];
+    }
+    if (inter_grid(s.inter)) {
+        base += gridDim.x; /* the barrier after the first positions (when it runs out, so does the first step's) */
+        if (tid == 0) {
+            grid_barrier(y, base);
+        }
     }
     __syncthreads();
 
@@ -477,7 +546,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     st.list = reinterpret_cast<uint8_t*>(dyn + (size_t)NW * (3 * S + 2)) + (size_t)wid * S;
     st.groups = S / 32;
     RunSync* y = s.sync;
-    const unsigned long long base = y->base;
+    unsigned long long base = y->base;
     const int flags = s.ctl->flags;
     const int cur0 = s.ctl->cur;
     const int64_t step0 = s.ctl->step, left = steps_of_launch(s);
@@ -496,6 +565,18 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     if (threadIdx.x == 0) {
         moved_sh = 0;
         next_sh[0] = next_sh[1] = NW;
+    }
+    if (inter_grid(INTER)) {
+        /* the positions of the first step */
+        base += gridDim.x;
+        const int64_t end = s1 * S < s.N ? s1 * S : s.N;
+        for (int64_t p = s0 * S + threadIdx.x; p < end; p += blockDim.x) {
+            s.ahead[s.N + p] = u_next<STEP_SOFT>(s, s.u[cur0], s.v[cur0], s.a[cur0], p);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            grid_barrier(y, base);
+        }
     }
     __syncthreads();
     int64_t t = 0;
@@ -589,6 +670,10 @@ const void* run_kernel(const DevSys& s, int mode)
         }
     }
     switch (s.inter) {
+        case INTER_LAPLACE2D:
+            return s.pot == POT_CUSPY        ? run_kernel_t<POT_CUSPY, INTER_LAPLACE2D>(mode)
+                   : s.pot == POT_SEMISMOOTH ? run_kernel_t<POT_SEMISMOOTH, INTER_LAPLACE2D>(mode)
+                                             : run_kernel_t<POT_SMOOTH, INTER_LAPLACE2D>(mode);
         case INTER_QUARTIC1D: return run_kernel_t<POT_CUSPY, INTER_QUARTIC1D>(mode);
         case INTER_QUARTICGRAD1D: return run_kernel_t<POT_CUSPY, INTER_QUARTICGRAD1D>(mode);
         case INTER_LAPLACE1D:
@@ -605,7 +690,7 @@ const void* run_kernel(const DevSys& s, int mode)
 RunGeom run_geometry(const DevSys& s)
 {
     RunGeom g = {};
-    if (!(inter_ring(s.inter) || s.inter == INTER_NONE)) {
+    if (!(inter_ring(s.inter) || s.inter == INTER_NONE || s.inter == INTER_LAPLACE2D)) {
         return g;
     }
     int dev = 0, sms = 0, coop = 0;

@@ -362,6 +362,15 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_line(const __
             double uR = (li + 1 < T * PPT && p + 1 < N) ? sh_un[li + 1] : sh_halo[1];
             sfi = add_ring_force<INTER, SOFT>(s, sfi, uL, up, uR);
         }
+        else if (inter_grid(INTER)) {
+            /* Laplace2d, the repeat of the run kernel's pending strips: neighbours recomputed from the old state */
+            const int64_t C = s.cols, col = p % C;
+            const double uU = u_next(s, u0, v0, a0, p >= C ? p - C : p + (N - C));
+            const double uD = u_next(s, u0, v0, a0, p < N - C ? p + C : p - (N - C));
+            const double uL = u_next(s, u0, v0, a0, col == 0 ? p + (C - 1) : p - 1);
+            const double uR = u_next(s, u0, v0, a0, col == C - 1 ? p - (C - 1) : p + 1);
+            sfi = grid_force<SOFT>(s, sfi, uU, uD, uL, up, uR);
+        }
         else {
             sfi = add_zero(sfi);
         }
@@ -574,6 +583,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid(const __
  * the tile's new positions and a recomputed halo of 96 positions per 512 particles, computed by three
  * whole warps (the 8 x 32 tiles of k_step_grid recompute their side columns in one lane per warp and
  * row).  Per particle the same operations in the same order as k_step_grid, so the same results.
+ * Takes single steps and the kernel-by-kernel form of the run loop; longer runs take the run kernel.
  */
 template <int POT, unsigned SOFT = STEP_SOFT>
 __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(const __grid_constant__ DevSys s, int redo)
@@ -666,9 +676,7 @@ __global__ void __launch_bounds__(256, StepOcc<POT>::value) k_step_grid2(const _
         const double uD = sh_un[r + 2][1 + tx];
         const double uL = sh_un[1 + r][tx];
         const double uR = sh_un[1 + r][tx + 2];
-        /* 4 u is exact: the subtraction is one fma (as f + k (...), for a power of two k) */
-        const double lap = FQ_FMA(up[q], -4.0, S_ADD(7, S_ADD(8, FQ_ADD(uU, uD), uL), uR));
-        double sfi = scale_add(lap, s.s_k, sfp);
+        const double sfi = grid_force<SOFT>(s, sfp, uU, uD, uL, up[q], uR);
         double vv, aa, f;
         verlet_velocity<SOFT>(s, sfi, vr[q], ar[q], vv, aa, f);
         s.u[cur ^ 1][p] = up[q];
@@ -1171,6 +1179,19 @@ static void* step_kernel(const DevSys& s, const LineGeom& g)
     }
 }
 
+/* The kernel that repeats the run kernel's pending strips */
+static void* redo_kernel(const DevSys& s, const LineGeom& g)
+{
+    if (s.inter == INTER_LAPLACE2D) {
+        switch (s.pot) {
+            case POT_CUSPY: return (void*)k_step_line<POT_CUSPY, INTER_LAPLACE2D, 1>;
+            case POT_SEMISMOOTH: return (void*)k_step_line<POT_SEMISMOOTH, INTER_LAPLACE2D, 1>;
+            default: return (void*)k_step_line<POT_SMOOTH, INTER_LAPLACE2D, 1>;
+        }
+    }
+    return step_kernel(s, g);
+}
+
 static cudaError_t add_kernel(cudaGraphNode_t* node, cudaGraph_t graph, const cudaGraphNode_t* deps, size_t ndeps,
                               void* func, dim3 grid, dim3 block, void** args)
 {
@@ -1256,8 +1277,9 @@ cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t s
     } while (0)
 
 /*
- * The run graph: WHILE(h_while) { step pass 1, or for Line1d / Particles systems the resident run kernel's
- * many steps ; IF(h_if) { regenerate windows ; redo pending CTAs } ; [2d: reduce + finalise] }.  `s` is updated with the two conditional handles (kernel arguments).
+ * The run graph: WHILE(h_while) { step pass 1, or the resident run kernel's many steps (rg) ; IF(h_if) { regenerate
+ * windows ; redo pending CTAs or strips } ; [grid by tiles: reduce + finalise] }.  `s` is updated with the two
+ * conditional handles (kernel arguments).
  */
 cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cudaGraphExec_t* exec, int mode)
 {
@@ -1276,7 +1298,7 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
     s.h_if = hi;
     s.in_graph = 1;
 
-    bool is2d = inter_grid(s.inter);
+    const bool is2d = inter_grid(s.inter) && !rg.ctas; /* tiles of the grid, else strips of the flat index */
     dim3 grid, block;
     if (is2d) {
         grid = dim3((unsigned)((s.cols + 31) / 32), (unsigned)((s.rows + grid_tile_rows(s) - 1) / grid_tile_rows(s)));
@@ -1286,7 +1308,7 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
         grid = dim3((unsigned)g0.grid);
         block = dim3((unsigned)g0.threads);
     }
-    void* fstep = step_kernel(s, g0);
+    void* fstep = rg.ctas ? redo_kernel(s, g0) : step_kernel(s, g0);
     int pass1 = 0, pass2 = 1;
     void* args1[] = {(void*)&s, (void*)&pass1};
     void* args2[] = {(void*)&s, (void*)&pass2};

@@ -17,6 +17,16 @@ __device__ __forceinline__ double u_next(const DevSys& s, const double* u0, cons
     return S_ADD(3, S_ADD(2, u0[q], S_MULC(0, s.f_dt, s.dt, v0[q])), S_MULC(1, s.f_hdt2, s.hdt2, a0[q]));
 }
 
+/* f + the Laplace2d force of a particle with neighbours above, below, left and right, in the step's operations (sites
+ * 7, 8): 4 u is exact, so its subtraction is one fma (as f + k (...), for a power of two k). */
+template <unsigned SOFT>
+__device__ __forceinline__ double grid_force(const DevSys& s, double f, double uU, double uD, double uL, double u,
+                                             double uR)
+{
+    const double lap = FQ_FMA(u, -4.0, S_ADD(7, S_ADD(8, FQ_ADD(uU, uD), uL), uR));
+    return scale_add(lap, s.s_k, f);
+}
+
 /*
  * The force sum of a particle without interactions and damping, f_frame + f_potential, and f_frame itself.
  * d: centre - u of a Cuspy well (the others take w).  k_frame is most often a power of two or general:
