@@ -7,7 +7,7 @@
  * (tile = threads x particles-per-thread, a power of two); one CTA = one tile of one realisation.
  * Each realisation has a control block (Inst) with its protocol phase, buffer parity, frame position,
  * StopList window and counters.  Every iteration of the run graph's WHILE loop advances every
- * unfinished realisation by one phase step:
+ * unfinished realisation by one phase step (with k_batch_run many phase steps, the realisations independently):
  *   PH_EVT_MIN    maxUniformDisplacement (detail.h:1901-1905, Cuspy :176-187): exact min over particles
  *   PH_EVT_APPLY  advanceUniformly(du - eps/2) (detail.h:1937-1943, 2027-2050)
  *   PH_KICK_APPLY advanceUniformly(eps) (detail.h:1945-1947)
@@ -53,6 +53,8 @@ struct Inst {
     unsigned long long min_key;
     double du_p, du_frame;
     int64_t sl_pos, sl_ge_tol, sl_ge_tol2, sl_asc;
+    uint32_t gen;  /* phase steps finished */
+    uint32_t halt; /* the launch (BatchRun::epoch) of k_batch_run in which it takes no further phase step */
     double ring[BATCH_RING];
 };
 
@@ -66,6 +68,8 @@ struct BatchRun {
     int64_t launch_iters, iters;
     int32_t n_active_tiles; /* entries of BatchDev::active_tiles: the tiles of unfinished realisations */
     int32_t rebuild;        /* a realisation finished this iteration: rebuild the list at its end */
+    uint32_t epoch;         /* k_batch_run: number of this launch; the launch is to end; a wait ran out */
+    int32_t stop, failed;
 };
 
 struct BatchDev {
@@ -78,6 +82,7 @@ struct BatchDev {
     int tile, ppt;
     double2* partials;
     int32_t* tile_pending;
+    uint32_t* tile_gen; /* phase steps taken by each tile */
     int32_t* regen_list;
     double *out_uframe, *out_fframe;
     int64_t *out_S, *out_inc;
@@ -95,9 +100,10 @@ __device__ __forceinline__ uint64_t gtimer()
 struct BShared {
     int skip, phase, cur, last_inst, last_glob, pending, nan, nact, tile;
     double uf, du_p;
+    Scale skf;
     unsigned long long ds;
     unsigned long long mkey;
-    double red[32];
+    double red[64];
 };
 
 /* canonical tree over the tile partials of one realisation (tiles are aligned subtrees) */
@@ -120,10 +126,7 @@ __device__ double2 inst_tree(const double2* partials, int64_t G, double* sh)
         x = t.x;
         y = t.y;
     }
-    double sx = cta_tree(x, sh);
-    __syncthreads();
-    double sy = cta_tree(y, sh);
-    return make_double2(sx, sy);
+    return cta_tree2(x, y, sh);
 }
 
 /* per-realisation state machine; thread 0 of the realisation's last CTA; tot = tree of tile partials */
@@ -158,15 +161,15 @@ __device__ void inst_finalize(const BatchDev& b, Inst* I, int j, double2 tot)
                     I->sl_ge_tol2 -= 1;
                 }
                 if (n >= 2) {
-                    if (I->ring[(pos + 1) % n] > old) {
+                    if (I->ring[pos + 1 < n ? pos + 1 : 0] > old) {
                         I->sl_asc -= 1;
                     }
-                    if (r > I->ring[(pos + n - 1) % n]) {
+                    if (r > I->ring[pos > 0 ? pos - 1 : n - 1]) {
                         I->sl_asc += 1;
                     }
                 }
                 I->ring[pos] = r;
-                I->sl_pos = (pos + 1) % n;
+                I->sl_pos = pos + 1 < n ? pos + 1 : 0;
                 if (r >= R->tol) {
                     I->sl_ge_tol += 1;
                 }
@@ -291,7 +294,7 @@ __device__ void rebuild_active_tiles(const BatchDev& b)
     __threadfence();
 }
 
-/* global end of one loop iteration (thread 0 of the grid's last CTA of this pass) */
+/* global end of one loop iteration (thread 0 of the CTA that ends it) */
 __device__ void batch_iteration_end(const BatchDev& b, bool redo)
 {
     BatchRun* R = b.run;
@@ -317,7 +320,7 @@ __device__ void batch_iteration_end(const BatchDev& b, bool redo)
     }
     R->launch_iters += 1;
     R->iters += 1;
-    bool more = R->active > 0 && R->walk_flag == 0 && (now - R->launch_t0) < R->budget_ns;
+    bool more = R->active > 0 && R->walk_flag == 0 && R->failed == 0 && (now - R->launch_t0) < R->budget_ns;
     __threadfence();
     if (b.in_graph) {
         cudaGraphSetConditional((cudaGraphConditionalHandle)b.h_while, more ? 1u : 0u);
@@ -329,22 +332,10 @@ __device__ void batch_iteration_end(const BatchDev& b, bool redo)
  * neighbours on the realisation's ring come from shared memory or are recomputed at the tile edges.
  */
 template <int PPT>
-__global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
+__device__ __forceinline__ void batch_tile(const BatchDev& b, BShared& sh, double* sh_un, const int64_t t,
+                                           const int redo, const bool resident, const uint32_t epoch,
+                                           const uint64_t t_end)
 {
-    __shared__ BShared sh;
-    __shared__ double sh_un[256 * PPT];
-    if (threadIdx.x == 0) {
-        /* CTA k takes the k-th tile of an unfinished realisation; the others have nothing to do.  While
-         * no realisation has finished the list is the identity (no second dependent load). */
-        sh.nact = ((volatile BatchRun*)b.run)->n_active_tiles;
-        sh.tile = sh.nact == (int)b.ntiles ? (int)blockIdx.x
-                                            : ((int)blockIdx.x < sh.nact ? b.active_tiles[blockIdx.x] : -1);
-    }
-    __syncthreads();
-    if (sh.tile < 0) {
-        return;
-    }
-    const int64_t t = sh.tile;
     const int j = b.tile_inst[t];
     Inst* I = b.inst + j;
     const DevSys& s = b.d;
@@ -354,6 +345,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
         sh.cur = vi->cur;
         sh.uf = vi->u_frame;
         sh.du_p = vi->du_p;
+        sh.skf = I->s_kf;
         sh.skip = redo ? !b.tile_pending[t] : 0;
         sh.pending = 0;
         sh.nan = 0;
@@ -386,7 +378,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
     if (phase == PH_MIN_STEP) {
         constexpr unsigned SOFT = STEP_SOFT; /* fp64 / integer-pipe split of the step's operations */
         const double uf = sh.uf;
-        const Scale skf = I->s_kf;
+        const Scale& skf = sh.skf;
         double un[PPT], vr[PPT], ar[PPT];
 #pragma unroll
         for (int q = 0; q < PPT; ++q) {
@@ -588,9 +580,9 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
     bool tree = phase == PH_MIN_STEP || phase == PH_REPORT;
     double sf = 0.0, sff = 0.0;
     if (tree) {
-        sf = cta_tree(rf, sh.red);
-        __syncthreads();
-        sff = cta_tree(rff, sh.red);
+        const double2 sum = cta_tree2(rf, rff, sh.red);
+        sf = sum.x;
+        sff = sum.y;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -622,6 +614,10 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
                 sh.last_inst = (k == (unsigned)I->ntiles - 1u) && I->n_pending == 0;
                 if (k == (unsigned)I->ntiles - 1u && I->n_pending > 0) {
                     I->ticket = 0; /* the redo of this realisation's pending tiles finalises */
+                    if (resident) {
+                        ((volatile BatchRun*)b.run)->stop = 1;
+                        ((volatile Inst*)I)->halt = epoch;
+                    }
                 }
             }
         }
@@ -635,7 +631,16 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
         }
         if (threadIdx.x == 0) {
             inst_finalize(b, I, j, tot);
+            if (resident && (((volatile BatchRun*)b.run)->stop || gtimer() >= t_end)) {
+                ((volatile Inst*)I)->halt = epoch;
+            }
+            /* after what the phase step has written (fences: the CTAs' tickets, inst_finalize) */
+            __threadfence();
+            ((volatile Inst*)I)->gen = I->gen + 1u;
         }
+    }
+    if (resident) {
+        return;
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -658,6 +663,112 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchDev b, int redo)
         }
         if (threadIdx.x == 0) {
             batch_iteration_end(b, redo != 0);
+        }
+    }
+}
+
+/* One pass over the batch: CTA k takes the k-th tile of an unfinished realisation; the others have nothing to
+ * do.  redo: only tiles marked pending (after k_batch_regen moved their particles' windows). */
+template <int PPT>
+__global__ void __launch_bounds__(256, 4) k_batch(const __grid_constant__ BatchDev b, int redo)
+{
+    __shared__ BShared sh;
+    __shared__ double sh_un[256 * PPT];
+    if (threadIdx.x == 0) {
+        /* while no realisation has finished the list is the identity (no second dependent load) */
+        sh.nact = ((volatile BatchRun*)b.run)->n_active_tiles;
+        sh.tile = sh.nact == (int)b.ntiles ? (int)blockIdx.x
+                                            : ((int)blockIdx.x < sh.nact ? b.active_tiles[blockIdx.x] : -1);
+    }
+    __syncthreads();
+    if (sh.tile >= 0) {
+        batch_tile<PPT>(b, sh, sh_un, sh.tile, redo, false, 0u, 0ull);
+    }
+}
+
+constexpr uint64_t BATCH_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
+
+/*
+ * Many phase steps of every realisation in one cooperative launch, until windows must move, all realisations are
+ * finished or the launch's time is up.  (A pass of k_batch per phase step pays the graph loop's iteration, a launch
+ * and the grid's ticket: 23 us a step with 10276 particles, 12 us here.)  CTA c owns the tiles c, c + gridDim, ... and takes whichever of them is
+ * ready: a tile takes its next phase step when its realisation has finished the one before (Inst::gen).  So no
+ * realisation waits for another one, and where a CTA has several tiles the end of one realisation's step
+ * (tickets, residual, stop test) passes beside the step of another.
+ * A tile whose windows must move ends the launch (BatchRun::stop): its realisation stays unfinished for the
+ * redo, the others halt after the phase step they are in.  The waits are on resident CTAs and end after BATCH_WAIT_NS.
+ */
+template <int PPT>
+__global__ void __launch_bounds__(256, 4) k_batch_run(const __grid_constant__ BatchDev b)
+{
+    __shared__ BShared sh;
+    __shared__ double sh_un[256 * PPT];
+    volatile BatchRun* R = b.run;
+    const uint32_t epoch = R->epoch;
+    const uint64_t t_end = gtimer() + R->budget_ns;
+    const int own = (int)((b.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x); /* tiles of this CTA */
+    int first = 0; /* the one looked at first */
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            /* the next ready tile, 32 of them looked at together, or none: all are finished or halted */
+            const int lane = threadIdx.x;
+            int take = -1;
+            uint64_t t0 = 0;
+            for (unsigned i = 1; take < 0; ++i) {
+                bool waiting = false;
+                for (int m0 = 0; m0 < own && take < 0; m0 += 32) {
+                    int m = first + m0 + lane;
+                    m = m >= own ? m - own : m;
+                    const bool in = m0 + lane < own;
+                    const int64_t t = blockIdx.x + (int64_t)(in ? m : 0) * gridDim.x;
+                    const volatile Inst* I = b.inst + b.tile_inst[t];
+                    const uint32_t gen = I->gen;
+                    __threadfence();
+                    const bool alive = in && I->halt != epoch && I->phase != PH_DONE;
+                    const bool ready = alive && gen == b.tile_gen[t];
+                    const unsigned r = __ballot_sync(0xffffffffu, ready);
+                    waiting = waiting || __any_sync(0xffffffffu, alive);
+                    if (r) {
+                        const int src = __ffs(r) - 1;
+                        if (lane == src) {
+                            b.tile_gen[t] = gen + 1u;
+                        }
+                        const int mt = __shfl_sync(0xffffffffu, m, src);
+                        take = (int)(blockIdx.x + (int64_t)mt * gridDim.x);
+                        first = mt + 1 < own ? mt + 1 : 0;
+                    }
+                }
+                if (take >= 0 || !waiting) {
+                    break;
+                }
+                if ((i & 255u) == 0u) {
+                    const uint64_t now = gtimer();
+                    t0 = t0 == 0 ? now : t0;
+                    if (__any_sync(0xffffffffu, R->failed || now - t0 > BATCH_WAIT_NS)) {
+                        R->failed = 1;
+                        break;
+                    }
+                }
+            }
+            if (lane == 0) {
+                sh.tile = take;
+            }
+        }
+        __syncthreads();
+        if (sh.tile < 0) {
+            break;
+        }
+        batch_tile<PPT>(b, sh, sh_un, sh.tile, 0, true, epoch, t_end);
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&b.run->ticket, 1u) == gridDim.x - 1u) {
+            /* all CTAs are through */
+            __threadfence();
+            R->stop = 0;
+            R->epoch = epoch + 1u;
+            batch_iteration_end(b, false);
         }
     }
 }
@@ -763,6 +874,27 @@ static cudaError_t add_cond(cudaGraphNode_t* node, cudaGraph_t graph, const cuda
     return e;
 }
 
+/*
+ * CTAs of k_batch_run: as many as can be resident together; 0: a pass of k_batch per iteration of the graph's loop
+ * instead, where a CTA would own more than two tiles.  A pass has 17 us of fixed cost, k_batch_run 4, but there
+ * each tile pays for being looked for.  One quasistatic cycle by tiles of 128 x 2, passes and k_batch_run: 10276
+ * particles 85 and 55 ms, 253727 117 and 93, 671087 (two to three tiles per CTA) 201 and 213, 2761199 616 and 830.
+ */
+static unsigned batch_resident_ctas(const BatchDev& b, int threads)
+{
+    const void* f = b.ppt == 2 ? (const void*)k_batch_run<2> : (const void*)k_batch_run<1>;
+    int dev = 0, sms = 0, coop = 0, per = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, threads, 0) != cudaSuccess || !coop) {
+        cudaGetLastError();
+        return 0;
+    }
+    const int64_t most = (int64_t)per * sms;
+    return b.ntiles > 2 * most ? 0u : (unsigned)std::min(b.ntiles, most);
+}
+
 static cudaError_t build_batch_graph(BatchDev& b, int threads, cudaGraphExec_t* exec)
 {
     cudaGraph_t g;
@@ -793,7 +925,17 @@ static cudaError_t build_batch_graph(BatchDev& b, int threads, cudaGraphExec_t* 
     void* a2[] = {(void*)&b, (void*)&pass2};
     void* ar[] = {(void*)&b};
     cudaGraphNode_t ns, nif, nr, nd;
-    BG(add_kernel_node(&ns, body, nullptr, 0, fk, dim3((unsigned)b.ntiles), dim3((unsigned)threads), a1));
+    const unsigned resident = batch_resident_ctas(b, threads);
+    if (resident) {
+        void* fr = b.ppt == 2 ? (void*)k_batch_run<2> : (void*)k_batch_run<1>;
+        BG(add_kernel_node(&ns, body, nullptr, 0, fr, dim3(resident), dim3((unsigned)threads), ar));
+        cudaKernelNodeAttrValue coop = {};
+        coop.cooperative = 1;
+        BG(cudaGraphKernelNodeSetAttribute(ns, cudaLaunchAttributeCooperative, &coop));
+    }
+    else {
+        BG(add_kernel_node(&ns, body, nullptr, 0, fk, dim3((unsigned)b.ntiles), dim3((unsigned)threads), a1));
+    }
     cudaGraph_t ifb;
     BG(add_cond(&nif, body, &ns, 1, hi, cudaGraphCondTypeIf, &ifb));
     BG(add_kernel_node(&nr, ifb, nullptr, 0, (void*)k_batch_regen, dim3(4 * 152), dim3(128), ar));
@@ -875,6 +1017,33 @@ static cudaError_t balloc(fqsb_batch* h, T** p, size_t count)
     return e;
 }
 
+/*
+ * Tile where the caller leaves it open: 128 threads x 1 particle while all tiles are resident together (8 CTAs per
+ * SM), x 2 up to four times as many, else 256 x 2.  One quasistatic cycle by tiles of 128 x 1, 128 x 2 and 256 x 2:
+ * 10276 particles 44, 55 and 57 ms, 253727 150, 93 and 94, 671087 230, 201 and 215, 2761199 770, 616 and 596.
+ */
+static void batch_default_tile(const fqsb_batch_config* c, int& threads, int& ppt)
+{
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
+        cudaGetLastError();
+    }
+    auto tiles = [&](int64_t tile) {
+        int64_t k = 0;
+        for (int64_t j = 0; j < c->n_instances; ++j) {
+            k += (std::max(c->sizes[j], (int64_t)0) + tile - 1) / tile;
+        }
+        return k;
+    };
+    const int64_t most = 8 * (int64_t)sms;
+    if (threads == 0) {
+        threads = tiles(128 * (int64_t)(ppt ? ppt : 2)) <= 4 * most ? 128 : 256;
+    }
+    if (ppt == 0) {
+        ppt = tiles(threads) <= most * 128 / threads ? 1 : 2;
+    }
+}
+
 extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
 {
     FQSB_API_RANGE();
@@ -884,10 +1053,8 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     if (c->nchunk < 34 || c->window < 34 || c->window > c->nchunk || c->n_parameters < 0 || c->n_parameters > 4) {
         return berr(nullptr, FQSB_ERR_INVALID, "need 34 <= window <= nchunk and at most 4 parameters");
     }
-    /* default tile: 256 threads x 2 particles (measured fastest of the autotuner's candidates on a
-     * log-uniform [256, 65536] batch: 15.6 G particle-steps/s against 11.6 for 256 x 1) */
-    int threads = c->threads ? c->threads : 256;
-    int ppt = c->ppt ? c->ppt : 2;
+    int threads = c->threads, ppt = c->ppt;
+    batch_default_tile(c, threads, ppt);
     if (!(threads == 32 || threads == 64 || threads == 128 || threads == 256) || !(ppt == 1 || ppt == 2)) {
         return berr(nullptr, FQSB_ERR_INVALID, "threads must be 32, 64, 128 or 256 and ppt 1 or 2");
     }
@@ -1045,6 +1212,7 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     b.tile_inst = ti;
     BA(b.partials, (size_t)b.ntiles);
     BA(b.tile_pending, (size_t)b.ntiles);
+    BA(b.tile_gen, (size_t)b.ntiles);
     BA(b.active_tiles, (size_t)b.ntiles);
     b.ninst = h->ninst;
     BA(b.regen_list, N);
@@ -1171,7 +1339,9 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
         I.nan_flag = 0;
         I.s_signed = 0;
         I.min_key = 0x7ff0000000000000ULL;
+        I.gen = I.halt = 0;
     }
+    QCU(cudaMemsetAsync(b.tile_gen, 0, sizeof(uint32_t) * (size_t)b.ntiles, h->stream));
     QCU(cudaMemcpyAsync(b.inst, inst.data(), sizeof(Inst) * inst.size(), cudaMemcpyHostToDevice, h->stream));
     BatchRun R;
     memset(&R, 0, sizeof(R));
@@ -1186,6 +1356,7 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
     /* every realisation starts the protocol: all tiles are active */
     R.n_active_tiles = (int32_t)b.ntiles;
     R.rebuild = 0;
+    R.epoch = 1;
     {
         std::vector<int32_t> all((size_t)b.ntiles);
         for (size_t k = 0; k < all.size(); ++k) {
@@ -1223,7 +1394,7 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
             QCU(cudaGraphLaunch(h->graph, h->stream));
             QCU(cudaMemcpyAsync(&R, b.run, sizeof(R), cudaMemcpyDeviceToHost, h->stream));
             QCU(cudaStreamSynchronize(h->stream));
-            if (R.active <= 0 || R.walk_flag) {
+            if (R.active <= 0 || R.walk_flag || R.failed) {
                 break;
             }
             int64_t zero = 0;
@@ -1242,6 +1413,9 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
     }
     if (R.walk_flag) {
         return berr(h, FQSB_ERR_TIMEOUT, "yield search exceeded its bound");
+    }
+    if (R.failed) {
+        return berr(h, FQSB_ERR_CUDA, "batch: a CTA waited in vain for the end of a pass");
     }
     return FQSB_OK;
 }
