@@ -147,6 +147,7 @@ struct Thermal {
 struct RunSync {
     unsigned long long arrived; /* arrivals at the grid barrier, over all launches */
     unsigned long long base;    /* arrivals before the next launch */
+    unsigned long long left;    /* CTAs that have read the flags after their last barrier of the launch */
     int32_t failed;             /* a wait at the barrier ran out */
     int32_t stop[2];            /* the run stops after the step before this one */
     int32_t pending[2];         /* strips with a particle whose chunk window must move */

@@ -57,14 +57,11 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
-/* Grid barrier up to `want` arrivals, for thread 0 of a CTA (the others wait at a CTA barrier on both sides);
- * false when it ran out. */
-__device__ __forceinline__ bool grid_barrier(RunSync* y, unsigned long long want)
+/* Waits until a counter of y has reached `want`; false when the wait ran out. */
+__device__ __forceinline__ bool wait_for(RunSync* y, const unsigned long long* counter, unsigned long long want)
 {
-    __threadfence();
-    atomicAdd(&y->arrived, 1ull);
     uint64_t t0 = 0;
-    for (unsigned k = 1; load_acquire(&y->arrived) < want; ++k) {
+    for (unsigned k = 1; load_acquire(counter) < want; ++k) {
         if ((k & 255u) == 0u) {
             if (((volatile RunSync*)y)->failed) {
                 return false;
@@ -78,6 +75,15 @@ __device__ __forceinline__ bool grid_barrier(RunSync* y, unsigned long long want
         }
     }
     return true;
+}
+
+/* Grid barrier up to `want` arrivals, for thread 0 of a CTA (the others wait at a CTA barrier on both sides);
+ * false when it ran out. */
+__device__ __forceinline__ bool grid_barrier(RunSync* y, unsigned long long want)
+{
+    __threadfence();
+    atomicAdd(&y->arrived, 1ull);
+    return wait_for(y, &y->arrived, want);
 }
 
 /* The barrier after step t; returns how the launch goes on. */
@@ -488,9 +494,11 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     if (tid == 0) {
         volatile RunSync* vy = y;
         const int q = (int)(t & 1);
-        if (how == END_BARRIER) {
+        /* the flags below are cleared for the next launch: every CTA has to have read them after its last barrier */
+        if (how == END_BARRIER || vy->failed || !wait_for(y, &y->left, gridDim.x - 1u)) {
             sc.error = DERR_BARRIER;
         }
+        vy->left = 0;
         if (how == END_PENDING) {
             /* step t is finished by the repeat of its pending strips; what its other strips counted stays */
             sc.s_sum = (long long)((unsigned long long)sc.s_sum + (unsigned long long)vy->ds[q]);
@@ -634,6 +642,10 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
         if (how_sh != END_NOT) {
             break;
         }
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&y->left, 1ull);
     }
     if (how_sh == END_STOPPED) {
         /* drop step t: its wells back to those of its input state, its marks cleared */

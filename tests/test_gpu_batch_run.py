@@ -29,6 +29,9 @@ def test_tiles_per_cta(monkeypatch, count, hi, threads, ppt):
             out[-1]["u"] = np.concatenate([b.field(j, "u") for j in range(count)])
             out[-1]["i"] = np.concatenate([b.index_at_align(j) for j in range(count)])
         del b
-    for k in ("u_frame", "f_frame", "S", "inc", "status", "u", "i"):
-        assert np.array_equal(out[0][k], out[2][k], equal_nan=True), k
-        assert np.array_equal(out[1][k], out[3][k], equal_nan=True), k
+    for a, b in ((out[0], out[2]), (out[1], out[3])):
+        for k in ("status", "u", "i"):
+            assert np.array_equal(a[k], b[k]), k
+        for k in ("u_frame", "f_frame", "S", "inc"):
+            # (a realisation that reached max_iter has no outputs of its last cycle)
+            assert np.array_equal(a[k][a["status"] == 0], b[k][b["status"] == 0]), k
