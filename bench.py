@@ -61,9 +61,9 @@ PAR = dict(m=1.0, eta=0.1, mu=1.0, k_interactions=1.0, dt=0.1, seed=1, distribut
 V_FRAME = 1e-3  # u_frame += v_frame * dt = 1e-4 per step
 BYTES_PER_PARTICLE_STEP = 64  # read+write u, v, a (48 B) + read the current well {y_left, y_right} (16 B)
 FP64_OPS_PER_PARTICLE_STEP = 24  # binary64 add/mul of the exact-order step; compares and 2^k scalings are integer work
-# of those, the step kernel issues these on the fp64 pipe; the rest (the 8 multiplications and the 2 additions of
-# the position update) run bit-identically on the integer pipes (csrc/fq_soft64.h)
-FP64_PIPE_OPS_PER_PARTICLE_STEP = 14
+# of those, the run kernel's flow steps issue these on the fp64 pipe; the rest (the 8 multiplications and 6 additions) run
+# bit-identically on the integer pipes (csrc/fq_soft64.h)
+FP64_PIPE_OPS_PER_PARTICLE_STEP = 10
 STEP_PROFILE = ROOT / "profiles" / "k_step_line_cuspy_laplace1d_N4M.md"
 FORMS = ("small_system", "line2d", "batched", "adjoint", "next_rows")
 
@@ -649,10 +649,10 @@ def main():
     t_wall = time.perf_counter() - t_wall0
     clk = clocks.stop()
     dev_s = max_over_ranks(e0.elapsed_time(e1) / 1e3)
-    launches = args.steps * INNER
+    launches = args.steps  # the resident run kernel takes the INNER time steps of a flowSteps in one launch
     particle_steps = N * INNER * args.steps
     value = world * particle_steps / dev_s
-    kernel_s = dev_s / launches
+    kernel_s = dev_s / (args.steps * INNER)  # per time step
     hbm_peak, peak_kind = peaks()
     achieved_gbs = BYTES_PER_PARTICLE_STEP * N / kernel_s / 1e9
 
@@ -730,9 +730,10 @@ def main():
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                      "frac": achieved_gbs / hbm_peak, "traffic": traffic,
-                     "traffic_unit": "bytes per launch (ncu capture of " + STEP_PROFILE.name + ", scaled by N)",
+                     "traffic_unit": "bytes per time step (ncu capture of the one-kernel-per-step form, " + STEP_PROFILE.name +
+                                     ", scaled by N)",
                      "peak_kind": peak_kind, "algorithmic_bytes_per_particle_step": BYTES_PER_PARTICLE_STEP,
-                     "kernel": "k_step_line<Cuspy, Laplace1d, 2 per thread>", "kernel_us": kernel_s * 1e6},
+                     "kernel": "k_run_line<Cuspy, Laplace1d>, per time step", "kernel_us": kernel_s * 1e6},
         "fp64": {"ops_per_particle_step": FP64_OPS_PER_PARTICLE_STEP,
                  "ops_on_fp64_pipe": FP64_PIPE_OPS_PER_PARTICLE_STEP,
                  "ops_on_integer_pipes": FP64_OPS_PER_PARTICLE_STEP - FP64_PIPE_OPS_PER_PARTICLE_STEP,
