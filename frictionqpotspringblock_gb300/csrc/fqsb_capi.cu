@@ -712,7 +712,8 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
             }
             cudaError_t le = cudaSuccess;
             /* with thermal forcing a launch takes the planned steps: several plans and launches per wait */
-            const int64_t launches = h->d.f_th ? std::min((int64_t)16, (max_steps - c->step + h->d.th_K - 1) / h->d.th_K) : 1;
+            const int64_t left = max_steps - c->step;
+            const int64_t launches = !h->d.f_th ? 1 : left / 16 >= h->d.th_K ? 16 : (left + h->d.th_K - 1) / h->d.th_K;
             for (int64_t k = 0; k < launches && le == cudaSuccess; ++k) {
                 if (h->d.f_th) {
                     CU(h, launch_thermal_plan(h->d, h->d.th_K, TH_FROM_RUN, 0, h->stream));

@@ -1,0 +1,42 @@
+"""Thermal forcing at the limits of its plans (csrc/fqsb_thermal.cu): the largest numbers of steps, and plans of
+few steps over many particles."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def both(n, **kw):
+    import frictionqpotspringblock_gb300 as fqsb
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(n)
+    par = dict(m=1.0, eta=0.3, mu=1.0, k_interactions=1.0, k_frame=0.1, dt=0.1, mean=0.05, stddev=0.4, seed_forcing=9,
+               dinc_init=rng.integers(0, 40, n), dinc=rng.integers(1, 40, n), shape=[n], seed=4,
+               distribution="weibull", parameters=[2.0, 1.0, 1e-5], offset=-20.0, nchunk=45)
+    par.update(kw)
+    gpu = fqsb.Line1d.System_Cuspy_Laplace_RandomForcing(**par)
+    ref = O.line1d_random_forcing(**par, sum_mode=O.SUM_PAIRWISE, math_mode=O.MATH_PORTABLE)
+    return gpu, ref
+
+
+def same(gpu, ref):
+    for name in ("u", "v", "a", "f", "f_frame"):
+        assert np.array_equal(getattr(gpu, name), getattr(ref, name)), name
+    assert np.array_equal(gpu.external.f_thermal, ref.f_thermal)
+    assert np.array_equal(gpu.external.next, ref.thermal_next)
+    assert gpu.external.state == ref.thermal_state
+    assert np.array_equal(gpu.chunk.index_at_align, ref.chunk.index_at_align)
+    assert gpu.inc == ref.inc
+
+
+@pytest.mark.parametrize("path", ["cluster", "graph"])
+@pytest.mark.parametrize("max_iter", [2 ** 63 - 1, 2 ** 63 - 200, 4096, 4095])
+def test_many_steps_allowed(monkeypatch, path, max_iter):
+    """The number of launches for the steps allowed does not overflow."""
+    if path == "graph":
+        monkeypatch.setenv("FQSB_NO_SMALL", "1")
+    gpu, ref = both(1000, stddev=0.05)
+    assert gpu.timeStepsUntilEvent(max_iter=max_iter) == ref.timeStepsUntilEvent(max_iter=min(max_iter, 10 ** 9))
+    same(gpu, ref)
