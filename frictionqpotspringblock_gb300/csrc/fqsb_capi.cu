@@ -632,7 +632,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     }
     if (np) {
         if (h->use_graph && !h->graph_np) {
-            CU(h, build_nopass_graph(h->d, h->lg, *np, &h->graph_np));
+            CU(h, build_nopass_graph(h->d, line_geometry(h->d.N), *np, &h->graph_np));
         }
         if (!h->use_graph) {
             h->d.in_graph = 0;
@@ -701,7 +701,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
                 DevSys d = h->d;
                 d.in_graph = 0;
                 for (int i = 0; i < 64; ++i) {
-                    CU(h, launch_nopass_iteration(d, h->lg, *np, h->stream));
+                    CU(h, launch_nopass_iteration(d, line_geometry(h->d.N), *np, h->stream));
                 }
             }
         }
@@ -1286,7 +1286,7 @@ extern "C" int fqsb_minimise_nopassing(fqsb_system* h, double tol, uint64_t nite
     A.f_frame = h->fs[2];
     A.f = h->fs[4];
     A.den = 2 * h->d.k + h->d.k_frame + h->d.mu;
-    A.ppt = h->lg.ppt;
+    A.ppt = line_geometry(h->d.N).ppt;
     RunResult r; /* (the force arrays, kernel arguments of the graph, live as long as the handle) */
     int rc = run(h, (int64_t)max_iter, RF_RESID | RF_NOINC, tol, (int64_t)niter_tol, 0.0, 0, 0, nullptr, &r, nullptr,
                  &A);
