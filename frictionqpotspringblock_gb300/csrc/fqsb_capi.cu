@@ -1554,10 +1554,10 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         e = cudaMalloc(&di, sizeof(int64_t) * (size_t)N);
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&cnt, sizeof(int64_t) * (size_t)K);
+        e = cudaMalloc(&cnt, sizeof(int64_t) * (size_t)(K * th_blocks(words)));
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&cum, sizeof(int64_t) * (size_t)(K + 1));
+        e = cudaMalloc(&cum, sizeof(int64_t) * (size_t)(K * th_blocks(words) + 1));
     }
     if (e == cudaSuccess) {
         e = cudaMalloc(&list, sizeof(int64_t) * (size_t)(K * N));

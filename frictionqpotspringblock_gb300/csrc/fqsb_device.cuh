@@ -270,8 +270,8 @@ struct DevSys {
     /* the draws of the next th_K steps (fqsb_thermal.cu); th_words = ceil(N / 32) words per step */
     int64_t th_K, th_words;
     uint32_t* th_mask;  /* [th_K + 2][th_words]: which particles draw; the last two rows stay 0 */
-    int64_t* th_cnt;    /* [th_K] draws per step */
-    int64_t* th_cum;    /* [th_K + 1] draws before a step */
+    int64_t* th_cnt;    /* [th_K][th_blocks] draws of a block of particles in a step */
+    int64_t* th_cum;    /* [th_K * th_blocks + 1] draws before a block's of a step */
     int64_t* th_list;   /* the draws in order: step * N + particle (capacity th_K * N) */
     double* th_val;     /* [th_K][N] the drawn forces */
     double* th_w[2];    /* the run kernel's f_thermal after even and odd steps of a launch */

@@ -86,7 +86,11 @@ __device__ __forceinline__ int64_t cta_exclusive_scan256(int64_t x, int64_t* sh8
     return before + incl - x;
 }
 
-/* One CTA per planned step counts its draws; the last one turns the counts into the draws before each step. */
+/*
+ * The CTA (b, k) counts the draws of 8192 particles (256 words of the mask) in planned step k; the last one turns
+ * the counts into the draws before each of them.  (One CTA per step, whatever the size, left the GPU idle in plans
+ * of few steps over many particles: a step of 2^22 particles took 300 us longer.)
+ */
 __global__ void __launch_bounds__(256) k_th_count(const __grid_constant__ DevSys s, int K, int from, int64_t inc_arg)
 {
     __shared__ int64_t sh8[8];
@@ -95,35 +99,41 @@ __global__ void __launch_bounds__(256) k_th_count(const __grid_constant__ DevSys
     if (!th_first_inc(s, from, inc_arg, inc, K)) {
         return;
     }
-    const uint32_t* row = s.th_mask + (int64_t)blockIdx.x * s.th_words;
+    const int64_t B = gridDim.x, w = (int64_t)blockIdx.x * 256 + threadIdx.x;
     int64_t n = 0, total;
-    for (int64_t i = threadIdx.x; (int)blockIdx.x < K && i < s.th_words; i += 256) {
-        n += __popc(row[i]);
+    if ((int)blockIdx.y < K && w < s.th_words) {
+        n = __popc(s.th_mask[(int64_t)blockIdx.y * s.th_words + w]);
     }
     cta_exclusive_scan256(n, sh8, &total);
     if (threadIdx.x == 0) {
-        s.th_cnt[blockIdx.x] = total;
+        s.th_cnt[blockIdx.y * B + blockIdx.x] = total;
         __threadfence();
-        sh_last = atomicAdd(&s.th->ticket, 1u) == gridDim.x - 1u ? 1 : 0;
+        sh_last = atomicAdd(&s.th->ticket, 1u) == gridDim.x * gridDim.y - 1u ? 1 : 0;
     }
     __syncthreads();
     if (!sh_last) {
         return;
     }
     __threadfence();
-    const int64_t x = (int)threadIdx.x < K ? __ldcg(s.th_cnt + threadIdx.x) : 0;
-    const int64_t before = cta_exclusive_scan256(x, sh8, &total);
-    if ((int)threadIdx.x < K) {
-        s.th_cum[threadIdx.x] = before;
+    /* consecutive counts to each thread */
+    const int64_t M = (int64_t)K * B, per = (M + 255) / 256, i0 = threadIdx.x * per, i1 = i0 + per < M ? i0 + per : M;
+    int64_t x = 0;
+    for (int64_t i = i0; i < i1; ++i) {
+        x += __ldcg(s.th_cnt + i);
+    }
+    int64_t before = cta_exclusive_scan256(x, sh8, &total);
+    for (int64_t i = i0; i < i1; ++i) {
+        s.th_cum[i] = before;
+        before += __ldcg(s.th_cnt + i);
     }
     if (threadIdx.x == 0) {
-        s.th_cum[K] = total;
+        s.th_cum[M] = total;
         s.th->total = total;
         s.th->ticket = 0u;
     }
 }
 
-/* One CTA per planned step lists its draws in particle order. */
+/* The CTA (b, k) lists the draws of its 8192 particles in planned step k in particle order. */
 __global__ void __launch_bounds__(256) k_th_list(const __grid_constant__ DevSys s, int K, int from, int64_t inc_arg)
 {
     __shared__ int64_t sh8[8];
@@ -131,20 +141,16 @@ __global__ void __launch_bounds__(256) k_th_list(const __grid_constant__ DevSys 
     if (!th_first_inc(s, from, inc_arg, inc, K)) {
         return;
     }
-    if ((int)blockIdx.x >= K) {
+    if ((int)blockIdx.y >= K) {
         return;
     }
-    const uint32_t* row = s.th_mask + (int64_t)blockIdx.x * s.th_words;
-    int64_t base = s.th_cum[blockIdx.x];
-    for (int64_t w0 = 0; w0 < s.th_words; w0 += 256) {
-        const int64_t w = w0 + threadIdx.x;
-        uint32_t word = w < s.th_words ? row[w] : 0u;
-        int64_t total;
-        int64_t k = base + cta_exclusive_scan256(__popc(word), sh8, &total);
-        for (; word; word &= word - 1u) {
-            s.th_list[k++] = (int64_t)blockIdx.x * s.N + 32 * w + (__ffs((int)word) - 1);
-        }
-        base += total;
+    const int64_t w = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    uint32_t word = w < s.th_words ? s.th_mask[(int64_t)blockIdx.y * s.th_words + w] : 0u;
+    int64_t total;
+    int64_t k = cta_exclusive_scan256(__popc(word), sh8, &total);
+    k += s.th_cum[(int64_t)blockIdx.y * gridDim.x + blockIdx.x];
+    for (; word; word &= word - 1u) {
+        s.th_list[k++] = (int64_t)blockIdx.y * s.N + 32 * w + (__ffs((int)word) - 1);
     }
 }
 
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSy
     }
     if (p == 0 && steps > 0) {
         Thermal* th = s.th;
-        th->state = pcg_advance_inc(th->state, (uint64_t)s.th_cum[steps], th->inc);
+        th->state = pcg_advance_inc(th->state, (uint64_t)s.th_cum[steps * th_blocks(s.th_words)], th->inc);
     }
 }
 
@@ -211,10 +217,10 @@ static cudaError_t for_plan(const DevSys& s, int64_t K, int from, int64_t inc, F
     int k = (int)K;
     void* args[] = {(void*)&s, (void*)&k, (void*)&from, (void*)&inc};
     void* args_eval[] = {(void*)&s, (void*)&from, (void*)&inc};
-    const dim3 parts((unsigned)((s.N + 255) / 256)), steps((unsigned)K);
+    const dim3 parts((unsigned)((s.N + 255) / 256)), blocks((unsigned)th_blocks(s.th_words), (unsigned)K);
     const ThLaunch all[4] = {{(void*)k_th_mask, parts, dim3(256), args},
-                             {(void*)k_th_count, steps, dim3(256), args},
-                             {(void*)k_th_list, steps, dim3(256), args},
+                             {(void*)k_th_count, blocks, dim3(256), args},
+                             {(void*)k_th_list, blocks, dim3(256), args},
                              {(void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), args_eval}};
     for (const ThLaunch& l : all) {
         const cudaError_t e = launch(l);

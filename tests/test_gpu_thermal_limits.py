@@ -40,3 +40,24 @@ def test_many_steps_allowed(monkeypatch, path, max_iter):
     gpu, ref = both(1000, stddev=0.05)
     assert gpu.timeStepsUntilEvent(max_iter=max_iter) == ref.timeStepsUntilEvent(max_iter=min(max_iter, 10 ** 9))
     same(gpu, ref)
+
+
+@pytest.mark.parametrize("n", [8191, 8193, 2 ** 19 + 1])
+def test_blocks_of_particles(monkeypatch, n):
+    """The draws are counted and listed by blocks of 8192 particles: their edges, and many of them."""
+    gpu, ref = both(n, dinc=np.random.default_rng(n).choice([1, 3, 50, 100000], n, p=[0.05, 0.05, 0.4, 0.5]))
+    for k in (1, 33) if n > 100000 else (1, 300, 2):
+        gpu.flowSteps(k, 1.0)
+        ref.flowSteps(k, 1.0)
+        same(gpu, ref)
+
+
+def test_one_step_plans():
+    """Above 2^21 particles a plan holds one step, by the step kernel of two particles per thread."""
+    n = 2 ** 21 + 77
+    gpu, ref = both(n, dinc_init=np.random.default_rng(1).integers(0, 4, n), dinc=np.random.default_rng(2).integers(4, 90, n),
+                    nchunk=34)
+    for k in (1, 5):
+        gpu.flowSteps(k, 1.0)
+        ref.flowSteps(k, 1.0)
+        same(gpu, ref)
