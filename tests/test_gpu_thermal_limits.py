@@ -1,6 +1,8 @@
 """Thermal forcing at the limits of its plans (csrc/fqsb_thermal.cu): the largest numbers of steps, and plans of
 few steps over many particles."""
 
+import time
+
 import numpy as np
 import pytest
 
@@ -61,3 +63,30 @@ def test_one_step_plans():
         gpu.flowSteps(k, 1.0)
         ref.flowSteps(k, 1.0)
         same(gpu, ref)
+
+
+def step_seconds(n, steps=50):
+    gpu = both_gpu(n)
+    gpu.flowSteps(steps, 1e-3)
+    best = np.inf
+    for _ in range(4):
+        t0 = time.perf_counter()
+        gpu.flowSteps(steps, 1e-3)
+        best = min(best, time.perf_counter() - t0)
+    return best / steps
+
+
+def both_gpu(n, **kw):
+    import frictionqpotspringblock_gb300 as fqsb
+
+    par = dict(m=1.0, eta=0.1, mu=1.0, k_interactions=1.0, k_frame=1.0 / n, dt=0.1, mean=0.0, stddev=0.05, seed_forcing=9,
+               dinc_init=np.random.default_rng(n).integers(0, 100, n), dinc=np.full(n, 100), shape=[n], seed=4,
+               distribution="weibull", parameters=[2.0, 1.0, 1e-5], offset=-20.0, nchunk=40)
+    par.update(kw)
+    return fqsb.Line1d.System_Cuspy_Laplace_RandomForcing(**par)
+
+
+def test_large_systems_fill_the_gpu():
+    """Four times the particles take about four times as long (one CTA per planned step: twelve times)."""
+    ratio = step_seconds(2 ** 22) / step_seconds(2 ** 20)
+    assert ratio < 6.5, ratio
