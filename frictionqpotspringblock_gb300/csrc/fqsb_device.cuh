@@ -124,7 +124,9 @@ struct Ctl {
     double *rec_u, *rec_v, *rec_a;
     double4_32a* rec_w;
     double* rec_ffsum;
-    int64_t th_commit; /* steps of the plan of thermal draws that the launch has taken */
+    /* plan of thermal draws: steps that the launch has taken, planned steps used before it, and after it (0: the next
+     * launch needs a new plan) */
+    int64_t th_commit, th_from, th_used;
 };
 
 /*

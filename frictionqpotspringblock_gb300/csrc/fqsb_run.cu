@@ -179,7 +179,8 @@ struct Strip {
  */
 template <int POT, int INTER, int MODE, bool TH>
 __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, int64_t p0, int n, int cur, double uf,
-                                              int flags, int64_t step, int64_t t, bool& pending, int64_t* moved)
+                                              int flags, int64_t step, int64_t t, int64_t th_used, bool& pending,
+                                              int64_t* moved)
 {
     /* one more addition on the integer pipes where they do not also square the residual: at N = 2^22 142 us per
      * step instead of 144 us, but 173 us instead of 169 us with the squares */
@@ -342,8 +343,8 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
         double fth = 0.0;
         if (TH && k < n) {
             /* the planned draw of step t, or the force of the step before */
-            const uint32_t draw = __ldcg(s.th_mask + t * s.th_words + (p >> 5));
-            fth = draw >> (p & 31) & 1u ? __ldcg(s.th_val + t * N + p)
+            const uint32_t draw = __ldcg(s.th_mask + (th_used + t) * s.th_words + (p >> 5));
+            fth = draw >> (p & 31) & 1u ? __ldcg(s.th_val + (th_used + t) * N + p)
                                         : __ldcg((t == 0 ? s.f_th : s.th_w[(t - 1) & 1]) + p);
             s.th_w[t & 1][p] = fth;
         }
@@ -381,11 +382,11 @@ __device__ __forceinline__ double2 strip_step(const DevSys& s, const Strip& st, 
     return sum;
 }
 
-/* Steps that a launch takes at most: those the run has left, and with thermal forcing those planned */
+/* Steps that a launch takes at most: those the run has left, and with thermal forcing those left of the plan */
 __device__ __forceinline__ int64_t steps_of_launch(const DevSys& s)
 {
     const int64_t left = s.ctl->max_steps - s.ctl->step;
-    return s.f_th && s.th_K < left ? s.th_K : left;
+    return s.f_th && s.th_K - s.ctl->th_used < left ? s.th_K - s.ctl->th_used : left;
 }
 
 /* The CTA without strips: sums and stop tests of each step, one step behind the others */
@@ -518,6 +519,11 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
         }
         vy->base = base + (unsigned long long)(t + 1) * gridDim.x;
         sc.th_commit = how == END_BARRIER ? 0 : how == END_STOPPED ? t : t + 1;
+        sc.th_from = sc.th_used;
+        sc.th_used += sc.th_commit;
+        if (sc.th_used >= s.th_K) {
+            sc.th_used = 0;
+        }
         *s.ctl = sc;
         const bool more = !sc.done && !sc.error && (sc.launch_steps == 0 || globaltimer() - sc.launch_t0 < sc.budget_ns);
         __threadfence();
@@ -557,7 +563,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
     unsigned long long base = y->base;
     const int flags = s.ctl->flags;
     const int cur0 = s.ctl->cur;
-    const int64_t step0 = s.ctl->step, left = steps_of_launch(s);
+    const int64_t step0 = s.ctl->step, left = steps_of_launch(s), th_used = TH ? s.ctl->th_used : 0;
     const double vdt = s.ctl->vdt;
     const double* sched = s.ctl->sched;
     const bool tree = MODE == KMODE_RESID || (MODE == KMODE_GENERAL && (flags & (RF_RESID | RF_FFSUM)) != 0);
@@ -601,7 +607,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
             const int64_t p0 = k * S;
             bool pending;
             const double2 sum = strip_step<POT, INTER, MODE, TH>(s, st, p0, (int)(s.N - p0 < S ? s.N - p0 : S), cur0 ^ q, uf,
-                                                             flags, step0 + t, t, pending, &moved_sh);
+                                                             flags, step0 + t, t, th_used, pending, &moved_sh);
             if (lane == 0) {
                 if (tree) {
                     s.partials[k] = sum;

@@ -9,8 +9,9 @@
  * particle order), k_th_list lists them, and k_th_eval computes one per thread from the stream's state
  * jumped ahead, so that the erfinv work (600 fp64 operations, one after the other) is dense and not in the
  * path of a step.  The run kernels then only read the drawn forces.  k_th_commit makes the steps that a
- * launch has taken the system's state (f_thermal, next, the stream); a step that the launch dropped is
- * planned again.  Per time step of 1000 particles, each redrawn every 100 steps: 46.4 us with the draws
+ * launch has taken the system's state (f_thermal, next, the stream).  A plan serves the launches of a run until it
+ * is used up: steps in which chunk windows move end a launch early (N = 65536, one in most steps: 266 us a step with
+ * a plan for every launch, 118 us).  Per time step of 1000 particles, each redrawn every 100 steps: 46.4 us with the draws
  * of each step made before it (four launches in the run graph's loop), 3.1 us planned for 256 steps and
  * taken by the one-cluster kernel.
  */
@@ -19,7 +20,7 @@
 namespace fqsb {
 
 /* The increment of the plan's first step, and in K its steps (no more than the run has left); false when the
- * run is over or takes no time steps.  Every thread reads the control block, so by plain loads that the first-level
+ * run is over or takes no time steps, or the plan that it has is not used up.  Every thread reads the control block, so by plain loads that the first-level
  * cache serves (volatile ones all go to one line of the second: 2^22 particles, k_th_mask 18 us and 202 us,
  * k_th_commit 23 us and 103 us). */
 __device__ __forceinline__ bool th_first_inc(const DevSys& s, int from, int64_t inc_arg, int64_t& inc, int& K)
@@ -29,7 +30,7 @@ __device__ __forceinline__ bool th_first_inc(const DevSys& s, int from, int64_t 
         return true;
     }
     const Ctl* c = s.ctl;
-    if (c->done || c->error || (c->flags & RF_NOINC)) {
+    if (c->done || c->error || (c->flags & RF_NOINC) || c->th_used != 0) {
         return false;
     }
     inc = c->inc + 1;
@@ -177,8 +178,9 @@ __global__ void __launch_bounds__(128) k_th_eval(const __grid_constant__ DevSys 
 __global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSys s, int what)
 {
     const Ctl* c = s.ctl;
-    int64_t steps = 1;
+    int64_t from = 0, steps = 1;
     if (what == TH_COMMIT_RUN) {
+        from = c->th_from;
         steps = c->th_commit;
     }
     else if (what == TH_COMMIT_ONE && (c->done || c->error || (c->flags & RF_NOINC))) {
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSy
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p < s.N) {
         int64_t draws = 0, last = -1;
-        for (int64_t k = 0; k < steps; ++k) {
+        for (int64_t k = from; k < from + steps; ++k) {
             if (s.th_mask[k * s.th_words + (p >> 5)] >> (p & 31) & 1u) {
                 ++draws;
                 last = k;
@@ -200,7 +202,8 @@ __global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSy
     }
     if (p == 0 && steps > 0) {
         Thermal* th = s.th;
-        th->state = pcg_advance_inc(th->state, (uint64_t)s.th_cum[steps * th_blocks(s.th_words)], th->inc);
+        const int64_t B = th_blocks(s.th_words);
+        th->state = pcg_advance_inc(th->state, (uint64_t)(s.th_cum[(from + steps) * B] - s.th_cum[from * B]), th->inc);
     }
 }
 

@@ -90,3 +90,45 @@ def test_large_systems_fill_the_gpu():
     """Four times the particles take about four times as long (one CTA per planned step: twelve times)."""
     ratio = step_seconds(2 ** 22) / step_seconds(2 ** 20)
     assert ratio < 6.5, ratio
+
+
+DRIVEN = dict(k_frame=0.5, eta=0.5, nchunk=40)
+
+
+@pytest.mark.parametrize("n", [40, 5003, 40001])
+def test_plan_outlives_window_moves(monkeypatch, n):
+    """A launch of the run kernel ends at every step in which windows move; the plan goes on behind it, over its own
+    end and from run to run."""
+    monkeypatch.setenv("FQSB_NO_SMALL", "1")
+    gpu, ref = both(n, **DRIVEN)
+    for k in (1, 254, 3, 300) if n < 10000 else (1, 120, 3):
+        gpu.flowSteps(k, 2.0)
+        ref.flowSteps(k, 2.0)
+        same(gpu, ref)
+    assert np.array_equal(gpu.chunk.start, ref.chunk.start) and np.max(ref.chunk.start) > 0
+    gpu.external.state = ref.thermal_state = 0x9E3779B97F4A7C15
+    gpu.flowSteps(20, 2.0)
+    ref.flowSteps(20, 2.0)
+    same(gpu, ref)
+
+
+def driven_seconds(s, steps=300):
+    s.flowSteps(steps, 2.0)
+    best = np.inf
+    for _ in range(3):
+        t0 = time.perf_counter()
+        s.flowSteps(steps, 2.0)
+        best = min(best, time.perf_counter() - t0)
+    return best
+
+
+def test_window_moves_plan_once():
+    """Where windows move in most steps, thermal forcing costs less than the step itself (with a plan for every launch
+    it cost one and a half steps)."""
+    import frictionqpotspringblock_gb300 as fqsb
+
+    n = 65536
+    athermal = fqsb.Line1d.System_Cuspy_Laplace(m=1.0, mu=1.0, k_interactions=1.0, dt=0.1, shape=[n], seed=4,
+                                                distribution="weibull", parameters=[2.0, 1.0, 1e-5], offset=-20.0, **DRIVEN)
+    ratio = driven_seconds(both_gpu(n, **DRIVEN)) / driven_seconds(athermal)
+    assert ratio < 2.0, ratio
