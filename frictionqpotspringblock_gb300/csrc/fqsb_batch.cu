@@ -610,13 +610,17 @@ __device__ __forceinline__ void batch_tile(const BatchDev& b, BShared& sh, doubl
                 sh.last_inst = k == (unsigned)I->n_pending - 1u;
             }
             else {
-                unsigned k = atomicAdd(&I->ticket, 1u);
-                sh.last_inst = (k == (unsigned)I->ntiles - 1u) && I->n_pending == 0;
-                if (k == (unsigned)I->ntiles - 1u && I->n_pending > 0) {
-                    I->ticket = 0; /* the redo of this realisation's pending tiles finalises */
-                    if (resident) {
-                        ((volatile BatchRun*)b.run)->stop = 1;
-                        ((volatile Inst*)I)->halt = epoch;
+                if (atomicAdd(&I->ticket, 1u) == (unsigned)I->ntiles - 1u) {
+                    /* the tiles' pending counts, written before their tickets */
+                    __threadfence();
+                    const bool pend = ((volatile Inst*)I)->n_pending > 0;
+                    sh.last_inst = !pend;
+                    if (pend) {
+                        I->ticket = 0; /* the redo of this realisation's pending tiles finalises */
+                        if (resident) {
+                            ((volatile BatchRun*)b.run)->stop = 1;
+                            ((volatile Inst*)I)->halt = epoch;
+                        }
                     }
                 }
             }
