@@ -52,7 +52,7 @@ struct RunGeom {
     int S;               /* particles per strip: 32 .. 256, a power of two */
     int threads, ctas;   /* launch shape (the last CTA is the control CTA); ctas = 0: not available */
     int64_t nstrips, node_strips, nnodes;
-    size_t smem;
+    size_t smem, smem_max; /* shared memory of a CTA; that of the longest strips */
 };
 RunGeom run_geometry(const DevSys& s);
 const void* run_kernel(const DevSys& s, int mode);

@@ -705,6 +705,13 @@ const void* run_kernel(const DevSys& s, int mode)
     }
 }
 
+static size_t run_smem(int S, int64_t warps)
+{
+    return (sizeof(double) * (3 * (size_t)S + 2) + (size_t)S) * (size_t)warps;
+}
+
+constexpr int RUN_STRIP_MAX = 256;
+
 RunGeom run_geometry(const DevSys& s)
 {
     RunGeom g = {};
@@ -722,7 +729,7 @@ RunGeom run_geometry(const DevSys& s)
     /* strips as long as they can be while a CTA's strips still occupy as many warps as possible: 32 to 256 */
     const int64_t workers = sms - 1, warps = g.threads / 32;
     g.S = 32;
-    while (g.S < 256 && (s.N + g.S - 1) / g.S > workers * warps) {
+    while (g.S < RUN_STRIP_MAX && (s.N + g.S - 1) / g.S > workers * warps) {
         g.S *= 2;
     }
     g.nstrips = (s.N + g.S - 1) / g.S;
@@ -733,7 +740,8 @@ RunGeom run_geometry(const DevSys& s)
     }
     g.nnodes = (g.nstrips + g.node_strips - 1) / g.node_strips;
     g.ctas = (int)(g.nnodes < workers ? g.nnodes : workers) + 1;
-    g.smem = (sizeof(double) * (3 * (size_t)g.S + 2) + (size_t)g.S) * (size_t)warps;
+    g.smem = run_smem(g.S, warps);
+    g.smem_max = run_smem(RUN_STRIP_MAX, warps);
     return g;
 }
 

@@ -1336,7 +1336,8 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
         kp.gridDim = dim3((unsigned)rg.ctas);
         kp.blockDim = dim3((unsigned)rg.threads);
         kp.sharedMemBytes = (unsigned)rg.smem;
-        GR(cudaFuncSetAttribute(kp.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rg.smem));
+        /* the limit is the kernel's, not this graph's: the same for every handle (another thread may be building one) */
+        GR(cudaFuncSetAttribute(kp.func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rg.smem_max));
         kp.kernelParams = argsl;
         cudaGraphNode_t nplan;
         if (s.f_th) {
