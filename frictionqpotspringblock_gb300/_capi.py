@@ -137,6 +137,7 @@ SIGNATURES = [
     ("fqsb_get_stream", _I, [_P, ctypes.POINTER(_P)]),
     ("fqsb_residual_noalloc", _I, [_P, _P, _I64, _P, _P]),
     ("fqsb_set_parameters", _I, [_P, _D, _D, _D]),
+    ("fqsb_set_wait_limit", _I, [_P, ctypes.c_uint64]),
     ("fqsb_set_random_forcing", _I, [_P, _D, _D, _U64, _PI64, _PI64]),
     ("fqsb_random_forcing_get", _I, [_P, _PU64, _PD, _PI64]),
     ("fqsb_random_forcing_set", _I, [_P, _PU64, _PD, _PI64]),

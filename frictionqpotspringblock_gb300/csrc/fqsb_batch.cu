@@ -1346,6 +1346,8 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
         I.gen = I.halt = 0;
     }
     QCU(cudaMemsetAsync(b.tile_gen, 0, sizeof(uint32_t) * (size_t)b.ntiles, h->stream));
+    /* marks left by a call whose wait ran out */
+    QCU(cudaMemsetAsync(b.tile_pending, 0, sizeof(int32_t) * (size_t)b.ntiles, h->stream));
     QCU(cudaMemcpyAsync(b.inst, inst.data(), sizeof(Inst) * inst.size(), cudaMemcpyHostToDevice, h->stream));
     BatchRun R;
     memset(&R, 0, sizeof(R));

@@ -38,6 +38,8 @@ struct fqsb_system {
     bool is2d;
     LineGeom lg;
     RunGeom rg;     /* resident run kernel (ctas = 0: none) */
+    uint64_t wait_ns;
+    int64_t n_pending_marks; /* size of DevSys::cta_pending */
     /* host mirrors of the run state */
     int cur;
     int64_t inc, qs_first, qs_last;
@@ -528,6 +530,8 @@ static int materialise_forces(fqsb_system* h)
 
 /* Device time after which a run's graph launch yields back to the host (which relaunches it). */
 static const uint64_t RUN_BUDGET_NS = 200ull * 1000ull * 1000ull;
+/* Limit on a wait of the run kernel's CTAs for one another (fqsb_set_wait_limit). */
+static const uint64_t RUN_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
 static const int64_t RING_MIN = 1024;
 
 static int ensure_graph(fqsb_system* h, int mode = KMODE_GENERAL)
@@ -663,6 +667,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     c->qs_first = h->qs_first;
     c->qs_last = h->qs_last;
     c->budget_ns = RUN_BUDGET_NS;
+    c->wait_ns = h->wait_ns;
     if (io) {
         c->sched = io->sched;
         c->rec_u = io->rec_u;
@@ -781,6 +786,13 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
         return set_err(h, FQSB_ERR_TIMEOUT, "yield search exceeded its bound (position too far from the chunk)");
     }
     if (c->error == DERR_BARRIER) {
+        /* the counters no longer agree and strips may be marked: set back, and the wells to the positions' */
+        CU(h, cudaMemsetAsync(h->d.sync, 0, sizeof(RunSync), h->stream));
+        CU(h, cudaMemsetAsync(h->d.cta_pending, 0, sizeof(int32_t) * (size_t)h->n_pending_marks, h->stream));
+        rc = align_all(h);
+        if (rc) {
+            return rc;
+        }
         return set_err(h, FQSB_ERR_TIMEOUT, "a wait of the run kernel's CTAs for one another ran out");
     }
     return FQSB_OK;
@@ -906,6 +918,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     h->graph_resid = nullptr;
     h->graph_one = nullptr;
     h->graph_np = nullptr;
+    h->wait_ns = RUN_WAIT_NS;
     h->graph_k = 0;
     {
         const char* ng = getenv("FQSB_NO_GRAPH");
@@ -998,6 +1011,7 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
         /* a RandomNormalForcing attached later takes the step kernel's own shape */
         nsteps_cta = std::max(nsteps_cta, line_geometry(N).grid);
     }
+    h->n_pending_marks = nsteps_cta;
     int64_t npart = h->is2d ? std::max(grid_reduce_ctas(N), nsteps_cta) : nsteps_cta;
     npart = std::max(npart, (int64_t)SMALL_MAX_CTAS); /* the one-cluster run kernel's CTA subtrees */
     d.npartials = npart;
@@ -2022,6 +2036,15 @@ __global__ void k_rewell(DevSys d)
         const double* y = d.data + p * d.W + d.cidx[p];
         store_well(d, p, make_wc(d, y[0], y[1]));
     }
+}
+
+extern "C" int fqsb_set_wait_limit(fqsb_system* h, uint64_t ns)
+{
+    if (!h) {
+        return FQSB_ERR_INVALID;
+    }
+    h->wait_ns = ns;
+    return FQSB_OK;
 }
 
 extern "C" int fqsb_set_parameters(fqsb_system* h, double mu, double k_interactions, double eta)

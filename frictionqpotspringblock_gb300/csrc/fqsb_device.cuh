@@ -127,6 +127,7 @@ struct Ctl {
     /* plan of thermal draws: steps that the launch has taken, planned steps used before it, and after it (0: the next
      * launch needs a new plan) */
     int64_t th_commit, th_from, th_used;
+    uint64_t wait_ns; /* limit on a wait of the run kernel's CTAs for one another */
 };
 
 /*

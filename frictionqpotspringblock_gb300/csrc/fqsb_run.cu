@@ -31,7 +31,8 @@
  * IF branch moves the windows, repeats the marked strips and finishes the step (fqsb_step.cu), and the
  * loop launches this kernel again.
  *
- * The kernel's waits are on CTAs that a cooperative launch keeps resident, and end after BARRIER_NS.
+ * The kernel's waits are on CTAs that a cooperative launch keeps resident, and end after Ctl::wait_ns (5 s).  The host
+ * then sets RunSync and the marks of pending strips back (run(), fqsb_capi.cu).
  */
 #include "fqsb_stepcore.cuh"
 
@@ -43,7 +44,6 @@ struct RunWarps {
     static constexpr int value = POT == POT_SMOOTH ? 16 : 28;
 };
 
-constexpr uint64_t BARRIER_NS = 5ull * 1000ull * 1000ull * 1000ull;
 constexpr int RUN_RING = 1024; /* StopList windows up to this length are kept in shared memory */
 
 /* Why a launch ends after step t: the run stopped after step t - 1 (step t is dropped); particles of step
@@ -57,9 +57,10 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
-/* Waits until a counter of y has reached `want`; false when the wait ran out. */
-__device__ __forceinline__ bool wait_for(RunSync* y, const unsigned long long* counter, unsigned long long want)
+/* Waits until a counter of s.sync has reached `want`; false when the wait ran out. */
+__device__ __forceinline__ bool wait_for(const DevSys& s, const unsigned long long* counter, unsigned long long want)
 {
+    RunSync* y = s.sync;
     uint64_t t0 = 0;
     for (unsigned k = 1; load_acquire(counter) < want; ++k) {
         if ((k & 255u) == 0u) {
@@ -68,7 +69,7 @@ __device__ __forceinline__ bool wait_for(RunSync* y, const unsigned long long* c
             }
             const uint64_t now = globaltimer();
             t0 = t0 == 0 ? now : t0;
-            if (now - t0 > BARRIER_NS) {
+            if (now - t0 > s.ctl->wait_ns) {
                 atomicOr(&y->failed, 1);
                 return false;
             }
@@ -79,20 +80,20 @@ __device__ __forceinline__ bool wait_for(RunSync* y, const unsigned long long* c
 
 /* Grid barrier up to `want` arrivals, for thread 0 of a CTA (the others wait at a CTA barrier on both sides);
  * false when it ran out. */
-__device__ __forceinline__ bool grid_barrier(RunSync* y, unsigned long long want)
+__device__ __forceinline__ bool grid_barrier(const DevSys& s, unsigned long long want)
 {
     __threadfence();
-    atomicAdd(&y->arrived, 1ull);
-    return wait_for(y, &y->arrived, want);
+    atomicAdd(&s.sync->arrived, 1ull);
+    return wait_for(s, &s.sync->arrived, want);
 }
 
 /* The barrier after step t; returns how the launch goes on. */
-__device__ __forceinline__ int barrier_after(RunSync* y, unsigned long long base, int64_t t, bool last)
+__device__ __forceinline__ int barrier_after(const DevSys& s, unsigned long long base, int64_t t, bool last)
 {
-    if (!grid_barrier(y, base + (unsigned long long)(t + 1) * gridDim.x)) {
+    if (!grid_barrier(s, base + (unsigned long long)(t + 1) * gridDim.x)) {
         return END_BARRIER;
     }
-    const volatile RunSync* vy = y;
+    const volatile RunSync* vy = s.sync;
     if (vy->stop[t & 1]) {
         return END_STOPPED;
     }
@@ -419,7 +420,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
     if (inter_grid(s.inter)) {
         base += gridDim.x; /* the barrier after the first positions (when it runs out, so does the first step's) */
         if (tid == 0) {
-            grid_barrier(y, base);
+            grid_barrier(s, base);
         }
     }
     __syncthreads();
@@ -475,7 +476,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
             const bool stop =
                 t > 0 && (sc.done || sc.error || (globaltimer() - sc.launch_t0) >= sc.budget_ns);
             ((volatile RunSync*)y)->stop[t & 1] = stop ? 1 : 0;
-            how_sh = barrier_after(y, base, t, t + 1 == left);
+            how_sh = barrier_after(s, base, t, t + 1 == left);
         }
         __syncthreads();
         uf = uf_t;
@@ -496,7 +497,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
         volatile RunSync* vy = y;
         const int q = (int)(t & 1);
         /* the flags below are cleared for the next launch: every CTA has to have read them after its last barrier */
-        if (how == END_BARRIER || vy->failed || !wait_for(y, &y->left, gridDim.x - 1u)) {
+        if (how == END_BARRIER || vy->failed || !wait_for(s, &y->left, gridDim.x - 1u)) {
             sc.error = DERR_BARRIER;
         }
         vy->left = 0;
@@ -518,7 +519,7 @@ static __device__ __noinline__ void run_control(const DevSys& s, const RunGeom& 
             vy->da[k] = 0;
         }
         vy->base = base + (unsigned long long)(t + 1) * gridDim.x;
-        sc.th_commit = how == END_BARRIER ? 0 : how == END_STOPPED ? t : t + 1;
+        sc.th_commit = how == END_BARRIER || how == END_STOPPED ? t : t + 1;
         sc.th_from = sc.th_used;
         sc.th_used += sc.th_commit;
         if (sc.th_used >= s.th_K) {
@@ -589,7 +590,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            grid_barrier(y, base);
+            grid_barrier(s, base);
         }
     }
     __syncthreads();
@@ -642,7 +643,7 @@ __global__ void __launch_bounds__(32 * RunWarps<POT>::value, 1)
         }
         if (threadIdx.x == 0) {
             next_sh[q] = NW;
-            how_sh = barrier_after(y, base, t, t + 1 == left);
+            how_sh = barrier_after(s, base, t, t + 1 == left);
         }
         __syncthreads();
         if (how_sh != END_NOT) {

@@ -188,6 +188,13 @@ int fqsb_set_field_device(fqsb_system* h, int field, const double* in_device);
 int fqsb_get_stream(fqsb_system* h, void** stream);
 
 /*
+ * Limit in ns on a wait of the resident kernels' thread blocks for one another (5 s by default; no counterpart in
+ * the reference).  A run whose wait runs out returns FQSB_ERR_TIMEOUT.  The handle can be used again, but its u, v and
+ * a may be of different time steps: set them, and u_frame and inc, before the next run.
+ */
+int fqsb_set_wait_limit(fqsb_system* h, uint64_t ns);
+
+/*
  * Parameters mu, k_interactions and eta of an existing system (no counterpart in the reference, whose
  * parameters are fixed at construction; needed to differentiate with respect to them).
  */
