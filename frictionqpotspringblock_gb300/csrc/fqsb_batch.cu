@@ -899,7 +899,7 @@ static unsigned batch_resident_ctas(const BatchDev& b, int threads)
     return b.ntiles > 2 * most ? 0u : (unsigned)std::min(b.ntiles, most);
 }
 
-static cudaError_t build_batch_graph(BatchDev& b, int threads, cudaGraphExec_t* exec)
+static cudaError_t build_batch_graph(BatchDev& b, int threads, bool passes, cudaGraphExec_t* exec)
 {
     cudaGraph_t g;
     cudaError_t e = cudaGraphCreate(&g, 0);
@@ -929,7 +929,7 @@ static cudaError_t build_batch_graph(BatchDev& b, int threads, cudaGraphExec_t* 
     void* a2[] = {(void*)&b, (void*)&pass2};
     void* ar[] = {(void*)&b};
     cudaGraphNode_t ns, nif, nr, nd;
-    const unsigned resident = batch_resident_ctas(b, threads);
+    const unsigned resident = passes ? 0u : batch_resident_ctas(b, threads);
     if (resident) {
         void* fr = b.ppt == 2 ? (void*)k_batch_run<2> : (void*)k_batch_run<1>;
         BG(add_kernel_node(&ns, body, nullptr, 0, fr, dim3(resident), dim3((unsigned)threads), ar));
@@ -963,12 +963,25 @@ struct fqsb_batch {
     cudaStream_t stream;
     bool own_stream;
     bool no_graph; /* FQSB_NO_GRAPH=1 at creation: passes launched one by one (for profilers) */
+    bool passes;   /* never k_batch_run: FQSB_NO_RUN=1 at creation, or its grid cannot be resident here */
     cudaGraphExec_t graph;
     std::string err;
     std::vector<void*> allocs;
 };
 
 static std::string g_batch_error;
+
+/* The graph of h for its present output pointers */
+static cudaError_t batch_graph(fqsb_batch* h)
+{
+    cudaError_t e = build_batch_graph(h->b, h->threads, h->passes, &h->graph);
+    if (e == cudaErrorCooperativeLaunchTooLarge && !h->passes) {
+        cudaGetLastError();
+        h->passes = true;
+        e = build_batch_graph(h->b, h->threads, true, &h->graph);
+    }
+    return e;
+}
 
 static int berr(fqsb_batch* h, int code, const std::string& m)
 {
@@ -1080,6 +1093,8 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
     {
         const char* ng = getenv("FQSB_NO_GRAPH");
         h->no_graph = ng && ng[0] == '1';
+        const char* nr = getenv("FQSB_NO_RUN");
+        h->passes = nr && nr[0] == '1';
     }
     h->ninst = c->n_instances;
     h->nchunk = c->nchunk;
@@ -1252,7 +1267,7 @@ extern "C" int fqsb_batch_create(const fqsb_batch_config* c, fqsb_batch** out)
         batch_free(h);
         return berr(nullptr, FQSB_ERR_CUDA, m);
     }
-    e = build_batch_graph(b, threads, &h->graph);
+    e = batch_graph(h);
     if (e != cudaSuccess) {
         std::string m = std::string("batch graph: ") + cudaGetErrorString(e);
         batch_free(h);
@@ -1330,7 +1345,7 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
     b.out_S = dS;
     b.out_inc = dI;
     /* the output pointers are kernel arguments: build the graph for this run */
-    QCU(build_batch_graph(b, h->threads, &h->graph));
+    QCU(batch_graph(h));
     /* reset every realisation's protocol state (keeps u, v, a, wells and frame positions) */
     std::vector<Inst> inst((size_t)h->ninst);
     QCU(cudaMemcpy(inst.data(), b.inst, sizeof(Inst) * inst.size(), cudaMemcpyDeviceToHost));
@@ -1397,7 +1412,16 @@ extern "C" int fqsb_batch_quasistatic(fqsb_batch* h, int64_t ncycles, double eps
     }
     else {
         for (;;) {
-            QCU(cudaGraphLaunch(h->graph, h->stream));
+            const cudaError_t le = cudaGraphLaunch(h->graph, h->stream);
+            if (le == cudaErrorCooperativeLaunchTooLarge && !h->passes) {
+                cudaGetLastError();
+                h->passes = true;
+                cudaGraphExecDestroy(h->graph);
+                h->graph = nullptr;
+                QCU(batch_graph(h));
+                continue;
+            }
+            QCU(le);
             QCU(cudaMemcpyAsync(&R, b.run, sizeof(R), cudaMemcpyDeviceToHost, h->stream));
             QCU(cudaStreamSynchronize(h->stream));
             if (R.active <= 0 || R.walk_flag || R.failed) {

@@ -534,33 +534,51 @@ static const uint64_t RUN_BUDGET_NS = 200ull * 1000ull * 1000ull;
 static const uint64_t RUN_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
 static const int64_t RING_MIN = 1024;
 
-static int ensure_graph(fqsb_system* h, int mode = KMODE_GENERAL)
+static void drop_graphs(fqsb_system* h)
+{
+    for (cudaGraphExec_t* g : {&h->graph, &h->graph_plain, &h->graph_resid, &h->graph_one, &h->graph_np}) {
+        if (*g) {
+            cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
+    }
+}
+
+/* From now on one kernel per step: where the run kernel does not pay, or its grid cannot be resident. */
+static void leave_run_kernel(fqsb_system* h)
+{
+    drop_graphs(h);
+    h->rg = RunGeom{};
+    h->lg = line_geometry(h->d.N);
+}
+
+/* The graph for runs of `mode`; without the run kernel there is the general one only (then in `mode`). */
+static int ensure_graph(fqsb_system* h, int& mode)
 {
     if (!h->use_graph) {
         h->d.in_graph = 0;
         return FQSB_OK;
     }
-    if (mode == KMODE_ONE) {
-        if (!h->graph_one) {
-            DevSys d = h->d;
-            CU(h, build_run_graph(d, h->lg, RunGeom{}, &h->graph_one));
+    for (;;) {
+        cudaGraphExec_t* g = mode == KMODE_PLAIN   ? &h->graph_plain
+                             : mode == KMODE_RESID ? &h->graph_resid
+                             : mode == KMODE_ONE   ? &h->graph_one
+                                                   : &h->graph;
+        if (*g) {
+            return FQSB_OK;
         }
-        return FQSB_OK;
-    }
-    if (mode != KMODE_GENERAL) {
-        cudaGraphExec_t* g = mode == KMODE_PLAIN ? &h->graph_plain : &h->graph_resid;
-        if (!*g) {
-            /* built from a copy: its conditional handles are its own kernels' arguments */
-            DevSys d = h->d;
-            CU(h, build_run_graph(d, h->lg, h->rg, g, mode));
+        /* built from a copy: its conditional handles are its own kernels' arguments */
+        DevSys d = h->d;
+        const cudaError_t e = build_run_graph(d, h->lg, mode == KMODE_ONE ? RunGeom{} : h->rg, g,
+                                              mode == KMODE_ONE ? KMODE_GENERAL : mode);
+        if (e != cudaErrorCooperativeLaunchTooLarge || !h->rg.ctas) {
+            CU(h, e);
+            return FQSB_OK;
         }
-        return FQSB_OK;
+        cudaGetLastError();
+        leave_run_kernel(h);
+        mode = KMODE_GENERAL;
     }
-    if (h->graph) {
-        return FQSB_OK;
-    }
-    CU(h, build_run_graph(h->d, h->lg, h->rg, &h->graph));
-    return FQSB_OK;
 }
 
 struct RunResult {
@@ -602,27 +620,7 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
         h->d.ring = nullptr;
         CU(h, cudaMalloc(&h->d.ring, sizeof(double) * (size_t)niter_tol));
         h->ring_cap = niter_tol;
-        if (h->graph) {
-            /* the ring pointer is a kernel argument of the graph */
-            cudaGraphExecDestroy(h->graph);
-            h->graph = nullptr;
-        }
-        if (h->graph_plain) {
-            cudaGraphExecDestroy(h->graph_plain);
-            h->graph_plain = nullptr;
-        }
-        if (h->graph_resid) {
-            cudaGraphExecDestroy(h->graph_resid);
-            h->graph_resid = nullptr;
-        }
-        if (h->graph_one) {
-            cudaGraphExecDestroy(h->graph_one);
-            h->graph_one = nullptr;
-        }
-        if (h->graph_np) {
-            cudaGraphExecDestroy(h->graph_np);
-            h->graph_np = nullptr;
-        }
+        drop_graphs(h); /* the ring pointer is a kernel argument */
     }
     bool use_small = np == nullptr && h->small_ok && io == nullptr && !(flags & (RF_SCHEDULE | RF_RECORD | RF_FFSUM)) &&
                      !((flags & RF_RESID) && niter_tol > SMALL_RING_MAX);
@@ -742,11 +740,23 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
             CU(h, le);
         }
         else if (h->use_graph) {
-            CU(h, cudaGraphLaunch(kmode == KMODE_PLAIN ? h->graph_plain
-                                  : kmode == KMODE_RESID ? h->graph_resid
-                                  : kmode == KMODE_ONE   ? h->graph_one
-                                                         : h->graph,
-                                  h->stream));
+            const cudaError_t le = cudaGraphLaunch(kmode == KMODE_PLAIN   ? h->graph_plain
+                                                   : kmode == KMODE_RESID ? h->graph_resid
+                                                   : kmode == KMODE_ONE   ? h->graph_one
+                                                                          : h->graph,
+                                                   h->stream);
+            if (first_launch && le == cudaErrorCooperativeLaunchTooLarge && h->rg.ctas) {
+                /* the grid cannot be resident here (nothing ran) */
+                cudaGetLastError();
+                leave_run_kernel(h);
+                kmode = KMODE_GENERAL;
+                rc = ensure_graph(h, kmode);
+                if (rc) {
+                    return rc;
+                }
+                continue;
+            }
+            CU(h, le);
         }
         else {
             for (int i = 0; i < 64; ++i) {
@@ -839,21 +849,7 @@ static void free_all(fqsb_system* h)
             cudaFree(p);
         }
     }
-    if (h->graph) {
-        cudaGraphExecDestroy(h->graph);
-    }
-    if (h->graph_plain) {
-        cudaGraphExecDestroy(h->graph_plain);
-    }
-    if (h->graph_resid) {
-        cudaGraphExecDestroy(h->graph_resid);
-    }
-    if (h->graph_one) {
-        cudaGraphExecDestroy(h->graph_one);
-    }
-    if (h->graph_np) {
-        cudaGraphExecDestroy(h->graph_np);
-    }
+    drop_graphs(h);
     if (h->h_ctl) {
         cudaFreeHost(h->h_ctl);
     }
@@ -992,7 +988,11 @@ extern "C" int fqsb_create(const fqsb_config* cfg, fqsb_system** out)
     d.f_hdt = fq_s_factor(d.hdt);
     d.f_hdt2 = fq_s_factor(d.hdt2);
     d.f_me = fq_s_factor(d.me);
-    h->rg = run_geometry(d);
+    {
+        /* 1: one kernel per step, as where the run kernel's grid cannot be resident */
+        const char* nr = getenv("FQSB_NO_RUN");
+        h->rg = nr && nr[0] == '1' ? RunGeom{} : run_geometry(d);
+    }
     h->lg = h->rg.ctas ? strip_geometry(N, h->rg.S) : line_geometry(N);
     {
         /* small Line1d / Particles systems: whole runs in one thread-block cluster */
@@ -1636,25 +1636,9 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     d.th_sc = stddev * M_SQRT2; /* the association of the reference's normal transform */
     /* the run graph's kernels take the new pointers; few planned steps are not worth a launch of the run kernel */
     if (K < 8) {
-        h->rg = RunGeom{};
-        h->lg = line_geometry(N);
+        leave_run_kernel(h);
     }
-    if (h->graph) {
-        cudaGraphExecDestroy(h->graph);
-        h->graph = nullptr;
-    }
-    if (h->graph_plain) {
-        cudaGraphExecDestroy(h->graph_plain);
-        h->graph_plain = nullptr;
-    }
-    if (h->graph_resid) {
-        cudaGraphExecDestroy(h->graph_resid);
-        h->graph_resid = nullptr;
-    }
-    if (h->graph_one) {
-        cudaGraphExecDestroy(h->graph_one);
-        h->graph_one = nullptr;
-    }
+    drop_graphs(h);
     h->small_ok = h->small_ok && (h->sg.ctas <= 8 || small_cluster_fits(d, h->sg));
     int rc = updated_inc(h); /* the constructor's refresh */
     return rc ? rc : sync(h);
@@ -2064,26 +2048,7 @@ extern "C" int fqsb_set_parameters(fqsb_system* h, double mu, double k_interacti
     /* the cached well constants of SemiSmooth depend on mu */
     k_rewell<<<blocks_for(h->d.N, 256), 256, 0, h->stream>>>(h->d);
     CU(h, cudaGetLastError());
-    if (h->graph_np) {
-        cudaGraphExecDestroy(h->graph_np);
-        h->graph_np = nullptr;
-    }
-    if (h->graph) {
-        cudaGraphExecDestroy(h->graph); /* the parameters are kernel arguments of the run graph */
-        h->graph = nullptr;
-    }
-    if (h->graph_plain) {
-        cudaGraphExecDestroy(h->graph_plain);
-        h->graph_plain = nullptr;
-    }
-    if (h->graph_resid) {
-        cudaGraphExecDestroy(h->graph_resid);
-        h->graph_resid = nullptr;
-    }
-    if (h->graph_one) {
-        cudaGraphExecDestroy(h->graph_one);
-        h->graph_one = nullptr;
-    }
+    drop_graphs(h); /* the parameters are kernel arguments */
     h->stored = false;
     return sync(h);
 }
