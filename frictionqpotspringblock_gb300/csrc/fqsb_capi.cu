@@ -1544,43 +1544,41 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
                        "interactions");
     }
     const int64_t N = d.N;
-    /* steps planned ahead: bounded by the memory of their draws (2^24 values), one at least */
-    const int64_t K = std::max((int64_t)1, std::min(TH_STEPS_MAX, ((int64_t)1 << 24) / N));
+    /* steps planned ahead: bounded by the memory of their draws (2^24 values), and by what there is; one at least */
+    int64_t K = std::max((int64_t)1, std::min(TH_STEPS_MAX, ((int64_t)1 << 24) / N));
     const int64_t words = (N + 31) / 32;
     double *f_th = nullptr, *val = nullptr, *w0 = nullptr, *w1 = nullptr;
     int64_t *next = nullptr, *di = nullptr, *cnt = nullptr, *cum = nullptr, *list = nullptr;
     uint32_t* mask = nullptr;
     Thermal* th = nullptr;
-    cudaError_t e = cudaMalloc(&f_th, sizeof(double) * (size_t)padded(N));
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&w0, sizeof(double) * (size_t)N);
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&w1, sizeof(double) * (size_t)N);
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&val, sizeof(double) * (size_t)(K * N));
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&next, sizeof(int64_t) * (size_t)N);
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&di, sizeof(int64_t) * (size_t)N);
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&cnt, sizeof(int64_t) * (size_t)(K * th_blocks(words)));
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&cum, sizeof(int64_t) * (size_t)(K * th_blocks(words) + 1));
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&list, sizeof(int64_t) * (size_t)(K * N));
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&mask, sizeof(uint32_t) * (size_t)((K + 2) * words));
-    }
-    if (e == cudaSuccess) {
-        e = cudaMalloc(&th, sizeof(Thermal));
+    cudaError_t e = cudaSuccess;
+    auto alloc = [&](auto& p, int64_t count) {
+        if (e == cudaSuccess) {
+            e = cudaMalloc((void**)&p, sizeof(*p) * (size_t)count);
+        }
+    };
+    auto release = [](auto&... p) { ((cudaFree(p), p = nullptr), ...); };
+    alloc(f_th, padded(N));
+    alloc(next, N);
+    alloc(di, N);
+    alloc(th, 1);
+    const cudaError_t e_state = e;
+    for (;; K /= 2) {
+        alloc(val, K * N);
+        alloc(list, K * N);
+        alloc(cnt, K * th_blocks(words));
+        alloc(cum, K * th_blocks(words) + 1);
+        alloc(mask, (K + 2) * words);
+        if (K >= TH_RUN_STEPS && h->rg.ctas) {
+            alloc(w0, N);
+            alloc(w1, N);
+        }
+        if (e != cudaErrorMemoryAllocation || e_state != cudaSuccess || K == 1) {
+            break;
+        }
+        cudaGetLastError();
+        e = cudaSuccess;
+        release(val, list, cnt, cum, mask, w0, w1);
     }
     if (e == cudaSuccess) {
         e = cudaMemsetAsync(mask, 0, sizeof(uint32_t) * (size_t)((K + 2) * words), h->stream);
@@ -1611,12 +1609,8 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
         e = cudaStreamSynchronize(h->stream);
     }
     if (e != cudaSuccess) {
-        for (void* q : {(void*)f_th, (void*)w0, (void*)w1, (void*)val, (void*)next, (void*)di, (void*)cnt, (void*)cum,
-                        (void*)list, (void*)mask, (void*)th}) {
-            if (q) {
-                cudaFree(q);
-            }
-        }
+        cudaGetLastError();
+        release(f_th, w0, w1, val, next, di, cnt, cum, list, mask, th);
         return set_err(h, FQSB_ERR_CUDA, std::string("RandomNormalForcing allocation failed: ") + cudaGetErrorString(e));
     }
     d.f_th = f_th;
@@ -1635,7 +1629,7 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     d.th_mean = mean;
     d.th_sc = stddev * M_SQRT2; /* the association of the reference's normal transform */
     /* the run graph's kernels take the new pointers; few planned steps are not worth a launch of the run kernel */
-    if (K < 8) {
+    if (K < TH_RUN_STEPS) {
         leave_run_kernel(h);
     }
     drop_graphs(h);

@@ -94,6 +94,7 @@ cudaError_t launch_nopass_iteration(const DevSys& s, const LineGeom& g, const No
 enum : int { TH_AT_INC = 0, TH_FROM_RUN = 1 };
 enum : int { TH_COMMIT_NOW = 0, TH_COMMIT_ONE = 1, TH_COMMIT_RUN = 2 };
 static const int64_t TH_STEPS_MAX = 256;
+static const int64_t TH_RUN_STEPS = 8; /* fewer planned steps are not worth a launch of the run kernel */
 /* blocks of 256 words of the mask: the plan counts and lists the draws of each in each step */
 __host__ __device__ inline int64_t th_blocks(int64_t words)
 {
