@@ -1074,15 +1074,34 @@ __device__ __forceinline__ double scale(double x, const Scale& sc)
     return FQ_MUL(x, sc.c);
 }
 
-/* x * c + y with two roundings, as scale() followed by an addition.  A power of two scales exactly, so one
- * fma does both (the fp64 pipe takes it in the cycles of the addition); a general c first multiplies on the
- * integer pipes. */
+/* product and sum, out of line */
+static __device__ __noinline__ double scale_add_tiny(double x, double c, double y)
+{
+    return __dadd_rn(__dmul_rn(x, c), y);
+}
+
+/*
+ * x * c + y with two roundings, for a general c x already multiplied by it.  A power of two scales exactly, so one
+ * fma does both (the fp64 pipe takes it in the cycles of the addition) -- but for a product below 2^-1022, which is
+ * rounded.  From a sum of 2^-959 on (an exponent field of 64) that makes no difference: y is then a multiple of
+ * 2^-1012, and either product is less than a quarter of that.
+ */
+__device__ __forceinline__ double add_scaled(double x, const Scale& sc, double y)
+{
+    const double r = FQ_FMA(x, sc.c_add, y);
+    if ((fq_s_hi(r) & 0x7c000000u) == 0u && sc.mode == SCALE_POW2) {
+        return scale_add_tiny(x, sc.c, y);
+    }
+    return r;
+}
+
+/* x * c + y with two roundings, as scale() followed by an addition; a general c first multiplies on the integer pipes */
 __device__ __forceinline__ double scale_add(double x, const Scale& sc, double y)
 {
     if (sc.mode == SCALE_GENERAL) {
         x = scale_other(x, sc);
     }
-    return FQ_FMA(x, sc.c_add, y);
+    return add_scaled(x, sc, y);
 }
 
 /* x + 0 (f_interactions of a system without interactions): only a -0 changes */

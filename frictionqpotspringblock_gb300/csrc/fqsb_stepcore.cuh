@@ -30,7 +30,7 @@ __device__ __forceinline__ double grid_force(const DevSys& s, double f, double u
 /*
  * The force sum of a particle without interactions and damping, f_frame + f_potential, and f_frame itself.
  * d: centre - u of a Cuspy well (the others take w).  k_frame is most often a power of two or general:
- * for a power of two f_frame is exact and one fma forms the sum (site 6; where f_frame is also needed and
+ * for a power of two f_frame is exact and one fma forms the sum (site 6, add_scaled; where f_frame is also needed and
  * latency counts, SOFT = 0, the sum is formed from it).
  */
 template <int POT, unsigned SOFT = 0u>
@@ -50,7 +50,7 @@ __device__ __forceinline__ double frame_pot(const DevSys& s, const double4_32a& 
     else {
         ff = scale(x, s.s_kf); /* read for the residual and frame-force sums only */
     }
-    return FQ_FMA(x, s.s_kf.c_add, fp);
+    return add_scaled(x, s.s_kf, fp);
 }
 
 __device__ __forceinline__ long long absll(long long x)
