@@ -569,7 +569,8 @@ static int ensure_graph(fqsb_system* h, int& mode)
         }
         /* built from a copy: its conditional handles are its own kernels' arguments */
         DevSys d = h->d;
-        const cudaError_t e = build_run_graph(d, h->lg, mode == KMODE_ONE ? RunGeom{} : h->rg, g,
+        const cudaError_t e = build_run_graph(d, mode == KMODE_ONE ? line_geometry(h->d.N) : h->lg,
+                                              mode == KMODE_ONE ? RunGeom{} : h->rg, g,
                                               mode == KMODE_ONE ? KMODE_GENERAL : mode);
         if (e != cudaErrorCooperativeLaunchTooLarge || !h->rg.ctas) {
             CU(h, e);
@@ -629,8 +630,9 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
     if (np == nullptr && h->rg.ctas && h->use_graph && !h->d.f_th && !(flags & (RF_FFSUM | RF_ACT | RF_TRUNCATE | RF_EVENT | RF_RECORD))) {
         kmode = (flags & RF_RESID) ? KMODE_RESID : KMODE_PLAIN;
     }
-    if (np == nullptr && h->rg.ctas && h->use_graph && h->is2d && max_steps == 1) {
+    if (np == nullptr && h->use_graph && max_steps == 1 && (h->d.f_th || (h->rg.ctas && h->is2d))) {
         kmode = KMODE_ONE;
+        use_small = false;
     }
     if (np) {
         if (h->use_graph && !h->graph_np) {
@@ -719,11 +721,11 @@ static int run(fqsb_system* h, int64_t max_steps, int flags, double tol, int64_t
             const int64_t launches = !h->d.f_th ? 1 : left / 16 >= h->d.th_K ? 16 : (left + h->d.th_K - 1) / h->d.th_K;
             for (int64_t k = 0; k < launches && le == cudaSuccess; ++k) {
                 if (h->d.f_th) {
-                    CU(h, launch_thermal_plan(h->d, h->d.th_K, TH_FROM_RUN, 0, h->stream));
+                    CU(h, launch_thermal_plan(h->d, std::min(h->d.th_K, left), h->stream));
                 }
                 le = launch_small_run(h->d, h->sg, h->stream);
                 if (h->d.f_th && le == cudaSuccess) {
-                    CU(h, launch_thermal_commit(h->d, TH_COMMIT_RUN, h->stream));
+                    CU(h, launch_thermal_commit(h->d, h->stream));
                 }
             }
             if (first_launch && (le == cudaErrorInvalidClusterSize || le == cudaErrorLaunchOutOfResources)) {
@@ -1501,8 +1503,7 @@ static int updated_inc(fqsb_system* h)
     if (!h->d.f_th) {
         return FQSB_OK;
     }
-    CU(h, launch_thermal_plan(h->d, 1, TH_AT_INC, h->inc, h->stream));
-    CU(h, launch_thermal_commit(h->d, TH_COMMIT_NOW, h->stream));
+    CU(h, launch_thermal_draw(h->d, h->inc, h->stream));
     if (h->stored) {
         /* f from the stored components (f_damping is -eta v in the store) and the new f_thermal */
         k_store_damp<<<blocks_for(h->d.N, 128), 128, 0, h->stream>>>(h->d, cur_v(h), h->fs[0], h->fs[1], h->fs[2],
@@ -1583,6 +1584,9 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     if (e == cudaSuccess) {
         e = cudaMemsetAsync(mask, 0, sizeof(uint32_t) * (size_t)((K + 2) * words), h->stream);
     }
+    if (e == cudaSuccess) {
+        e = cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (size_t)(K * th_blocks(words)), h->stream);
+    }
     /* prrng pcg32(seed): the PCG seeding procedure on the default stream */
     Thermal t0;
     t0.inc = (PCG_DEFAULT_STREAM << 1u) | 1u;
@@ -1590,6 +1594,7 @@ extern "C" int fqsb_set_random_forcing(fqsb_system* h, double mean, double stdde
     t0.state = t0.state * PCG_MULT + t0.inc;
     t0.state += seed;
     t0.state = t0.state * PCG_MULT + t0.inc;
+    t0.base = t0.state;
     t0.total = 0;
     t0.ticket = 0u;
     t0.pad = 0u;

@@ -132,12 +132,13 @@ struct Ctl {
 
 /*
  * RandomNormalForcing (detail.h:881-1000): the pcg32 stream all draws come from, in particle order
- * (prrng's pcg32 m_state / m_inc), and the bookkeeping of a plan of draws: their number and the ticket
- * of its counting kernel.
+ * (prrng's pcg32 m_state / m_inc), and the bookkeeping of a plan of draws: the state before them, their
+ * number and the ticket of its counting kernel.
  */
 struct Thermal {
-    uint64_t state; /* before the planned draws */
+    uint64_t state;
     uint64_t inc;
+    uint64_t base;  /* before the planned draws */
     int64_t total;  /* planned draws */
     uint32_t ticket;
     uint32_t pad;
@@ -273,7 +274,7 @@ struct DevSys {
     /* the draws of the next th_K steps (fqsb_thermal.cu); th_words = ceil(N / 32) words per step */
     int64_t th_K, th_words;
     uint32_t* th_mask;  /* [th_K + 2][th_words]: which particles draw; the last two rows stay 0 */
-    int64_t* th_cnt;    /* [th_K][th_blocks] draws of a block of particles in a step */
+    int64_t* th_cnt;    /* [th_K][th_blocks] draws of a block of particles in a step, 0 between plans */
     int64_t* th_cum;    /* [th_K * th_blocks + 1] draws before a block's of a step */
     int64_t* th_list;   /* the draws in order: step * N + particle (capacity th_K * N) */
     double* th_val;     /* [th_K][N] the drawn forces */

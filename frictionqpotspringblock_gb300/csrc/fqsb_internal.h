@@ -40,7 +40,8 @@ int64_t step_ctas(const DevSys& s, const LineGeom& g);
  * frame-force sums or recording (timeSteps / flowSteps), and runs with the residual only (minimise) -- with
  * the other code compiled out.  KMODE_ONE: runs of one step on a grid, by tiles (k_step_grid2): the run kernel's pass
  * for the first positions is not worth one step (N = 4194304, a call of timeStep: 192 us by tiles, 334 us with the first
- * step's positions recomputed where they are read). */
+ * step's positions recomputed where they are read).  And of thermal systems, whose plan and commit are not (N = 1000, a
+ * call of timeStep: 72 us in the one-cluster kernel, 66 us so). */
 enum : int { KMODE_GENERAL = 0, KMODE_PLAIN = 1, KMODE_RESID = 2, KMODE_ONE = 3 };
 struct RunGeom;
 cudaError_t build_run_graph(DevSys& s, const LineGeom& g, const RunGeom& rg, cudaGraphExec_t* exec,
@@ -86,13 +87,11 @@ cudaError_t build_nopass_graph(const DevSys& s, const LineGeom& g, const NopassA
 cudaError_t launch_nopass_iteration(const DevSys& s, const LineGeom& g, const NopassArgs& A, cudaStream_t st);
 
 /*
- * RandomNormalForcing (fqsb_thermal.cu).  A plan holds the draws of the next K steps, the first at the step a run
- * is about to make (TH_FROM_RUN) or at increment `inc` (TH_AT_INC); it changes nothing of the system's state.
- * Committing its first steps (all of a one-step plan; those that the launch has taken, Ctl::th_commit) updates
- * f_thermal, the next increments and the stream.
+ * RandomNormalForcing (fqsb_thermal.cu).  A plan holds the draws of the next K steps of a run; it changes nothing of
+ * the system's state.  Committing the steps of it that a launch has taken (Ctl::th_commit) updates f_thermal, the next
+ * increments and the stream.  The draws of one step, or at an increment, do that at once.
  */
 enum : int { TH_AT_INC = 0, TH_FROM_RUN = 1 };
-enum : int { TH_COMMIT_NOW = 0, TH_COMMIT_ONE = 1, TH_COMMIT_RUN = 2 };
 static const int64_t TH_STEPS_MAX = 256;
 static const int64_t TH_RUN_STEPS = 8; /* fewer planned steps are not worth a launch of the run kernel */
 /* blocks of 256 words of the mask: the plan counts and lists the draws of each in each step */
@@ -100,12 +99,14 @@ __host__ __device__ inline int64_t th_blocks(int64_t words)
 {
     return (words + 255) / 256;
 }
-cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, int from, int64_t inc, cudaStream_t st);
-cudaError_t launch_thermal_commit(const DevSys& s, int what, cudaStream_t st);
-/* the same as nodes of a graph: the plan first in `body` (its last node in *node), the commit after *dep */
+cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, cudaStream_t st);
+cudaError_t launch_thermal_commit(const DevSys& s, cudaStream_t st);
+cudaError_t launch_thermal_step(const DevSys& s, cudaStream_t st);
+cudaError_t launch_thermal_draw(const DevSys& s, int64_t inc, cudaStream_t st);
+/* the same as nodes of a graph: plan and step first in `body` (the last node in *node), the commit after *dep */
 cudaError_t add_thermal_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K);
-cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s,
-                               int what);
+cudaError_t add_thermal_step(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s);
+cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s);
 
 /* One loop iteration launched kernel by kernel by the host (s.in_graph must be 0). */
 cudaError_t launch_iteration(const DevSys& s, const LineGeom& g, cudaStream_t st);

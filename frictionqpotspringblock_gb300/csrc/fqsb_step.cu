@@ -1244,10 +1244,7 @@ cudaError_t launch_iteration(const DevSys& s, const LineGeom& g0, cudaStream_t s
     void* argsr[] = {(void*)&s};
     cudaError_t e = cudaSuccess;
     if (s.f_th) {
-        e = launch_thermal_plan(s, 1, TH_FROM_RUN, 0, st);
-        if (e == cudaSuccess) {
-            e = launch_thermal_commit(s, TH_COMMIT_ONE, st);
-        }
+        e = launch_thermal_step(s, st);
     }
     if (e == cudaSuccess && s.inter == INTER_LONGRANGE1D) {
         e = cudaLaunchKernel((void*)k_lr_position, dim3((unsigned)((s.N + 255) / 256)), dim3(256), argsr, 0, st);
@@ -1317,8 +1314,7 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
     if (s.f_th && !rg.ctas) {
         /* updated_inc of the step: thermal draws before the step's forces */
         cudaGraphNode_t ndraw;
-        GR(add_thermal_plan(&ndraw, body, s, 1));
-        GR(add_thermal_commit(&ndraw, body, &ndraw, s, TH_COMMIT_ONE));
+        GR(add_thermal_step(&ndraw, body, s));
         GR(add_kernel(&nstep, body, &ndraw, 1, fstep, grid, block, args1));
     }
     else if (s.inter == INTER_LONGRANGE1D) {
@@ -1349,7 +1345,7 @@ cudaError_t build_run_graph(DevSys& s, const LineGeom& g0, const RunGeom& rg, cu
         coop.cooperative = 1;
         GR(cudaGraphKernelNodeSetAttribute(nstep, cudaLaunchAttributeCooperative, &coop));
         if (s.f_th) {
-            GR(add_thermal_commit(&nstep, body, &nstep, s, TH_COMMIT_RUN));
+            GR(add_thermal_commit(&nstep, body, &nstep, s));
         }
     }
     else {

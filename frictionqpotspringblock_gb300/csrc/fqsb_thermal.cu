@@ -61,10 +61,10 @@ __global__ void __launch_bounds__(256) k_th_mask(const __grid_constant__ DevSys 
     }
 }
 
-/* Exclusive prefix of x over the CTA's 256 threads (8 warps); *total gets the CTA's sum. */
-__device__ __forceinline__ int64_t cta_exclusive_scan256(int64_t x, int64_t* sh8, int64_t* total)
+/* Exclusive prefix of x over the CTA's threads (whole warps); *total gets the CTA's sum.  sh: a word per warp. */
+__device__ __forceinline__ int64_t cta_exclusive_scan(int64_t x, int64_t* sh, int64_t* total)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     int64_t incl = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -74,13 +74,12 @@ __device__ __forceinline__ int64_t cta_exclusive_scan256(int64_t x, int64_t* sh8
         }
     }
     if (lane == 31) {
-        sh8[warp] = incl;
+        sh[warp] = incl;
     }
     __syncthreads();
     int64_t before = 0, all = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        int64_t t = sh8[w];
+    for (int w = 0; w < warps; ++w) {
+        int64_t t = sh[w];
         before += w < warp ? t : 0;
         all += t;
     }
@@ -107,7 +106,7 @@ __global__ void __launch_bounds__(256) k_th_count(const __grid_constant__ DevSys
     if ((int)blockIdx.y < K && w < s.th_words) {
         n = __popc(s.th_mask[(int64_t)blockIdx.y * s.th_words + w]);
     }
-    cta_exclusive_scan256(n, sh8, &total);
+    cta_exclusive_scan(n, sh8, &total);
     if (threadIdx.x == 0) {
         s.th_cnt[blockIdx.y * B + blockIdx.x] = total;
         __threadfence();
@@ -124,15 +123,69 @@ __global__ void __launch_bounds__(256) k_th_count(const __grid_constant__ DevSys
     for (int64_t i = i0; i < i1; ++i) {
         x += __ldcg(s.th_cnt + i);
     }
-    int64_t before = cta_exclusive_scan256(x, sh8, &total);
+    int64_t before = cta_exclusive_scan(x, sh8, &total);
     for (int64_t i = i0; i < i1; ++i) {
         s.th_cum[i] = before;
         before += __ldcg(s.th_cnt + i);
+        s.th_cnt[i] = 0;
     }
     if (threadIdx.x == 0) {
         s.th_cum[M] = total;
         s.th->total = total;
         s.th->ticket = 0u;
+        s.th->base = s.th->state;
+    }
+}
+
+/*
+ * One step, whose draws k_th_eval makes the system's state: marked, counted by blocks and numbered in one kernel (the
+ * last CTA to finish; the stream moves on).
+ */
+__global__ void __launch_bounds__(1024) k_th_one(const __grid_constant__ DevSys s, int from, int64_t inc_arg)
+{
+    __shared__ int64_t sh[32];
+    __shared__ int sh_last;
+    int64_t inc;
+    int K = 1;
+    if (!th_first_inc(s, from, inc_arg, inc, K)) {
+        return;
+    }
+    const int64_t T = blockDim.x, B = th_blocks(s.th_words), p = (int64_t)blockIdx.x * T + threadIdx.x;
+    const bool draw = p < s.N && inc >= s.th_next[p];
+    const unsigned word = __ballot_sync(0xffffffffu, draw);
+    if ((threadIdx.x & 31) == 0 && p < s.N) {
+        s.th_mask[p >> 5] = word;
+    }
+    const int n = __syncthreads_count(draw);
+    if (threadIdx.x == 0) {
+        if (n) {
+            atomicAdd((unsigned long long*)s.th_cnt + (p >> 13), (unsigned long long)n);
+            __threadfence();
+        }
+        sh_last = atomicAdd(&s.th->ticket, 1u) == gridDim.x - 1u ? 1 : 0;
+    }
+    __syncthreads();
+    if (!sh_last) {
+        return;
+    }
+    __threadfence();
+    const int64_t per = (B + T - 1) / T, i0 = threadIdx.x * per, i1 = i0 + per < B ? i0 + per : B;
+    int64_t x = 0, total;
+    for (int64_t i = i0; i < i1; ++i) {
+        x += __ldcg(s.th_cnt + i);
+    }
+    int64_t before = cta_exclusive_scan(x, sh, &total);
+    for (int64_t i = i0; i < i1; ++i) {
+        s.th_cum[i] = before;
+        before += __ldcg(s.th_cnt + i);
+        s.th_cnt[i] = 0;
+    }
+    if (threadIdx.x == 0) {
+        Thermal* th = s.th;
+        th->total = total;
+        th->ticket = 0u;
+        th->base = th->state;
+        th->state = pcg_advance_inc(th->state, (uint64_t)total, th->inc);
     }
 }
 
@@ -150,15 +203,15 @@ __global__ void __launch_bounds__(256) k_th_list(const __grid_constant__ DevSys 
     const int64_t w = (int64_t)blockIdx.x * 256 + threadIdx.x;
     uint32_t word = w < s.th_words ? s.th_mask[(int64_t)blockIdx.y * s.th_words + w] : 0u;
     int64_t total;
-    int64_t k = cta_exclusive_scan256(__popc(word), sh8, &total);
+    int64_t k = cta_exclusive_scan(__popc(word), sh8, &total);
     k += s.th_cum[(int64_t)blockIdx.y * gridDim.x + blockIdx.x];
     for (; word; word &= word - 1u) {
         s.th_list[k++] = (int64_t)blockIdx.y * s.N + 32 * w + (__ffs((int)word) - 1);
     }
 }
 
-/* One thread per draw: entry k of the list takes output k of the stream. */
-__global__ void __launch_bounds__(128) k_th_eval(const __grid_constant__ DevSys s, int from, int64_t inc_arg)
+/* One thread per draw: entry k of the list takes output k of the stream.  now: the draws are the system's state. */
+__global__ void __launch_bounds__(128) k_th_eval(const __grid_constant__ DevSys s, int from, int64_t inc_arg, int now)
 {
     int64_t inc;
     int K = 0;
@@ -166,26 +219,26 @@ __global__ void __launch_bounds__(128) k_th_eval(const __grid_constant__ DevSys 
         return;
     }
     const int64_t total = s.th->total;
-    const uint64_t state = s.th->state, sinc = s.th->inc;
+    const uint64_t base = s.th->base, sinc = s.th->inc;
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t u32 = pcg_output(pcg_advance_inc(state, (uint64_t)k, sinc));
+        const uint32_t u32 = pcg_output(pcg_advance_inc(base, (uint64_t)k, sinc));
         const double r = FQ_MUL((double)u32, 0x1p-32);
         const double z = fq_erfinv(FQ_SUB(FQ_MUL(2.0, r), 1.0));
-        s.th_val[s.th_list[k]] = FQ_ADD(s.th_mean, FQ_MUL(s.th_sc, z));
+        const double f = FQ_ADD(s.th_mean, FQ_MUL(s.th_sc, z));
+        const int64_t e = s.th_list[k]; /* now: of step 0, the particle */
+        if (now) {
+            s.f_th[e] = f;
+            s.th_next[e] += s.th_dinc[e];
+        }
+        else {
+            s.th_val[e] = f;
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSys s, int what)
+__global__ void __launch_bounds__(256) k_th_commit(const __grid_constant__ DevSys s)
 {
-    const Ctl* c = s.ctl;
-    int64_t from = 0, steps = 1;
-    if (what == TH_COMMIT_RUN) {
-        from = c->th_from;
-        steps = c->th_commit;
-    }
-    else if (what == TH_COMMIT_ONE && (c->done || c->error || (c->flags & RF_NOINC))) {
-        steps = 0;
-    }
+    const int64_t from = s.ctl->th_from, steps = s.ctl->th_commit;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p < s.N) {
         int64_t draws = 0, last = -1;
@@ -217,18 +270,22 @@ struct ThLaunch {
 };
 
 template <class F>
-static cudaError_t for_plan(const DevSys& s, int64_t K, int from, int64_t inc, F launch)
+static cudaError_t for_plan(const DevSys& s, int64_t K, int from, int64_t inc, int now, F launch)
 {
     int k = (int)K;
     void* args[] = {(void*)&s, (void*)&k, (void*)&from, (void*)&inc};
-    void* args_eval[] = {(void*)&s, (void*)&from, (void*)&inc};
-    const dim3 parts((unsigned)((s.N + 255) / 256)), blocks((unsigned)th_blocks(s.th_words), (unsigned)K);
-    const ThLaunch all[4] = {{(void*)k_th_mask, parts, dim3(256), args},
-                             {(void*)k_th_count, blocks, dim3(256), args},
-                             {(void*)k_th_list, blocks, dim3(256), args},
-                             {(void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), args_eval}};
-    for (const ThLaunch& l : all) {
-        const cudaError_t e = launch(l);
+    void* args_one[] = {(void*)&s, (void*)&from, (void*)&inc};
+    void* args_eval[] = {(void*)&s, (void*)&from, (void*)&inc, (void*)&now};
+    /* one step: few CTAs where their tickets would count */
+    const unsigned T = now && s.N > (1 << 18) ? 1024u : 256u;
+    const dim3 parts((unsigned)((s.N + T - 1) / T)), blocks((unsigned)th_blocks(s.th_words), (unsigned)K);
+    const ThLaunch list = {(void*)k_th_list, blocks, dim3(256), args};
+    const ThLaunch eval = {(void*)k_th_eval, dim3(TH_EVAL_CTAS), dim3(128), args_eval};
+    const ThLaunch step[] = {{(void*)k_th_one, parts, dim3(T), args_one}, list, eval};
+    const ThLaunch plan[] = {{(void*)k_th_mask, parts, dim3(T), args}, {(void*)k_th_count, blocks, dim3(256), args}, list, eval};
+    const ThLaunch *l = now ? step : plan, *end = now ? step + 3 : plan + 4;
+    for (; l != end; ++l) {
+        const cudaError_t e = launch(*l);
         if (e != cudaSuccess) {
             return e;
         }
@@ -236,14 +293,30 @@ static cudaError_t for_plan(const DevSys& s, int64_t K, int from, int64_t inc, F
     return cudaSuccess;
 }
 
-cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, int from, int64_t inc, cudaStream_t st)
+static cudaError_t launch_plan(const DevSys& s, int64_t K, int from, int64_t inc, int now, cudaStream_t st)
 {
-    return for_plan(s, K, from, inc, [&](const ThLaunch& l) { return cudaLaunchKernel(l.f, l.grid, l.block, l.args, 0, st); });
+    return for_plan(s, K, from, inc, now,
+                    [&](const ThLaunch& l) { return cudaLaunchKernel(l.f, l.grid, l.block, l.args, 0, st); });
 }
 
-cudaError_t launch_thermal_commit(const DevSys& s, int what, cudaStream_t st)
+cudaError_t launch_thermal_plan(const DevSys& s, int64_t K, cudaStream_t st)
 {
-    k_th_commit<<<(unsigned)((s.N + 255) / 256), 256, 0, st>>>(s, what);
+    return launch_plan(s, K, TH_FROM_RUN, 0, 0, st);
+}
+
+cudaError_t launch_thermal_step(const DevSys& s, cudaStream_t st)
+{
+    return launch_plan(s, 1, TH_FROM_RUN, 0, 1, st);
+}
+
+cudaError_t launch_thermal_draw(const DevSys& s, int64_t inc, cudaStream_t st)
+{
+    return launch_plan(s, 1, TH_AT_INC, inc, 1, st);
+}
+
+cudaError_t launch_thermal_commit(const DevSys& s, cudaStream_t st)
+{
+    k_th_commit<<<(unsigned)((s.N + 255) / 256), 256, 0, st>>>(s);
     return cudaGetLastError();
 }
 
@@ -260,20 +333,29 @@ static cudaError_t add_node(cudaGraphNode_t* node, cudaGraph_t body, const cudaG
     return e;
 }
 
-cudaError_t add_thermal_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K)
+static cudaError_t add_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K, int now)
 {
     bool first = true;
-    return for_plan(s, K, TH_FROM_RUN, 0, [&](const ThLaunch& l) {
+    return for_plan(s, K, TH_FROM_RUN, 0, now, [&](const ThLaunch& l) {
         const cudaError_t e = add_node(node, body, first ? nullptr : node, l);
         first = false;
         return e;
     });
 }
 
-cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s,
-                               int what)
+cudaError_t add_thermal_plan(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s, int64_t K)
 {
-    void* args[] = {(void*)&s, (void*)&what};
+    return add_plan(node, body, s, K, 0);
+}
+
+cudaError_t add_thermal_step(cudaGraphNode_t* node, cudaGraph_t body, const DevSys& s)
+{
+    return add_plan(node, body, s, 1, 1);
+}
+
+cudaError_t add_thermal_commit(cudaGraphNode_t* node, cudaGraph_t body, const cudaGraphNode_t* dep, const DevSys& s)
+{
+    void* args[] = {(void*)&s};
     return add_node(node, body, dep, {(void*)k_th_commit, dim3((unsigned)((s.N + 255) / 256)), dim3(256), args});
 }
 
