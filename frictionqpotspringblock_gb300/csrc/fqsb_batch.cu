@@ -695,10 +695,8 @@ constexpr uint64_t BATCH_WAIT_NS = 5ull * 1000ull * 1000ull * 1000ull;
 /*
  * Many phase steps of every realisation in one cooperative launch, until windows must move, all realisations are
  * finished or the launch's time is up.  (A pass of k_batch per phase step pays the graph loop's iteration, a launch
- * and the grid's ticket: 23 us a step with 10276 particles, 12 us here.)  CTA c owns the tiles c, c + gridDim, ... and takes whichever of them is
- * ready: a tile takes its next phase step when its realisation has finished the one before (Inst::gen).  So no
- * realisation waits for another one, and where a CTA has several tiles the end of one realisation's step
- * (tickets, residual, stop test) passes beside the step of another.
+ * and the grid's ticket: 23 us a step with 10276 particles, 12 us here.)  A CTA per tile, which takes its next phase
+ * step when its realisation has finished the one before (Inst::gen): no realisation waits for another one.
  * A tile whose windows must move ends the launch (BatchRun::stop): its realisation stays unfinished for the
  * redo, the others halt after the phase step they are in.  The waits are on resident CTAs and end after BATCH_WAIT_NS.
  */
@@ -710,60 +708,45 @@ __global__ void __launch_bounds__(256, 4) k_batch_run(const __grid_constant__ Ba
     volatile BatchRun* R = b.run;
     const uint32_t epoch = R->epoch;
     const uint64_t t_end = gtimer() + R->budget_ns;
-    const int own = (int)((b.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x); /* tiles of this CTA */
-    int first = 0; /* the one looked at first */
+    const int64_t t = blockIdx.x;
+    const volatile Inst* I = b.inst + b.tile_inst[t];
+    uint32_t gen = b.tile_gen[t]; /* phase steps that this tile has taken */
     for (;;) {
         __syncthreads();
-        if (threadIdx.x < 32) {
-            /* the next ready tile, 32 of them looked at together, or none: all are finished or halted */
-            const int lane = threadIdx.x;
-            int take = -1;
+        if (threadIdx.x == 0) {
+            /* until the realisation has finished the step before (1), or is finished or halted (0) */
+            int take = 0;
             uint64_t t0 = 0;
-            for (unsigned i = 1; take < 0; ++i) {
-                bool waiting = false;
-                for (int m0 = 0; m0 < own && take < 0; m0 += 32) {
-                    int m = first + m0 + lane;
-                    m = m >= own ? m - own : m;
-                    const bool in = m0 + lane < own;
-                    const int64_t t = blockIdx.x + (int64_t)(in ? m : 0) * gridDim.x;
-                    const volatile Inst* I = b.inst + b.tile_inst[t];
-                    const uint32_t gen = I->gen;
-                    __threadfence();
-                    const bool alive = in && I->halt != epoch && I->phase != PH_DONE;
-                    const bool ready = alive && gen == b.tile_gen[t];
-                    const unsigned r = __ballot_sync(0xffffffffu, ready);
-                    waiting = waiting || __any_sync(0xffffffffu, alive);
-                    if (r) {
-                        const int src = __ffs(r) - 1;
-                        if (lane == src) {
-                            b.tile_gen[t] = gen + 1u;
-                        }
-                        const int mt = __shfl_sync(0xffffffffu, m, src);
-                        take = (int)(blockIdx.x + (int64_t)mt * gridDim.x);
-                        first = mt + 1 < own ? mt + 1 : 0;
-                    }
+            for (unsigned i = 1;; ++i) {
+                const uint32_t finished = I->gen;
+                __threadfence();
+                if (I->halt == epoch || I->phase == PH_DONE) {
+                    break;
                 }
-                if (take >= 0 || !waiting) {
+                if (finished == gen) {
+                    take = 1;
                     break;
                 }
                 if ((i & 255u) == 0u) {
                     const uint64_t now = gtimer();
                     t0 = t0 == 0 ? now : t0;
-                    if (__any_sync(0xffffffffu, R->failed || now - t0 > BATCH_WAIT_NS)) {
+                    if (R->failed || now - t0 > BATCH_WAIT_NS) {
                         R->failed = 1;
                         break;
                     }
                 }
             }
-            if (lane == 0) {
-                sh.tile = take;
-            }
+            sh.tile = take;
         }
         __syncthreads();
-        if (sh.tile < 0) {
+        if (!sh.tile) {
             break;
         }
-        batch_tile<PPT>(b, sh, sh_un, sh.tile, 0, true, epoch, t_end);
+        ++gen;
+        batch_tile<PPT>(b, sh, sh_un, t, 0, true, epoch, t_end);
+    }
+    if (threadIdx.x == 0) {
+        b.tile_gen[t] = gen;
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -879,10 +862,11 @@ static cudaError_t add_cond(cudaGraphNode_t* node, cudaGraph_t graph, const cuda
 }
 
 /*
- * CTAs of k_batch_run: as many as can be resident together; 0: a pass of k_batch per iteration of the graph's loop
- * instead, where a CTA would own more than two tiles.  A pass has 17 us of fixed cost, k_batch_run 4, but there
- * each tile pays for being looked for.  One quasistatic cycle by tiles of 128 x 2, passes and k_batch_run: 10276
- * particles 85 and 55 ms, 253727 117 and 93, 671087 (two to three tiles per CTA) 201 and 213, 2761199 616 and 830.
+ * CTAs of k_batch_run, one per tile; 0: a pass of k_batch per iteration of the graph's loop instead, where they cannot
+ * all be resident together.  A pass has 17 us of fixed cost, k_batch_run 4.  One quasistatic cycle by tiles of 128 x 2,
+ * 1216 of them resident, passes and k_batch_run, ms: 819 tiles 121 and 83, 949 126 and 98, 1203 135 and 93.  (CTAs that
+ * own up to two tiles and look for a ready one lost to the passes: 1292 tiles 157 and 197, 1541 168 and 193, 2103 194 and
+ * 202.)
  */
 static unsigned batch_resident_ctas(const BatchDev& b, int threads)
 {
@@ -896,7 +880,7 @@ static unsigned batch_resident_ctas(const BatchDev& b, int threads)
         return 0;
     }
     const int64_t most = (int64_t)per * sms;
-    return b.ntiles > 2 * most ? 0u : (unsigned)std::min(b.ntiles, most);
+    return b.ntiles > most ? 0u : (unsigned)b.ntiles;
 }
 
 static cudaError_t build_batch_graph(BatchDev& b, int threads, bool passes, cudaGraphExec_t* exec)
