@@ -64,7 +64,7 @@ FP64_OPS_PER_PARTICLE_STEP = 24  # binary64 add/mul of the exact-order step; com
 # of those, the run kernel's flow steps issue these on the fp64 pipe; the rest (the 8 multiplications and 6 additions) run
 # bit-identically on the integer pipes (csrc/fq_soft64.h)
 FP64_PIPE_OPS_PER_PARTICLE_STEP = 10
-STEP_PROFILE = ROOT / "profiles" / "k_step_line_cuspy_laplace1d_N4M.md"
+STEP_PROFILE = ROOT / "profiles" / "k_run_line_N4M.md"
 FORMS = ("small_system", "line2d", "batched", "adjoint", "next_rows")
 
 
@@ -705,7 +705,7 @@ def main():
                "sample": f"oracle (reference restated in C, loop per statement, libm, sequential sums), "
                          f"N=65536 ring of the same parameters, flowSteps(3000), {secs:.1f} s on 1 core"}
     figs = profile_figures()
-    traffic = figs["traffic_bytes_per_launch"] / figs["traffic_particles"] * N
+    traffic = figs["traffic_bytes_per_step"] / figs["traffic_particles"] * N
     fp64_gops = FP64_OPS_PER_PARTICLE_STEP * N / kernel_s / 1e9
     fp64_pipe_gops = FP64_PIPE_OPS_PER_PARTICLE_STEP * N / kernel_s / 1e9
     peak_gops = fp64_peak if isinstance(fp64_peak, float) else None
@@ -730,7 +730,7 @@ def main():
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                      "frac": achieved_gbs / hbm_peak, "traffic": traffic,
-                     "traffic_unit": "bytes per time step (ncu capture of the one-kernel-per-step form, " + STEP_PROFILE.name +
+                     "traffic_unit": "bytes per time step (ncu capture, " + STEP_PROFILE.name +
                                      ", scaled by N)",
                      "peak_kind": peak_kind, "algorithmic_bytes_per_particle_step": BYTES_PER_PARTICLE_STEP,
                      "kernel": "k_run_line<Cuspy, Laplace1d>, per time step", "kernel_us": kernel_s * 1e6},

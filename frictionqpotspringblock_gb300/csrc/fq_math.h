@@ -240,8 +240,9 @@ __device__ static const double fq_log_tab_dev[FQ_LOG_N][4] = FQ_LOG_TABLE_INIT;
 static const double fq_log_tab_host[FQ_LOG_N][4] = FQ_LOG_TABLE_INIT;
 
 /*
- * Quick phases.  log and sin below first compute a double-double hi + lo of a known relative error in a
- * fraction of the operations of the full evaluation, and round it when every value within that error
+ * Quick phases.  log and sin below first compute a double-double hi + lo of a relative error below a bound (checked
+ * against the full evaluation, over all arguments of a yield distance and 10^10 sines) in a
+ * fraction of the operations of the full evaluation, and round it when every value within that bound
  * rounds alike (Ziv, "Fast evaluation of elementary mathematical functions with correctly rounded last
  * bit", 1991); else they evaluate in full.  The bounds cover the full evaluation's own error as well, so where
  * the quick phase rounds, it rounds to the same double.

@@ -5,9 +5,9 @@
  * Why.  With one kernel per time step inside the run graph's WHILE loop every step pays the loop's
  * iteration, the launch, each CTA's read of the run state and its ticket: 13 us at N = 1024, 18 us at
  * N = 2^22.  Here the CTAs (one per SM) stay, and a grid barrier (2 us with the start of the next step)
- * separates the steps.  Measured per step, one kernel per step and this kernel: N = 65536 16.6 and 6.1 us,
- * 2^20 50 and 37 us, 2^22 177 and 144 us (minimise 206 and 169 us).  It is then bound by the fp64 and the
- * ALU pipe together (60% of their practical rates each) and by how well the warps' phases interleave.
+ * separates the steps.  Measured per step, one kernel per step and this kernel: N = 65536 17.3 and 6.6 us,
+ * 2^20 50 and 37 us, 2^22 177 and 136 us (minimise 221 and 161 us).  It is then bound by the fp64 and the
+ * ALU pipe together (61% and 64% of their practical rates) and by how well the warps' phases interleave.
  *
  * Work split.  The ring is cut into strips of 32 to 256 consecutive particles; each warp takes whole
  * strips and needs no barrier with the others inside a step (in the one-kernel-per-step form the warps

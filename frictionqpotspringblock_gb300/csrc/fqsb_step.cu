@@ -12,7 +12,10 @@
  * bookkeeping (:1768-1778, :1855-1866).
  *
  * Run loop.  A run (timeSteps, flowSteps, minimise, minimise_truncate, timeStepsUntilEvent) is one
- * CUDA graph: a conditional WHILE node whose body is one step.  The last CTA to finish a step
+ * CUDA graph: a conditional WHILE node whose body is many steps of the resident run kernel
+ * (fqsb_run.cu), or one step of the kernels here: QuarticGradient2d, LongRange1d, single steps of grids
+ * and of thermal systems, thermal systems of more than 2^21 particles, and GPUs on which the run kernel's grid
+ * does not fit.  The last CTA to finish a step
  * evaluates the stop tests and sets the loop condition (cudaGraphSetConditional), so the host
  * launches the graph once and synchronises once.  A launch also yields after a device-time budget
  * (%globaltimer), so the host regains control every ~0.2 s of a long run.
@@ -20,9 +23,9 @@
  * Chunk windows.  The step kernels only search a particle's current chunk window (a few loads).
  * When the new well lies outside the window's margins the window must move and be regenerated from
  * the particle's pcg32 stream (heavy code: distribution transforms).  That code is kept out of the
- * step kernels (it would raise them to 128 registers and cost ~12% throughput); instead the CTA is
- * marked pending, a conditional IF branch of the same graph iteration regenerates the marked
- * particles' windows (k_regen) and re-runs the marked CTAs (redo pass).  The step is a pure function
+ * step kernels (it would raise them to 128 registers and cost ~12% throughput); instead the CTA (or the
+ * run kernel's strip) is marked pending, a conditional IF branch of the same graph iteration regenerates the marked
+ * particles' windows (k_regen) and repeats the marked CTAs or strips (redo pass).  The step is a pure function
  * of the old state, so the redo reproduces exactly the reference's step.
  *
  * State is double buffered (u, v, a)[cur] -> (u, v, a)[cur ^ 1].  Arithmetic uses explicit
