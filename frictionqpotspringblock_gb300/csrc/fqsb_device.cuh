@@ -565,7 +565,8 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
     int64_t start = s.start[p];
     const int64_t li0 = s.cidx[p];
     int64_t li = li0;
-    int64_t gi;
+    int64_t gi = 0; /* global index of u's well (of either sign) */
+    enum { INSIDE, ABOVE, BELOW } where = INSIDE;
     int kind;
     int64_t ko;
     uint64_t sto;
@@ -593,16 +594,13 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
         }
         gi = start + li;
     }
-    else if (u >= y[W - 1]) {
-        gi = -1; /* found below */
-    }
     else {
-        gi = -2;
+        where = u >= y[W - 1] ? ABOVE : BELOW;
     }
 
     int64_t end = start + W - 1;
     bool fast = end >= ko; /* the forward walker is exact from the window end */
-    if (gi == -1) {
+    if (where == ABOVE) {
         if (fast) {
             Walker w;
             w.k = end;
@@ -646,7 +644,7 @@ static __device__ __noinline__ bool dev_align(const DevSys& s, int64_t p, double
             }
         }
     }
-    else if (gi == -2) {
+    else if (where == BELOW) {
         int64_t k = start; /* y_k > u */
         for (int64_t it = 0;; ++it) {
             if (it * 64 >= MAX_WALK) {
