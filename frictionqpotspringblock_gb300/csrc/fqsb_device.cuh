@@ -1088,7 +1088,7 @@ static __device__ __noinline__ double scale_add_tiny(double x, double c, double 
 __device__ __forceinline__ double add_scaled(double x, const Scale& sc, double y)
 {
     const double r = FQ_FMA(x, sc.c_add, y);
-    if ((fq_s_hi(r) & 0x7c000000u) == 0u && sc.mode == SCALE_POW2) {
+    if (FQ_S_UNLIKELY(sc.mode == SCALE_POW2 && (fq_s_hi(r) & 0x7c000000u) == 0u)) {
         return scale_add_tiny(x, sc.c, y);
     }
     return r;
